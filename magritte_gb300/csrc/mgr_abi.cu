@@ -104,8 +104,9 @@ void set_line_scales(MgrModel* m, double Ke, double Ko) {
 // One correctly rounded erff table per device (51 MB), shared by every model on it.
 static std::mutex g_erf_mutex;
 static const float* g_erf_band[64] = {};
+static const float4* g_erf_node[64] = {};
 
-cudaError_t erf_band_table(const float** out) {
+cudaError_t erf_band_table(const float** out, const float4** nodes) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -115,11 +116,14 @@ cudaError_t erf_band_table(const float** out) {
         int nsm = 1;
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
         void* p = nullptr;
-        e = cudaMalloc(&p, (size_t)kErfBandCount * sizeof(float));
+        // the node table follows the band table
+        constexpr size_t band_bytes = ((size_t)kErfBandCount * sizeof(float) + 255) & ~size_t(255);
+        e = cudaMalloc(&p, band_bytes + kErfNodes * sizeof(float4));
         if (e != cudaSuccess) return e;
         cudaStream_t s = nullptr;
         e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = fill_erf_band(static_cast<float*>(p), s, nsm);
+        float4* nd = reinterpret_cast<float4*>(static_cast<unsigned char*>(p) + band_bytes);
+        if (e == cudaSuccess) e = fill_erf_band(static_cast<float*>(p), nd, s, nsm);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (s) cudaStreamDestroy(s);
         if (e != cudaSuccess) {
@@ -127,8 +131,10 @@ cudaError_t erf_band_table(const float** out) {
             return e;
         }
         g_erf_band[dev] = static_cast<const float*>(p);
+        g_erf_node[dev] = nd;
     }
     *out = g_erf_band[dev];
+    *nodes = g_erf_node[dev];
     return cudaSuccess;
 }
 
@@ -368,6 +374,30 @@ int mgr_model_create(const MgrModelDesc* d, MgrModel** out) {
     }
     std::vector<float> dls, dll;
     line_offset_tables(d->line, d->sorted_line, L, dls, dll);
+    // offsets of each line's neighbours in frequency, and whether any two lines can be within
+    // reach of one element pair: max_dist widths on either side plus the Doppler jump of the
+    // fastest pair of points (the staged solve sums only the own line then)
+    std::vector<float2> line_nb(L);
+    m->lines_apart = true;
+    {
+        double ub_max = 0.0, v2 = 0.0;
+        for (uint32_t p = 0; p < P; p++) {
+            ub_max = std::max(ub_max, ub[p]);
+            const double* v = d->velocity + 3 * (size_t)p;
+            v2 = std::max(v2, v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+        }
+        const double reach = d->max_distance_opacity_contribution * ub_max + 4.0 * std::sqrt(v2);
+        for (uint32_t s = 0; s < L; s++) {
+            const uint32_t l = d->sorted_line_map[s];
+            const size_t row = (size_t)l * L;
+            line_nb[l].x = s > 0 ? dls[row + s - 1] : -INFINITY;
+            line_nb[l].y = s + 1 < L ? dls[row + s + 1] : INFINITY;
+            if (s > 0 && !(d->sorted_line[s] - d->sorted_line[s - 1] > 2.0 * reach * d->sorted_line[s]))
+                m->lines_apart = false;
+        }
+    }
+    m->line_blocks = line_disc;
+    for (uint32_t f = 0; f < F && m->line_blocks; f++) m->line_blocks = d->corr_line[f] == f / d->nquads;
     std::vector<float> bkt(2 * (size_t)d->nboundary);  // h / (k T) per boundary, double-float
     for (uint32_t b = 0; b < d->nboundary; b++) {
         const double k = HH_OVER_KB / (d->boundary_condition[b] == BC_THERMAL ? d->boundary_temperature[b] : T_CMB);
@@ -412,6 +442,7 @@ int mgr_model_create(const MgrModelDesc* d, MgrModel** out) {
         if ((e = upload(m, &dm.dls, dls.data(), (size_t)L * L)) != cudaSuccess) break;
         if ((e = upload(m, &dm.lq2f, lq2f.data(), lq2f.size())) != cudaSuccess) break;
         if ((e = upload(m, &dm.dll, dll.data(), (size_t)L * L)) != cudaSuccess) break;
+        if ((e = upload(m, &dm.line_nb, line_nb.data(), line_nb.size())) != cudaSuccess) break;
         if ((e = upload(m, &dm.line_df, line_df.data(), line_df.size())) != cudaSuccess) break;
         if ((e = dalloc(m, &m->em, PL)) != cudaSuccess) break;
         if ((e = dalloc(m, &m->op, PL)) != cudaSuccess) break;
@@ -472,7 +503,7 @@ int mgr_model_create(const MgrModelDesc* d, MgrModel** out) {
     dm.iw_f = m->iw_f;
     dm.Sp_f = m->Sp_f;
     dm.iw_lo = m->iw_lo;
-    if ((e = erf_band_table(&dm.erf_band)) != cudaSuccess) {
+    if ((e = erf_band_table(&dm.erf_band, &dm.erf_node)) != cudaSuccess) {
         int rc = cuda_fail(e, "erff table");
         mgr_model_free(m);
         return rc;

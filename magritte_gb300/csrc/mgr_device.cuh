@@ -112,6 +112,10 @@ struct DevModel {
     // (float)erf((double)x) for every float x in [kErfBandLo, 3.919206), indexed by the
     // bit pattern of x minus that of kErfBandLo (one table per device, owned by the library)
     const float* erf_band;
+    // erf about the nodes x0 = i / 2048 up to 3.92 (kErfNodes, one table per device): erf(x0)
+    // and erf'(x0), each as two floats
+    const float4* erf_node;
+    const float2* line_nb;       // [L] offsets of the neighbouring lines (sorted by frequency), -+inf at the ends
     const float* dls;            // [L][L] (float)(sorted_line[s] - line[l0]) at l0*L + s
     const float* dll;            // [L][L] (float)(line[l] - line[l0]) at l0*L + l
     float max_dist_f;            // (float)max_dist
@@ -311,6 +315,7 @@ MGR_HD uint32_t n_interp_all_lines(const DevModel& m, uint32_t crt, uint32_t nxt
 constexpr uint32_t kMaxOffDiag = 4;  // largest n_off_diag of the banded (non-local ALO) solve
 
 constexpr float kErfBandLo = 1.4375f;
+constexpr uint32_t kErfNodes = 8028;  // nearest nodes of |x| < 3.919206: 0 .. 8027
 constexpr uint32_t kErfBandCount = 0x407ad445u - 0x3fb80000u;  // bits(3.919206f) - bits(1.4375f)
 
 // Correctly rounded single-precision erf (double erf rounded once to float).

@@ -2,6 +2,7 @@
 #include "mgr_internal.h"
 #include "mgr_reduce.cuh"
 #include "mgr_solve.cuh"
+#include "mgr_staged.cuh"
 
 namespace mgr {
 
@@ -38,15 +39,23 @@ __global__ void line_tables_kernel(const double* __restrict__ em, const double* 
 // Correctly rounded erff table of split precision's same-wing erf differences:
 // (float)erf((double)x) for every float x in [kErfBandLo, 3.919206).
 // ---------------------------------------------------------------------------------
-__global__ void erf_band_kernel(float* __restrict__ t) {
+__global__ void erf_band_kernel(float* __restrict__ t, float4* __restrict__ nodes) {
     const uint32_t base = __float_as_uint(kErfBandLo);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < kErfNodes; i += gridDim.x * blockDim.x) {
+        const double x = (double)i / 2048.0;
+        const double E = erf(x), D = 2.0 * INVERSE_SQRT_PI * exp(-x * x);
+        float4 v;
+        split_hl(E, v.x, v.y);
+        split_hl(D, v.z, v.w);
+        nodes[i] = v;
+    }
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < kErfBandCount; i += gridDim.x * blockDim.x)
         t[i] = (float)erf((double)__uint_as_float(base + i));
 }
 
-cudaError_t fill_erf_band(float* table, cudaStream_t stream, int sm_count) {
+cudaError_t fill_erf_band(float* table, float4* nodes, cudaStream_t stream, int sm_count) {
     count_launch();
-    erf_band_kernel<<<sm_count * 8, 256, 0, stream>>>(table);
+    erf_band_kernel<<<sm_count * 8, 256, 0, stream>>>(table, nodes);
     return cudaGetLastError();
 }
 
@@ -286,6 +295,51 @@ __global__ void __launch_bounds__(256, MINB)
                 if (!isfinite(r.u)) atomicOr(status, ST_NONFINITE);
             }
         }
+        __syncwarp();
+    }
+}
+
+// ---------------------------------------------------------------------------------
+// Formal solve, stage 1, staged (mgr_staged.cuh): one warp per K consecutive (origin, ray
+// pair) items, results as fo2_kernel's.
+// ---------------------------------------------------------------------------------
+template <int MODE, int AP, int MINB, int GEO>
+__global__ void __launch_bounds__(256, MINB)
+    fo2_staged_kernel(const __grid_constant__ DevModel m, uint32_t cap, StagedPlan plan, uint32_t o_begin,
+                      uint32_t o_end, uint32_t rr0, uint32_t nR, double* __restrict__ U, size_t u_stride, uint32_t u_o0,
+                      double* __restrict__ LD, size_t ld_stride, uint32_t ld_o0, const uint8_t* __restrict__ cls,
+                      uint32_t cls_id, int* status) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int nw = blockDim.x >> 5;
+    const int w = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    double* sl = reinterpret_cast<double*>(smem);
+    const uint32_t Lpad = (m.L + 1) & ~1u;
+    unsigned char* mine = smem + (size_t)Lpad * 8 + (size_t)w * staged_warp_bytes(MODE, cap, plan.K, plan.W);
+    for (uint32_t i = threadIdx.x; i < m.L; i += blockDim.x) sl[i] = m.sorted_line[i];
+    __syncthreads();
+
+    const uint64_t n_items = (uint64_t)(o_end - o_begin) * nR;
+    const uint64_t stride = (uint64_t)gridDim.x * nw * plan.K;
+    for (uint64_t item = ((uint64_t)blockIdx.x * nw + w) * plan.K; item < n_items; item += stride) {
+        bool any = false;
+        for (uint32_t j = 0; j < plan.K; j++) {
+            bool live = item + j < n_items;
+            const uint32_t o = live ? o_begin + (uint32_t)((item + j) / nR) : 0u;
+            const uint32_t rr = live ? rr0 + (uint32_t)((item + j) % nR) : 0u;
+            if (live && cls && cls[(size_t)o * m.hnrays + rr] != cls_id) live = false;  // another class's launch
+            staged_trace<MODE, GEO>(m, o, rr, cap, mine + staged_tile_bytes(MODE, plan.W), j, lane, status, live);
+            any = any || live;
+        }
+        __syncwarp();
+        if (!any) continue;
+        staged_solve<MODE, AP>(m, sl, cap, plan, mine, item, o_begin, nR, lane,
+                               [&](uint32_t j, uint32_t o, uint32_t f, const LaneResult& r) {
+                                   const size_t k = (size_t)((item + j) % nR);
+                                   U[k * u_stride + (size_t)(o - u_o0) * m.F + f] = r.u;
+                                   if (LD) LD[k * ld_stride + (size_t)(o - ld_o0) * m.F + f] = r.solved ? r.Ldiag : 0.0;
+                                   if (!isfinite(r.u)) atomicOr(status, ST_NONFINITE);
+                               });
         __syncwarp();
     }
 }
@@ -688,6 +742,76 @@ size_t fo2_work_bytes(const MgrModel* model, uint32_t n_origins, bool stage_u, b
     return chunk * per;
 }
 
+// Whether the staged solve serves this model: its tiles hold one line's data, so the
+// frequencies come line by line and pairs that reach several lines are rare.
+bool staged_ok(const MgrModel* model) {
+    const DevModel& m = model->dm;
+    if (!model->line_blocks) return false;
+    return m.approx == APPROX_ONELINE || m.L == 1 || (m.approx == APPROX_CLOSELINES && model->lines_apart);
+}
+
+// How a warp's lanes are dealt out: K ray pairs per warp and chunks of whole lines (S = the
+// largest multiple of Q up to 32) or of 32 frequencies, whichever leaves the fewest
+// warp passes per ray pair, weighted by what more streams and pairs of different lengths
+// per warp cost.
+StagedPlan staged_plan(const DevModel& m) {
+    StagedPlan best{1, 32, 32};
+    double best_cost = 1e30;
+    for (uint32_t K = 1; K <= 4; K++) {
+        for (int aligned = 0; aligned < 2; aligned++) {
+            const uint32_t S = aligned ? (m.Q <= 32 ? 32 / m.Q * m.Q : 0) : 32;
+            if (S == 0) continue;
+            const uint32_t total = K * m.F, chunks = (total + S - 1) / S;
+            uint32_t span = 1;
+            for (uint32_t c0 = 0; c0 < total; c0 += S) {
+                const uint32_t last = (c0 + S < total ? c0 + S : total) - 1;
+                const uint32_t n = last / m.Q - c0 / m.Q + 1;
+                if (n > span) span = n;
+            }
+            uint32_t ns = 1;
+            while (ns < span) ns *= 2;
+            if (ns > 8) continue;
+            const double more = ns == 1 ? 0.0 : ns == 2 ? 0.08 : ns == 4 ? 0.2 : 0.45;
+            const double cost = (double)chunks / K * (1.0 + more) * (1.0 + 0.12 * (K - 1));
+            if (cost < best_cost - 1e-9) {
+                best_cost = cost;
+                best = StagedPlan{K, S, 32 / ns};
+            }
+        }
+    }
+    return best;
+}
+
+template <int MODE, int AP, int MINB, int GEO>
+static cudaError_t launch_staged_variant(MgrModel* model, uint32_t o_begin, uint32_t o_end, uint32_t rr0, uint32_t nR,
+                                         double* U, size_t us, uint32_t uo, double* LD, size_t ls, uint32_t lo,
+                                         const uint8_t* cls, uint32_t cls_id) {
+    const DevModel& m = model->dm;
+    const uint32_t cap = cls ? model->class_cap[cls_id] : model->half_cap;
+    int nw = (MODE == MODE_SPLIT) ? model->fo2_warps_split : model->fo2_warps_fp64;
+    if (nw < 1 || nw > 8) nw = 8;
+    StagedPlan plan = staged_plan(m);
+    const uint32_t Lpad = (m.L + 1) & ~1u;
+    size_t smem = (size_t)Lpad * 8 + (size_t)nw * staged_warp_bytes(MODE, cap, plan.K, plan.W);
+    auto kern = fo2_staged_kernel<MODE, AP, MINB, GEO>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nw * 32, smem);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) return cudaErrorInvalidConfiguration;  // the ray buffers do not fit in shared memory
+    const uint64_t items = (uint64_t)(o_end - o_begin) * nR;
+    uint64_t grid = (uint64_t)model->sm_count * per_sm;
+    const uint64_t per_block = (uint64_t)nw * plan.K;
+    const uint64_t need = (items + per_block - 1) / per_block;
+    if (grid > need) grid = need;
+    if (grid < 1) grid = 1;
+    count_launch();
+    kern<<<(unsigned)grid, nw * 32, smem, model->stream>>>(m, cap, plan, o_begin, o_end, rr0, nR, U, us, uo, LD, ls, lo,
+                                                          cls, cls_id, model->status);
+    return cudaGetLastError();
+}
+
 // One launch of fo2_kernel over origins [o_begin, o_end) x ray pairs [rr0, rr0 + nR):
 // every pair (cls null, buffers sized for the model's longest half ray) or the pairs of
 // length class cls_id (buffers sized for that class's longest half ray).
@@ -735,6 +859,17 @@ static cudaError_t launch_fo2_minb(MgrModel* model, uint32_t o_begin, uint32_t o
     for (int c = 0; c < (cls ? kLenClasses : 1); c++) {
         if (cls && model->class_cap[c] == 0) continue;
         cudaError_t e;
+        if (staged_ok(model)) {
+            if (any_geo) e = launch_staged_variant<MODE, AP, 3, 1>(model, o_begin, o_end, rr0, nR, U, us, uo, LD, ls, lo, cls, c);
+            else if (minb == 2)
+                e = launch_staged_variant<MODE, AP, 2, 0>(model, o_begin, o_end, rr0, nR, U, us, uo, LD, ls, lo, cls, c);
+            else if (minb == 4)
+                e = launch_staged_variant<MODE, AP, 4, 0>(model, o_begin, o_end, rr0, nR, U, us, uo, LD, ls, lo, cls, c);
+            else
+                e = launch_staged_variant<MODE, AP, 3, 0>(model, o_begin, o_end, rr0, nR, U, us, uo, LD, ls, lo, cls, c);
+            if (e != cudaSuccess) return e;
+            continue;
+        }
         // spherical symmetry and adaptive rays: the run-time geometry variant, one tile
         if (any_geo) e = launch_fo2_variant<MODE, AP, 3, false, 1>(model, o_begin, o_end, rr0, nR, U, us, uo, LD, ls, lo,
                                                                   nullptr, cls, c);

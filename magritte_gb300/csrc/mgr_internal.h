@@ -48,6 +48,8 @@ struct MgrModel {
     int fo2_minb_fp64 = 2;
     int fo2_warps_fp64 = 4;
     int sm_count = 1;                // multiprocessors of the model's device
+    bool line_blocks = false;        // frequency f is quadrature point f % Q of line f / Q
+    bool lines_apart = false;        // no two lines within reach of one another (staged solve, mgr_staged.cuh)
     bool line_disc = true;           // frequencies form a line spectral discretisation
     bool inputs_replaced = false;    // velocities or frequencies replaced through a *_device setter
     int* status = nullptr;           // device status word
@@ -178,10 +180,11 @@ cudaError_t launch_nint_table(MgrModel* model);
 cudaError_t launch_hl_tables(MgrModel* model);  // trace filter tables (edge_hl, pos_hl)
 cudaError_t launch_edge_pack(MgrModel* model, const double4_32a* pos, const uint32_t* nbr, uint64_t E,
                              double4_32a* edge);
-// Fills the correctly rounded erff table (kErfBandCount floats) on `stream`.
-cudaError_t fill_erf_band(float* table, cudaStream_t stream, int sm_count);
-// The current device's erff table, created (cudaMalloc, one fill launch, synchronised)
+// Fills the correctly rounded erff table (kErfBandCount floats) and the erf node table
+// (kErfNodes entries) on `stream`.
+cudaError_t fill_erf_band(float* table, float4* nodes, cudaStream_t stream, int sm_count);
+// The current device's erff and erf node tables, created (cudaMalloc, one fill launch, synchronised)
 // by the first call on each device and kept until the process exits.
-cudaError_t erf_band_table(const float** out);
+cudaError_t erf_band_table(const float** out, const float4** nodes);
 
 }  // namespace mgr

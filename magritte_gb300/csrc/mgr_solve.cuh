@@ -61,6 +61,23 @@ MGR_HD void set_dsh0(HalfSmem& h, double shift0) {
 // one line's criterion, as the imagers trace.
 constexpr uint32_t kAllLines = 0xffffffffu;
 
+// What a trace stores per step (HalfSmem arrays): everything, or only what the staged
+// solve (mgr_staged.cuh) reads: ids, eid, dsh, dsl and dzs in split precision (20 bytes),
+// ids, eid, shift and dZ in FP64 mode (24 bytes).
+enum { LAY_FULL = 0, LAY_SPLIT = 1, LAY_FP64 = 2 };
+
+template <int LAY>
+__device__ __forceinline__ void store_dz(const DevModel& m, const HalfSmem& h, int s, double dZ) {
+    if (LAY == LAY_SPLIT) h.dzs[s] = (float)dZ * m.dz_scale;
+    else h.dZ[s] = dZ;
+}
+
+template <int LAY>
+__device__ __forceinline__ void store_shift(const HalfSmem& h, int s, double sh) {
+    if (LAY != LAY_SPLIT) h.shift[s] = sh;
+    if (LAY != LAY_FP64) store_dsh(h, s, sh);
+}
+
 // Shared-memory carve-up of one warp's two half-ray buffers.
 __device__ __forceinline__ void carve_halves(unsigned char* base, uint32_t cap, HalfSmem& bk, HalfSmem& fw) {
     double* d = reinterpret_cast<double*>(base);
@@ -280,7 +297,7 @@ __device__ __forceinline__ int warp_next_point_f32(const DevModel& m, const Trac
 // geometry.tpp:118-159): every lane steps the same shells; lane 0 stores the steps, with
 // each step's shift at its distance along the ray (get_shift_spherical_symmetry) and the
 // half's origin shift (shift0, not 1 in the comoving frame there).
-template <bool STORE, int FRAME>
+template <bool STORE, int FRAME, int LAY = LAY_FULL>
 __device__ int trace_half_sph(const DevModel& m, uint32_t o, uint32_t r, uint32_t cap, HalfSmem& h, int lane,
                               int* status) {
     const double* d = FRAME ? m.raydir + 3 * r : ray_dir(m, o, r);
@@ -311,11 +328,9 @@ __device__ int trace_half_sph(const DevModel& m, uint32_t o, uint32_t r, uint32_
         if (STORE && lane == 0) {
             h.ids[count] = nxt;
             h.eid[count] = sph_eid(crt, nxt);
-            h.dZ[count] = dZl;
-            const double sh = shift_sph(m, FRAME, o, r, nxt, Z, d);
-            h.shift[count] = sh;
-            store_dsh(h, count, sh);
-            h.dzs[count] = (float)dZl * m.dz_scale;
+            store_shift<LAY>(h, count, shift_sph(m, FRAME, o, r, nxt, Z, d));
+            store_dz<LAY>(m, h, count, dZl);
+            if (LAY == LAY_FULL) h.dzs[count] = (float)dZl * m.dz_scale;
         }
         count++;
         if (m.p2b[nxt] != m.P) break;
@@ -335,10 +350,10 @@ __device__ int trace_half_sph(const DevModel& m, uint32_t o, uint32_t r, uint32_
 // r >= hnrays, geometry.tpp:428-465).
 // GEO 0 compiles the general geometry with shared rays only (the caller has checked the
 // model); GEO 1 handles every geometry at run time.
-template <bool STORE, int FRAME = 0, int GEO = 1, bool FILTER = true>
+template <bool STORE, int FRAME = 0, int GEO = 1, bool FILTER = true, int LAY = LAY_FULL>
 __device__ int trace_half(const DevModel& m, uint32_t o, uint32_t r, uint32_t cap, HalfSmem& h, int lane,
                           int* status) {
-    if (GEO && m.sph) return trace_half_sph<STORE, FRAME>(m, o, r, cap, h, lane, status);
+    if (GEO && m.sph) return trace_half_sph<STORE, FRAME, LAY>(m, o, r, cap, h, lane, status);
     // the formal solves trace along the origin's (adaptive) directions, the old imager
     // along the shared ones (trace_ray<Rest, false>, solver.tpp:550-552)
     const double* d = (FRAME || !GEO) ? m.raydir + 3 * r : ray_dir(m, o, r);
@@ -370,11 +385,13 @@ __device__ int trace_half(const DevModel& m, uint32_t o, uint32_t r, uint32_t ca
             Zn = dot3_rn(dsub_rn(q.x, po.x), dsub_rn(q.y, po.y), dsub_rn(q.z, po.z), dx, dy, dz);
         }
         const int base = count - np;
+        double dz_lane = 0.0;
         for (int j = 0; j < np; j++) {
             const double dZl = dsub_rn(__shfl_sync(FULL_MASK, Zn, j), Z);
             Z = dadd_rn(Z, dZl);
-            if (STORE && lane == 0) h.dZ[base + j] = dZl;
+            if (lane == j) dz_lane = dZl;
         }
+        if (STORE && lane < np) store_dz<LAY>(m, h, base + lane, dz_lane);
         np = 0;
     };
     while (true) {
@@ -413,7 +430,7 @@ __device__ int trace_half(const DevModel& m, uint32_t o, uint32_t r, uint32_t ca
         if (STORE && lane == 0) {
             h.ids[count] = nxt;
             h.eid[count] = eid;
-            if (exact) h.dZ[count] = dZl;
+            if (exact) store_dz<LAY>(m, h, count, dZl);
         }
         if (!exact) {
             if (lane == np) pend = nxt;
@@ -433,10 +450,8 @@ __device__ int trace_half(const DevModel& m, uint32_t o, uint32_t r, uint32_t ca
     if (STORE && count > 0) {
         // Per-step Doppler shifts and FP32 copies, one step per lane.
         for (int s = lane; s < count; s += 32) {
-            const double sh = FRAME ? shift_rest(m, r, h.ids[s], d) : shift_comoving(m, o, h.ids[s], d);
-            h.shift[s] = sh;
-            store_dsh(h, s, sh);
-            h.dzs[s] = (float)h.dZ[s] * m.dz_scale;
+            store_shift<LAY>(h, s, FRAME ? shift_rest(m, r, h.ids[s], d) : shift_comoving(m, o, h.ids[s], d));
+            if (LAY == LAY_FULL) h.dzs[s] = (float)h.dZ[s] * m.dz_scale;
         }
         __syncwarp();
     }
@@ -1362,6 +1377,120 @@ template <int NB>
 MGR_HD void band_tail(const DevModel& m, const double* sl, const LaneCtx& c, const BandRing<NB>& tp,
                       const BandRing<NB>& bt, BandOut<NB>& out);
 
+// Both sweeps' states combined at the origin into u, L_diag (and v of the uv solve): the
+// two-sided row, or the boundary row of an origin at one end of the ray (boundary
+// intensity Io).  PROJ: the sweeps are in projective form (ptop, pbot), else in (top, bot).
+template <int MODE, bool UV, bool PROJ>
+MGR_HD void finish_lane(Sweep& top, Sweep& bot, const Proj& ptop, const Proj& pbot, double Io, LaneResult& res) {
+    if constexpr (PROJ) {
+        if (MODE == MODE_SPLIT && top.rows && bot.rows) {
+            // the origin's row in projective form with elim_row_proj's FP32 coefficients
+            // q = dtau_b / dtau_t, iC = (dtau_t + dtau_b) dtau_b / 2:
+            //   u = (q Su_t + S_in iC + Su_b) / (q G_t + iC + G_b),  L_diag = iC / (same)
+            // (the reference's u[c] and L_diag[c], with G = NG / D, Su = NS / D per side)
+            const float dto = top.dtf, dti = bot.dtf;
+            double q, iC;
+            if (dto > 1.0e-18f && dto < 1.0e18f && dti > 1.0e-18f && dti < 1.0e18f) {
+                q = f2d(fast_div(dti, dto));
+                iC = f2d(0.5f * (dto + dti) * dti);
+            } else {
+                const double2 k = elim_coeffs_fp64(dto, dti);
+                q = k.x;
+                iC = k.y;
+            }
+            const double qrt = q * drcp<MODE>(ptop.D);
+            const double rb = drcp<MODE>(pbot.D);
+            const double num = fma(qrt, ptop.NS, fma(rb, pbot.NS, f2d(bot.S_inf) * iC));
+            const double rd = drcp<MODE>(fma(qrt, ptop.NG, fma(rb, pbot.NG, iC)));
+            res.u = num * rd;
+            res.Ldiag = iC * rd;
+            return;
+        }
+        // one-sided rays: back to (F / (1 + F), 1 / (1 + F), Su) at the origin
+        if (top.rows) {
+            const double r = drcp<MODE>(ptop.D);
+            top.F = ptop.NG * r;  // G
+            top.FI = ptop.Dp * r;
+            top.Su = ptop.NS * r;
+        }
+        if (bot.rows) {
+            const double r = drcp<MODE>(pbot.D);
+            bot.F = pbot.NG * r;
+            bot.FI = pbot.Dp * r;
+            bot.Su = pbot.NS * r;
+        }
+    }
+
+    // ---- combine at the origin ----
+    if (top.rows && bot.rows) {
+        const double dtau_avg = 0.5 * (top.dt + bot.dt);
+        const double iA = dtau_avg * top.dt;
+        const double iC = dtau_avg * bot.dt;
+        const double A = drcp<MODE>(iA);
+        const double FFc = (A * (PROJ ? top.F : top.F * top.FI) + 1.0) * iC;
+        const double Su_pre = (A * top.Su + bot.S_in) * iC;
+        const double GP = PROJ ? bot.F : bot.F * bot.FI;
+        const double D = drcp<MODE>(FFc + GP);
+        res.u = (Su_pre + bot.Su) * D;
+        res.Ldiag = iC * D;
+        if constexpr (UV) {
+            // solve_feautrier_order_2_uv (solver.tpp:2896-2916): u at the neighbours of the
+            // origin from each side's last row, v the finite-difference derivative
+            const double u_min = top.Su + res.u * top.FI;
+            const double u_plus = bot.Su + res.u * bot.FI;
+            const double dtaumin = (double)top.dt;
+            double dtauplus = (double)bot.dt;
+            if (!top.last_large && !bot.last_large) {
+                // The reference evaluates the pair (origin, next) with compute_curr_opacity
+                // left false by the pair (previous, origin), so its "current" opacity is
+                // that of the previous element (solver.tpp:2899-2907, :2161-2170).
+                if constexpr (MODE == MODE_FP64) dtauplus = 0.5 * (top.chi_out + bot.chi_out) * bot.dz_last;
+                else dtauplus = (double)(0.5f * ((float)top.chi_out + (float)bot.chi_out) * (float)bot.dz_last);
+            }
+            res.dtm = dtaumin;
+            res.dtp = dtauplus;
+            const double coeffmin = -dtauplus / (dtaumin * dtaumin + dtaumin * dtauplus);
+            const double coeffplus = dtaumin / (dtaumin * dtauplus + dtauplus * dtauplus);
+            const double coeffzero = -coeffmin - coeffplus;
+            res.v = -(coeffmin * u_min + coeffplus * u_plus + coeffzero * res.u);
+        }
+    } else if (bot.rows) {  // origin is the first element
+        const double Ibdy = Io;
+        const double inverse_dtau_f = drcp<MODE>(bot.dt);
+        const double Cf = 2.0 * inverse_dtau_f * inverse_dtau_f;
+        const double Bf_min_Cf = 1.0 + 2.0 * inverse_dtau_f;
+        const double Bf = Bf_min_Cf + Cf;
+        double Suf;
+        if constexpr (MODE == MODE_FP64) Suf = (bot.S_in + 2.0 * Ibdy * inverse_dtau_f) / Bf;
+        else Suf = (bot.S_in + 2.0 * Ibdy * inverse_dtau_f) * drcp<MODE>(Bf);
+        const double FFf = 0.5 * Bf_min_Cf * bot.dt * bot.dt;
+        const double GP = PROJ ? bot.F : bot.F * bot.FI;
+        const double D = drcp<MODE>(FFf + GP);
+        res.u = (Suf * (1.0 + FFf) + bot.Su) * D;
+        res.Ldiag = drcp<MODE>(Cf) * D;
+        if constexpr (UV) res.v = Ibdy - res.u;  // Sv[first] = I_bdy_f - Su[first]
+    } else {  // origin is the last element
+        const double Ibdy = Io;
+        const double inverse_dtau_l = drcp<MODE>(top.dt);
+        const double Al = 2.0 * inverse_dtau_l * inverse_dtau_l;
+        const double Bl_min_Al = 1.0 + 2.0 * inverse_dtau_l;
+        const double Bl = Bl_min_Al + Al;
+        const double Sl = top.S_in + 2.0 * Ibdy * inverse_dtau_l;
+        if constexpr (PROJ) {
+            // with G = F / (1 + F) and FI = 1 / (1 + F): (1 + F) / (Bl F + Bl - Al) = 1 / (Bl G + (Bl - Al) FI)
+            const double den = drcp<MODE>(Bl * top.F + Bl_min_Al * top.FI);
+            res.u = (Al * top.Su + Sl) * den;
+            res.Ldiag = den;
+        } else {
+            const double denominator = drcp<MODE>(Bl * top.F + Bl_min_Al);
+            res.u = (Al * top.Su + Sl) * (1.0 + top.F) * denominator;
+            if constexpr (UV) res.v = res.u - Ibdy;  // Sv[last] = Su[last] - I_bdy_l
+            if constexpr (MODE == MODE_FP64) res.Ldiag = (1.0 + top.F) / (Bl_min_Al + Bl * top.F);
+            else res.Ldiag = (1.0 + top.F) * denominator;
+        }
+    }
+}
+
 // Two-sided Feautrier solve of frequency c.f on the ray pair staged in `bk`
 // (backward half, direction rr) and `fw` (forward half, antipode).  Both halves run
 // through the same sweep code (outer end first):
@@ -1505,113 +1634,7 @@ __host__ __device__ LaneResult solve_lane(const DevModel& m, const double* sl, c
 
     if constexpr (NB > 0) band_tail<NB>(m, sl, c, rtop, rbot, *bo);
 
-    if constexpr (PROJ) {
-        if (top.rows && bot.rows) {
-            // the origin's row in projective form with elim_row_proj's FP32 coefficients
-            // q = dtau_b / dtau_t, iC = (dtau_t + dtau_b) dtau_b / 2:
-            //   u = (q Su_t + S_in iC + Su_b) / (q G_t + iC + G_b),  L_diag = iC / (same)
-            // (the reference's u[c] and L_diag[c], with G = NG / D, Su = NS / D per side)
-            const float dto = top.dtf, dti = bot.dtf;
-            double q, iC;
-            if (dto > 1.0e-18f && dto < 1.0e18f && dti > 1.0e-18f && dti < 1.0e18f) {
-                q = f2d(fast_div(dti, dto));
-                iC = f2d(0.5f * (dto + dti) * dti);
-            } else {
-                const double2 k = elim_coeffs_fp64(dto, dti);
-                q = k.x;
-                iC = k.y;
-            }
-            const double qrt = q * drcp<MODE>(ptop.D);
-            const double rb = drcp<MODE>(pbot.D);
-            const double num = fma(qrt, ptop.NS, fma(rb, pbot.NS, f2d(bot.S_inf) * iC));
-            const double rd = drcp<MODE>(fma(qrt, ptop.NG, fma(rb, pbot.NG, iC)));
-            res.u = num * rd;
-            res.Ldiag = iC * rd;
-            return res;
-        }
-        // one-sided rays: back to (F / (1 + F), 1 / (1 + F), Su) at the origin
-        if (top.rows) {
-            const double r = drcp<MODE>(ptop.D);
-            top.F = ptop.NG * r;  // G
-            top.FI = ptop.Dp * r;
-            top.Su = ptop.NS * r;
-        }
-        if (bot.rows) {
-            const double r = drcp<MODE>(pbot.D);
-            bot.F = pbot.NG * r;
-            bot.FI = pbot.Dp * r;
-            bot.Su = pbot.NS * r;
-        }
-    }
-
-    // ---- combine at the origin ----
-    if (top.rows && bot.rows) {
-        const double dtau_avg = 0.5 * (top.dt + bot.dt);
-        const double iA = dtau_avg * top.dt;
-        const double iC = dtau_avg * bot.dt;
-        const double A = drcp<MODE>(iA);
-        const double FFc = (A * (PROJ ? top.F : top.F * top.FI) + 1.0) * iC;
-        const double Su_pre = (A * top.Su + bot.S_in) * iC;
-        const double GP = PROJ ? bot.F : bot.F * bot.FI;
-        const double D = drcp<MODE>(FFc + GP);
-        res.u = (Su_pre + bot.Su) * D;
-        res.Ldiag = iC * D;
-        if constexpr (UV) {
-            // solve_feautrier_order_2_uv (solver.tpp:2896-2916): u at the neighbours of the
-            // origin from each side's last row, v the finite-difference derivative
-            const double u_min = top.Su + res.u * top.FI;
-            const double u_plus = bot.Su + res.u * bot.FI;
-            const double dtaumin = (double)top.dt;
-            double dtauplus = (double)bot.dt;
-            if (!top.last_large && !bot.last_large) {
-                // The reference evaluates the pair (origin, next) with compute_curr_opacity
-                // left false by the pair (previous, origin), so its "current" opacity is
-                // that of the previous element (solver.tpp:2899-2907, :2161-2170).
-                if constexpr (MODE == MODE_FP64) dtauplus = 0.5 * (top.chi_out + bot.chi_out) * bot.dz_last;
-                else dtauplus = (double)(0.5f * ((float)top.chi_out + (float)bot.chi_out) * (float)bot.dz_last);
-            }
-            res.dtm = dtaumin;
-            res.dtp = dtauplus;
-            const double coeffmin = -dtauplus / (dtaumin * dtaumin + dtaumin * dtauplus);
-            const double coeffplus = dtaumin / (dtaumin * dtauplus + dtauplus * dtauplus);
-            const double coeffzero = -coeffmin - coeffplus;
-            res.v = -(coeffmin * u_min + coeffplus * u_plus + coeffzero * res.u);
-        }
-    } else if (bot.rows) {  // origin is the first element
-        const double Ibdy = Io;
-        const double inverse_dtau_f = drcp<MODE>(bot.dt);
-        const double Cf = 2.0 * inverse_dtau_f * inverse_dtau_f;
-        const double Bf_min_Cf = 1.0 + 2.0 * inverse_dtau_f;
-        const double Bf = Bf_min_Cf + Cf;
-        double Suf;
-        if constexpr (MODE == MODE_FP64) Suf = (bot.S_in + 2.0 * Ibdy * inverse_dtau_f) / Bf;
-        else Suf = (bot.S_in + 2.0 * Ibdy * inverse_dtau_f) * drcp<MODE>(Bf);
-        const double FFf = 0.5 * Bf_min_Cf * bot.dt * bot.dt;
-        const double GP = PROJ ? bot.F : bot.F * bot.FI;
-        const double D = drcp<MODE>(FFf + GP);
-        res.u = (Suf * (1.0 + FFf) + bot.Su) * D;
-        res.Ldiag = drcp<MODE>(Cf) * D;
-        if constexpr (UV) res.v = Ibdy - res.u;  // Sv[first] = I_bdy_f - Su[first]
-    } else {  // origin is the last element
-        const double Ibdy = Io;
-        const double inverse_dtau_l = drcp<MODE>(top.dt);
-        const double Al = 2.0 * inverse_dtau_l * inverse_dtau_l;
-        const double Bl_min_Al = 1.0 + 2.0 * inverse_dtau_l;
-        const double Bl = Bl_min_Al + Al;
-        const double Sl = top.S_in + 2.0 * Ibdy * inverse_dtau_l;
-        if constexpr (PROJ) {
-            // with G = F / (1 + F) and FI = 1 / (1 + F): (1 + F) / (Bl F + Bl - Al) = 1 / (Bl G + (Bl - Al) FI)
-            const double den = drcp<MODE>(Bl * top.F + Bl_min_Al * top.FI);
-            res.u = (Al * top.Su + Sl) * den;
-            res.Ldiag = den;
-        } else {
-            const double denominator = drcp<MODE>(Bl * top.F + Bl_min_Al);
-            res.u = (Al * top.Su + Sl) * (1.0 + top.F) * denominator;
-            if constexpr (UV) res.v = res.u - Ibdy;  // Sv[last] = Su[last] - I_bdy_l
-            if constexpr (MODE == MODE_FP64) res.Ldiag = (1.0 + top.F) / (Bl_min_Al + Bl * top.F);
-            else res.Ldiag = (1.0 + top.F) * denominator;
-        }
-    }
+    finish_lane<MODE, UV, PROJ>(top, bot, ptop, pbot, Io, res);
     return res;
 }
 
