@@ -385,11 +385,22 @@ __device__ int trace_half(const DevModel& m, uint32_t o, uint32_t r, uint32_t ca
             Zn = dot3_rn(dsub_rn(q.x, po.x), dsub_rn(q.y, po.y), dsub_rn(q.z, po.z), dx, dy, dz);
         }
         const int base = count - np;
-        double dz_lane = 0.0;
-        for (int j = 0; j < np; j++) {
-            const double dZl = dsub_rn(__shfl_sync(FULL_MASK, Zn, j), Z);
-            Z = dadd_rn(Z, dZl);
-            if (lane == j) dz_lane = dZl;
+        // Z after a step is the step's Zn unless Z + fl(Zn - Z) rounds away from it: take
+        // every step's distance from the previous Zn side by side, and the serial chain only
+        // when one of the sums does not come back to its Zn (two FP64 warp instructions for
+        // up to 32 steps instead of two per step).
+        const double Zb = __shfl_up_sync(FULL_MASK, Zn, 1);
+        const double Zprev = lane == 0 ? Z : Zb;
+        double dz_lane = dsub_rn(Zn, Zprev);
+        const bool back = __double_as_longlong(dadd_rn(Zprev, dz_lane)) == __double_as_longlong(Zn);
+        if (__all_sync(FULL_MASK, back || lane >= np)) {
+            Z = __shfl_sync(FULL_MASK, Zn, np - 1);
+        } else {
+            for (int j = 0; j < np; j++) {
+                const double dZl = dsub_rn(__shfl_sync(FULL_MASK, Zn, j), Z);
+                Z = dadd_rn(Z, dZl);
+                if (lane == j) dz_lane = dZl;
+            }
         }
         if (STORE && lane < np) store_dz<LAY>(m, h, base + lane, dz_lane);
         np = 0;
