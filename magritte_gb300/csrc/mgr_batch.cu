@@ -22,6 +22,7 @@
 #include "mgr_internal.h"
 #include "mgr_reduce.cuh"
 #include "mgr_solve.cuh"
+#include "mgr_staged.cuh"
 
 struct MgrBatch {
     int device = 0;
@@ -35,6 +36,14 @@ struct MgrBatch {
     uint64_t* d_offsets = nullptr;         // [n + 1] first origin of each model (cumulative P)
     uint64_t* d_item_off = nullptr;        // [n + 1] first (origin, ray pair) item of each model
     uint64_t* d_stage_off = nullptr;       // [n + 1] first staging entry of each model (cumulative P R F)
+    // staged solve (mgr_staged.cuh), when every model qualifies: each model's lane plan and ray
+    // capacity, the first group of K items of each model, and a warp's ray buffers per precision
+    bool staged = false;
+    mgr::StagedPlan* d_plans = nullptr;    // [n]
+    uint32_t* d_caps = nullptr;            // [n] longest half ray of each model
+    uint64_t* d_group_off = nullptr;       // [n + 1]
+    size_t staged_bytes[2] = {0, 0};       // FP64, split
+    std::vector<uint64_t> group_off;
     std::vector<uint64_t> item_off, stage_off, origin_off;  // host copies
     double* stage_u = nullptr;             // staging of u for one wave
     double* stage_ld = nullptr;            // staging of L_diag for one wave
@@ -86,6 +95,12 @@ __host__ __device__ inline size_t batch_head_bytes(uint32_t L_max) {
 }
 __host__ __device__ inline size_t batch_warp_bytes(uint32_t cap, uint32_t L_max) {
     return batch_head_bytes(L_max) + half_bytes_per_warp(cap);
+}
+
+// A warp's shared memory, the larger of the two precisions'.
+static size_t batch_need_bytes(const MgrBatch* b) {
+    if (!b->staged) return batch_warp_bytes(b->cap, b->L_max);
+    return batch_head_bytes(b->L_max) + std::max(b->staged_bytes[0], b->staged_bytes[1]);
 }
 
 __device__ __forceinline__ void copy_desc(const DevModel* __restrict__ src, DevModel* dst, int t, int nt) {
@@ -153,6 +168,65 @@ __global__ void __launch_bounds__(256, MINB)
     }
 }
 
+// Stage 1, staged (mgr_staged.cuh): one warp per K consecutive items of a model.
+template <int MODE, int AP, int MINB>
+__global__ void __launch_bounds__(256, MINB)
+    fo2_multi_staged_kernel(const DevModel* __restrict__ models, const StagedPlan* __restrict__ plans,
+                            const uint32_t* __restrict__ caps, uint32_t m0, uint32_t m1,
+                            const uint64_t* __restrict__ group_off, const uint64_t* __restrict__ stage_off,
+                            uint32_t warp_bytes, uint32_t L_max, double* __restrict__ U, double* __restrict__ LD,
+                            unsigned long long* __restrict__ tstamp, uint32_t n_models, int* status) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int nw = blockDim.x >> 5;
+    const int w = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    unsigned char* base = smem + (size_t)w * (batch_head_bytes(L_max) + warp_bytes);
+    DevModel* desc = reinterpret_cast<DevModel*>(base);
+    double* sl = reinterpret_cast<double*>(base + kDescBytes);
+    unsigned char* mine = base + batch_head_bytes(L_max);
+    if (threadIdx.x == 0) atomicMin(&tstamp[2 * n_models], global_ns());
+
+    const uint64_t g0 = group_off[m0], g1 = group_off[m1];
+    const uint64_t s0 = stage_off[m0];
+    const uint64_t stride = (uint64_t)gridDim.x * nw;
+    uint32_t mi = m0, desc_mi = 0xffffffffu;
+    StagedPlan plan{1, 32, 32};
+    uint32_t cap = 1;
+    for (uint64_t g = g0 + (uint64_t)blockIdx.x * nw + w; g < g1; g += stride) {
+        while (group_off[mi + 1] <= g) mi++;  // groups only grow within a warp
+        if (mi != desc_mi) {
+            __syncwarp();
+            copy_desc(models + mi, desc, lane, 32);
+            __syncwarp();
+            for (uint32_t i = lane; i < desc->L; i += 32) sl[i] = desc->sorted_line[i];
+            plan = plans[mi];
+            cap = caps[mi];
+            desc_mi = mi;
+            __syncwarp();
+        }
+        const DevModel& m = *desc;
+        const uint64_t item = (g - group_off[mi]) * plan.K, n_items = (uint64_t)m.P * m.hnrays;
+        if (item == 0 && lane == 0) tstamp[2 * mi] = global_ns();
+        for (uint32_t j = 0; j < plan.K; j++) {
+            const bool live = item + j < n_items;
+            const uint32_t o = live ? (uint32_t)((item + j) / m.hnrays) : 0u;
+            const uint32_t rr = live ? (uint32_t)((item + j) % m.hnrays) : 0u;
+            // general geometry with shared rays (mgr_batch_create refuses the other kinds)
+            staged_trace<MODE, 0>(m, o, rr, cap, mine + staged_tile_bytes(MODE, plan.W), j, lane, status, live);
+        }
+        __syncwarp();
+        const size_t at = (size_t)(stage_off[mi] - s0);
+        staged_solve<MODE, AP>(m, sl, cap, plan, mine, item, 0u, m.hnrays, lane,
+                               [&](uint32_t j, uint32_t o, uint32_t f, const LaneResult& r) {
+                                   const size_t k = at + ((size_t)((item + j) % m.hnrays) * m.P + o) * m.F + f;
+                                   U[k] = r.u;
+                                   if (LD) LD[k] = r.solved ? r.Ldiag : 0.0;
+                                   if (!isfinite(r.u)) atomicOr(status, ST_NONFINITE);
+                               });
+        __syncwarp();
+    }
+}
+
 // Stage 2 of models [m0, m1): J and the ALO diagonal of every (model, origin), one CTA
 // per origin, in the single-model reduction's order.  The CTA copies its model's
 // descriptor into shared memory when the model changes.
@@ -193,29 +267,49 @@ __global__ void __launch_bounds__(128)
     }
 }
 
-template <int MODE, int AP, int MINB>
-static cudaError_t launch_multi_variant(MgrBatch* b, uint32_t m0, uint32_t m1, bool want_lam) {
-    const int nw = b->warps;
-    const size_t smem = (size_t)nw * batch_warp_bytes(b->cap, b->L_max);
-    auto kern = fo2_multi_kernel<MODE, AP, MINB>;
+// Persistent grid of `kern` for `work` warps' worth of items.
+template <typename K>
+static cudaError_t multi_grid(K kern, int nw, size_t smem, int sms, uint64_t work, unsigned* grid) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nw * 32, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;  // the per-warp buffers do not fit
+    uint64_t g = (uint64_t)sms * per_sm;
+    const uint64_t need = (work + nw - 1) / nw;
+    if (g > need) g = need;
+    *grid = (unsigned)(g < 1 ? 1 : g);
+    return cudaSuccess;
+}
+
+template <int MODE, int AP, int MINB>
+static cudaError_t launch_multi_variant(MgrBatch* b, uint32_t m0, uint32_t m1, bool want_lam) {
+    const int nw = b->warps;
     int sms = 1;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
-    const uint64_t items = b->item_off[m1] - b->item_off[m0];
-    uint64_t grid = (uint64_t)sms * per_sm;
-    const uint64_t need = (items + nw - 1) / nw;
-    if (grid > need) grid = need;
-    if (grid < 1) grid = 1;
     const uint32_t n = (uint32_t)b->models.size();
-    count_launch();
-    kern<<<(unsigned)grid, nw * 32, smem, b->stream>>>(b->d_models, m0, m1, b->d_item_off, b->d_stage_off, b->cap,
-                                                       b->L_max, b->stage_u, want_lam ? b->stage_ld : nullptr,
-                                                       b->d_t, n, b->status);
+    unsigned grid = 1;
+    cudaError_t e;
+    if (b->staged) {
+        const size_t bytes = b->staged_bytes[MODE == MODE_SPLIT ? 1 : 0];
+        const size_t smem = (size_t)nw * (batch_head_bytes(b->L_max) + bytes);
+        auto kern = fo2_multi_staged_kernel<MODE, AP, MINB>;
+        e = multi_grid(kern, nw, smem, sms, b->group_off[m1] - b->group_off[m0], &grid);
+        if (e != cudaSuccess) return e;
+        count_launch();
+        kern<<<grid, nw * 32, smem, b->stream>>>(b->d_models, b->d_plans, b->d_caps, m0, m1, b->d_group_off,
+                                                 b->d_stage_off, (uint32_t)bytes, b->L_max, b->stage_u,
+                                                 want_lam ? b->stage_ld : nullptr, b->d_t, n, b->status);
+    } else {
+        const size_t smem = (size_t)nw * batch_warp_bytes(b->cap, b->L_max);
+        auto kern = fo2_multi_kernel<MODE, AP, MINB>;
+        e = multi_grid(kern, nw, smem, sms, b->item_off[m1] - b->item_off[m0], &grid);
+        if (e != cudaSuccess) return e;
+        count_launch();
+        kern<<<grid, nw * 32, smem, b->stream>>>(b->d_models, m0, m1, b->d_item_off, b->d_stage_off, b->cap, b->L_max,
+                                                 b->stage_u, want_lam ? b->stage_ld : nullptr, b->d_t, n, b->status);
+    }
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const uint64_t origins = b->origin_off[m1] - b->origin_off[m0];
@@ -268,6 +362,9 @@ static void batch_release(MgrBatch* b) {
     cudaFree(b->d_offsets);
     cudaFree(b->d_item_off);
     cudaFree(b->d_stage_off);
+    cudaFree(b->d_plans);
+    cudaFree(b->d_caps);
+    cudaFree(b->d_group_off);
     cudaFree(b->stage_u);
     cudaFree(b->stage_ld);
     cudaFree(b->d_J);
@@ -354,6 +451,23 @@ int mgr_batch_create(MgrModel* const* models, uint32_t n_models, MgrBatch** out)
         stage_off[i + 1] = stage_off[i] + entries;
         largest = std::max(largest, entries);
     }
+    // the staged solve when every model qualifies and a warp's ray buffers are no larger than
+    // the general kernel's (they hold K ray pairs of the model's own longest ray)
+    std::vector<StagedPlan> plans(n_models);
+    std::vector<uint32_t> caps(n_models);
+    b->group_off.assign(n_models + 1, 0);
+    b->staged = true;
+    for (uint32_t i = 0; i < n_models; i++) {
+        const MgrModel* m = models[i];
+        b->staged = b->staged && staged_ok(m);
+        plans[i] = staged_plan(m->dm);
+        caps[i] = m->half_cap;
+        b->group_off[i + 1] = b->group_off[i] + ((uint64_t)m->dm.P * m->dm.hnrays + plans[i].K - 1) / plans[i].K;
+        b->staged_bytes[0] =
+            std::max(b->staged_bytes[0], staged_warp_bytes(MODE_FP64, caps[i], plans[i].K, plans[i].W));
+        b->staged_bytes[1] =
+            std::max(b->staged_bytes[1], staged_warp_bytes(MODE_SPLIT, caps[i], plans[i].K, plans[i].W));
+    }
     b->n_items = offsets[n_models];
     b->origin_off = offsets;
     b->item_off = item_off;
@@ -366,6 +480,14 @@ int mgr_batch_create(MgrModel* const* models, uint32_t n_models, MgrBatch** out)
     if (e == cudaSuccess) e = cudaMalloc(&b->d_offsets, (n_models + 1) * sizeof(uint64_t));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_item_off, (n_models + 1) * sizeof(uint64_t));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_stage_off, (n_models + 1) * sizeof(uint64_t));
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_plans, n_models * sizeof(StagedPlan));
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_caps, n_models * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_group_off, (n_models + 1) * sizeof(uint64_t));
+    if (e == cudaSuccess)
+        e = cudaMemcpy(b->d_plans, plans.data(), n_models * sizeof(StagedPlan), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(b->d_caps, caps.data(), n_models * sizeof(uint32_t), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess)
+        e = cudaMemcpy(b->d_group_off, b->group_off.data(), (n_models + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMalloc(&b->stage_u, b->stage_entries * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&b->stage_ld, b->stage_entries * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_J, n_models * sizeof(double*));
@@ -385,7 +507,7 @@ int mgr_batch_create(MgrModel* const* models, uint32_t n_models, MgrBatch** out)
         batch_release(b);
         return cuda_fail(e, "batch set-up");
     }
-    const size_t per_warp = batch_warp_bytes(b->cap, b->L_max);
+    const size_t per_warp = batch_need_bytes(b);
     int max_smem = 0;
     cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
     while (b->warps > 1 && (size_t)b->warps * per_warp > (size_t)max_smem) b->warps /= 2;
@@ -417,7 +539,7 @@ int mgr_batch_set_tuning(MgrBatch* batch, int min_blocks_per_sm, int warps_per_b
     if (warps_per_block) {
         int max_smem = 0;
         cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, batch->device);
-        if ((size_t)warps_per_block * batch_warp_bytes(batch->cap, batch->L_max) > (size_t)max_smem) {
+        if ((size_t)warps_per_block * batch_need_bytes(batch) > (size_t)max_smem) {
             set_error("mgr_batch_set_tuning: that many warps do not fit in shared memory");
             return MGR_ERR_CAPACITY;
         }

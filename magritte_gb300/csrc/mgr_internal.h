@@ -180,6 +180,10 @@ cudaError_t launch_nint_table(MgrModel* model);
 cudaError_t launch_hl_tables(MgrModel* model);  // trace filter tables (edge_hl, pos_hl)
 cudaError_t launch_edge_pack(MgrModel* model, const double4_32a* pos, const uint32_t* nbr, uint64_t E,
                              double4_32a* edge);
+// The staged solve (mgr_staged.cuh): whether it serves the model, and its lane plan.
+struct StagedPlan;
+bool staged_ok(const MgrModel* model);
+StagedPlan staged_plan(const DevModel& m);
 // Fills the correctly rounded erff table (kErfBandCount floats) and the erf node table
 // (kErfNodes entries) on `stream`.
 cudaError_t fill_erf_band(float* table, float4* nodes, cudaStream_t stream, int sm_count);
