@@ -294,9 +294,14 @@ __device__ __forceinline__ int warp_next_point_f32(const DevModel& m, const Trac
 }
 
 // The walk of trace_half in 1D spherical symmetry (Geometry::get_next_spherical_symmetry,
-// geometry.tpp:118-159): every lane steps the same shells; lane 0 stores the steps, with
-// each step's shift at its distance along the ray (get_shift_spherical_symmetry) and the
-// half's origin shift (shift0, not 1 in the comoving frame there).
+// geometry.tpp:118-159, next_point_sph), with each step's shift at its distance along the
+// ray (get_shift_spherical_symmetry) and the half's origin shift (shift0, not 1 in the
+// comoving frame there).  The shells ahead are known before the steps are taken, so the
+// lanes form the distances of the next 32 shells from the ray's closest approach (a square
+// root each) side by side, the warp chains Z over them in the reference's order (three FP64
+// instructions a step), and the lanes then evaluate one step's shift each.  Every lane
+// stepping the shells by itself took some 45 FP64 warp instructions a step (200 shells, 25
+// ray pairs: 1439 us for the walks alone).
 template <bool STORE, int FRAME, int LAY = LAY_FULL>
 __device__ int trace_half_sph(const DevModel& m, uint32_t o, uint32_t r, uint32_t cap, HalfSmem& h, int lane,
                               int* status) {
@@ -304,6 +309,7 @@ __device__ int trace_half_sph(const DevModel& m, uint32_t o, uint32_t r, uint32_
     const double4_32a po = m.pos[o];
     const double Rcos = dot3_rn(po.x, po.y, po.z, d[0], d[1], d[2]);
     const double Rsin2 = dsub_rn(sqnorm_rn(po), dmul_rn(Rcos, Rcos));
+    const unsigned long long tangent = dkey(-Rcos);
     if (STORE) {
         h.shift0 = origin_shift(m, FRAME, o, r);
         set_dsh0(h, h.shift0);
@@ -311,30 +317,67 @@ __device__ int trace_half_sph(const DevModel& m, uint32_t o, uint32_t r, uint32_
     double Z = 0.0;
     uint32_t crt = o;
     int count = 0;
-    while (true) {
-        uint32_t nxt;
-        double dZl;
-        if (!next_point_sph(m, Rcos, Rsin2, crt, Z, nxt, dZl)) {
-            if (count > 0 && lane == 0) atomicOr(status, ST_TRACE);
-            if (count > 0) count = -1;
-            break;
+    bool ended = false;
+    while (!ended) {
+        const bool inward = dkey(Z) < tangent;  // Z < -Rcos
+        const bool valid = inward ? crt >= 1u + (uint32_t)lane : (uint64_t)crt + 1u + (uint32_t)lane < m.P;
+        const uint32_t s = inward ? crt - 1u - (uint32_t)lane : crt + 1u + (uint32_t)lane;
+        double root = 0.0;
+        bool meets = false, bdy = false;
+        if (valid) {
+            const double q = sqnorm_rn(m.pos[s]);
+            meets = !inward || q >= Rsin2;
+            root = dsqrt_rn(dsub_rn(q, Rsin2));
+            if (inward) root = -root;
+            bdy = m.p2b[s] != m.P;
         }
-        if (STORE && (uint32_t)count >= cap) {
-            if (lane == 0) atomicOr(status, ST_CAPACITY);
-            count = -1;
-            break;
+        const unsigned have = __ballot_sync(FULL_MASK, valid);
+        const unsigned meet = __ballot_sync(FULL_MASK, meets);
+        const unsigned stop = __ballot_sync(FULL_MASK, bdy);
+        double myZ = 0.0, my_dZ = 0.0;
+        uint32_t my_nxt = 0, my_crt = 0;
+        const int base = count;
+#pragma unroll 1
+        for (int j = 0; j < 32 && !ended; j++) {
+            if ((dkey(Z) < tangent) != inward) break;
+            if (!((have >> j) & 1u)) {
+                // no shell further along: from the origin an empty half, later a trace error
+                if (count > 0 && lane == 0) atomicOr(status, ST_TRACE);
+                if (count > 0) count = -1;
+                ended = true;
+                break;
+            }
+            if (STORE && (uint32_t)count >= cap) {
+                if (lane == 0) atomicOr(status, ST_CAPACITY);
+                count = -1;
+                ended = true;
+                break;
+            }
+            const double RcZ = dadd_rn(Rcos, Z);
+            const bool across = !((meet >> j) & 1u);  // the tangent point: back to the same shell
+            const double rj = __shfl_sync(FULL_MASK, root, j);
+            const uint32_t nxt = across ? crt : (inward ? crt - 1u : crt + 1u);
+            const double dZl = across ? dmul_rn(-2.0, RcZ) : dsub_rn(rj, RcZ);
+            Z = dadd_rn(Z, dZl);
+            if (lane == j) {
+                myZ = Z;
+                my_dZ = dZl;
+                my_nxt = nxt;
+                my_crt = crt;
+            }
+            count++;
+            ended = across ? m.p2b[nxt] != m.P : ((stop >> j) & 1u) != 0u;
+            crt = nxt;
+            if (across) break;
         }
-        Z = dadd_rn(Z, dZl);
-        if (STORE && lane == 0) {
-            h.ids[count] = nxt;
-            h.eid[count] = sph_eid(crt, nxt);
-            store_shift<LAY>(h, count, shift_sph(m, FRAME, o, r, nxt, Z, d));
-            store_dz<LAY>(m, h, count, dZl);
-            if (LAY == LAY_FULL) h.dzs[count] = (float)dZl * m.dz_scale;
+        if (STORE && count > 0 && lane < count - base) {
+            const int k = base + lane;
+            h.ids[k] = my_nxt;
+            h.eid[k] = sph_eid(my_crt, my_nxt);
+            store_shift<LAY>(h, k, shift_sph(m, FRAME, o, r, my_nxt, myZ, d));
+            store_dz<LAY>(m, h, k, my_dZ);
+            if (LAY == LAY_FULL) h.dzs[k] = (float)my_dZ * m.dz_scale;
         }
-        count++;
-        if (m.p2b[nxt] != m.P) break;
-        crt = nxt;
     }
     __syncwarp();
     return count;
