@@ -207,18 +207,19 @@ __global__ void __launch_bounds__(256, MINB)
         const DevModel& m = *desc;
         const uint64_t item = (g - group_off[mi]) * plan.K, n_items = (uint64_t)m.P * m.hnrays;
         if (item == 0 && lane == 0) tstamp[2 * mi] = global_ns();
+        const uint32_t o_first = (uint32_t)(item / m.hnrays), rr_first = (uint32_t)(item % m.hnrays);
         for (uint32_t j = 0; j < plan.K; j++) {
             const bool live = item + j < n_items;
-            const uint32_t o = live ? (uint32_t)((item + j) / m.hnrays) : 0u;
-            const uint32_t rr = live ? (uint32_t)((item + j) % m.hnrays) : 0u;
+            const uint32_t o = live ? o_first + (rr_first + j) / m.hnrays : 0u;
+            const uint32_t rr = live ? (rr_first + j) % m.hnrays : 0u;
             // general geometry with shared rays (mgr_batch_create refuses the other kinds)
             staged_trace<MODE, 0>(m, o, rr, cap, mine + staged_tile_bytes(MODE, plan.W), j, lane, status, live);
         }
         __syncwarp();
         const size_t at = (size_t)(stage_off[mi] - s0);
-        staged_solve<MODE, AP>(m, sl, cap, plan, mine, item, 0u, m.hnrays, lane,
+        staged_solve<MODE, AP>(m, sl, cap, plan, mine, o_first, rr_first, m.hnrays, lane,
                                [&](uint32_t j, uint32_t o, uint32_t f, const LaneResult& r) {
-                                   const size_t k = at + ((size_t)((item + j) % m.hnrays) * m.P + o) * m.F + f;
+                                   const size_t k = at + ((size_t)((rr_first + j) % m.hnrays) * m.P + o) * m.F + f;
                                    U[k] = r.u;
                                    if (LD) LD[k] = r.solved ? r.Ldiag : 0.0;
                                    if (!isfinite(r.u)) atomicOr(status, ST_NONFINITE);

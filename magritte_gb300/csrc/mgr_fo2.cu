@@ -290,19 +290,20 @@ __global__ void __launch_bounds__(256, MINB)
     const uint64_t stride = (uint64_t)gridDim.x * nw * plan.K;
     for (uint64_t item = ((uint64_t)blockIdx.x * nw + w) * plan.K; item < n_items; item += stride) {
         bool any = false;
+        const uint32_t o_first = o_begin + (uint32_t)(item / nR), k_first = (uint32_t)(item % nR);
         for (uint32_t j = 0; j < plan.K; j++) {
             bool live = item + j < n_items;
-            const uint32_t o = live ? o_begin + (uint32_t)((item + j) / nR) : 0u;
-            const uint32_t rr = live ? rr0 + (uint32_t)((item + j) % nR) : 0u;
+            const uint32_t o = live ? o_first + (k_first + j) / nR : 0u;
+            const uint32_t rr = live ? rr0 + (k_first + j) % nR : 0u;
             if (live && cls && cls[(size_t)o * m.hnrays + rr] != cls_id) live = false;  // another class's launch
             staged_trace<MODE, GEO>(m, o, rr, cap, mine + staged_tile_bytes(MODE, plan.W), j, lane, status, live);
             any = any || live;
         }
         __syncwarp();
         if (!any) continue;
-        staged_solve<MODE, AP>(m, sl, cap, plan, mine, item, o_begin, nR, lane,
+        staged_solve<MODE, AP>(m, sl, cap, plan, mine, o_first, k_first, nR, lane,
                                [&](uint32_t j, uint32_t o, uint32_t f, const LaneResult& r) {
-                                   const size_t k = (size_t)((item + j) % nR);
+                                   const size_t k = (k_first + j) % nR;
                                    U[k * u_stride + (size_t)(o - u_o0) * m.F + f] = r.u;
                                    if (LD) LD[k * ld_stride + (size_t)(o - ld_o0) * m.F + f] = r.solved ? r.Ldiag : 0.0;
                                    if (!isfinite(r.u)) atomicOr(status, ST_NONFINITE);
