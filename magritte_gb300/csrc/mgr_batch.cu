@@ -37,13 +37,17 @@ struct MgrBatch {
     uint64_t* d_item_off = nullptr;        // [n + 1] first (origin, ray pair) item of each model
     uint64_t* d_stage_off = nullptr;       // [n + 1] first staging entry of each model (cumulative P R F)
     // staged solve (mgr_staged.cuh), when every model qualifies: each model's lane plan and ray
-    // capacity, the first group of K items of each model, and a warp's ray buffers per precision
+    // capacity, the first group of K items of each model, the byte offset of its half rays, a
+    // warp's tile per precision, and the ray memory of one wave
     bool staged = false;
     mgr::StagedPlan* d_plans = nullptr;    // [n]
     uint32_t* d_caps = nullptr;            // [n] longest half ray of each model
     uint64_t* d_group_off = nullptr;       // [n + 1]
-    size_t staged_bytes[2] = {0, 0};       // FP64, split
-    std::vector<uint64_t> group_off;
+    size_t staged_bytes[2] = {0, 0};       // by precision mode
+    std::vector<uint64_t> group_off, ray_off;
+    uint64_t* d_ray_off = nullptr;         // [n + 1]
+    unsigned char* rays = nullptr;
+    uint64_t ray_bytes = 0;
     std::vector<uint64_t> item_off, stage_off, origin_off;  // host copies
     double* stage_u = nullptr;             // staging of u for one wave
     double* stage_ld = nullptr;            // staging of L_diag for one wave
@@ -63,6 +67,9 @@ namespace mgr {
 // Staged u (and L_diag) entries of one wave at most: 512 Mi doubles (4 GiB each) or,
 // when larger, the biggest single model.
 constexpr uint64_t kBatchStageEntries = uint64_t(1) << 29;
+
+// Ray memory of one wave of the staged solve at most (or the biggest single model's).
+constexpr uint64_t kBatchRayBytes = uint64_t(1) << 32;
 
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
@@ -100,7 +107,7 @@ __host__ __device__ inline size_t batch_warp_bytes(uint32_t cap, uint32_t L_max)
 // A warp's shared memory, the larger of the two precisions'.
 static size_t batch_need_bytes(const MgrBatch* b) {
     if (!b->staged) return batch_warp_bytes(b->cap, b->L_max);
-    return batch_head_bytes(b->L_max) + std::max(b->staged_bytes[0], b->staged_bytes[1]);
+    return kDescBytes + std::max(b->staged_bytes[0], b->staged_bytes[1]);
 }
 
 __device__ __forceinline__ void copy_desc(const DevModel* __restrict__ src, DevModel* dst, int t, int nt) {
@@ -168,23 +175,54 @@ __global__ void __launch_bounds__(256, MINB)
     }
 }
 
-// Stage 1, staged (mgr_staged.cuh): one warp per K consecutive items of a model.
+// Staged solve (mgr_staged.cuh): half rays of every (model, origin, ray pair), a warp each.
+template <int MODE>
+__global__ void __launch_bounds__(256)
+    trace_multi_kernel(const DevModel* __restrict__ models, const uint32_t* __restrict__ caps, uint32_t m0, uint32_t m1,
+                       const uint64_t* __restrict__ item_off, const uint64_t* __restrict__ ray_off,
+                       unsigned char* __restrict__ rays, unsigned long long* __restrict__ tstamp, uint32_t n_models,
+                       int* status) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int lane = threadIdx.x & 31;
+    DevModel* desc = reinterpret_cast<DevModel*>(smem + (size_t)(threadIdx.x >> 5) * kDescBytes);
+    if (threadIdx.x == 0) atomicMin(&tstamp[2 * n_models], global_ns());
+    const uint64_t i0 = item_off[m0], n = (item_off[m1] - i0) * 2;
+    const uint64_t stride = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    uint32_t mi = m0, desc_mi = 0xffffffffu;
+    for (uint64_t k = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < n; k += stride) {
+        const uint64_t item = i0 + (k >> 1);
+        while (item_off[mi + 1] <= item) mi++;  // items only grow within a warp
+        if (mi != desc_mi) {
+            __syncwarp();
+            copy_desc(models + mi, desc, lane, 32);
+            desc_mi = mi;
+            __syncwarp();
+        }
+        const uint64_t at = item - item_off[mi];
+        if (at == 0 && (k & 1u) == 0 && lane == 0) tstamp[2 * mi] = global_ns();
+        const uint32_t cap = caps[mi];
+        // general geometry with shared rays (mgr_batch_create refuses the other kinds)
+        staged_trace<MODE, 0>(*desc, (uint32_t)(at / desc->hnrays), (uint32_t)(at % desc->hnrays), (int)(k & 1u), cap,
+                              rays + (ray_off[mi] - ray_off[m0]) + (2 * at + (k & 1u)) * staged_half_bytes(MODE, cap),
+                              lane, status);
+    }
+}
+
+// Stage 1, staged: one warp per K consecutive items of a model.
 template <int MODE, int AP, int MINB>
 __global__ void __launch_bounds__(256, MINB)
     fo2_multi_staged_kernel(const DevModel* __restrict__ models, const StagedPlan* __restrict__ plans,
                             const uint32_t* __restrict__ caps, uint32_t m0, uint32_t m1,
                             const uint64_t* __restrict__ group_off, const uint64_t* __restrict__ stage_off,
-                            uint32_t warp_bytes, uint32_t L_max, double* __restrict__ U, double* __restrict__ LD,
-                            unsigned long long* __restrict__ tstamp, uint32_t n_models, int* status) {
+                            const uint64_t* __restrict__ ray_off, unsigned char* __restrict__ rays, uint32_t warp_bytes,
+                            double* __restrict__ U, double* __restrict__ LD, int* status) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int nw = blockDim.x >> 5;
     const int w = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    unsigned char* base = smem + (size_t)w * (batch_head_bytes(L_max) + warp_bytes);
+    unsigned char* base = smem + (size_t)w * (kDescBytes + warp_bytes);
     DevModel* desc = reinterpret_cast<DevModel*>(base);
-    double* sl = reinterpret_cast<double*>(base + kDescBytes);
-    unsigned char* mine = base + batch_head_bytes(L_max);
-    if (threadIdx.x == 0) atomicMin(&tstamp[2 * n_models], global_ns());
+    unsigned char* mine = base + kDescBytes;
 
     const uint64_t g0 = group_off[m0], g1 = group_off[m1];
     const uint64_t s0 = stage_off[m0];
@@ -197,8 +235,6 @@ __global__ void __launch_bounds__(256, MINB)
         if (mi != desc_mi) {
             __syncwarp();
             copy_desc(models + mi, desc, lane, 32);
-            __syncwarp();
-            for (uint32_t i = lane; i < desc->L; i += 32) sl[i] = desc->sorted_line[i];
             plan = plans[mi];
             cap = caps[mi];
             desc_mi = mi;
@@ -206,18 +242,12 @@ __global__ void __launch_bounds__(256, MINB)
         }
         const DevModel& m = *desc;
         const uint64_t item = (g - group_off[mi]) * plan.K, n_items = (uint64_t)m.P * m.hnrays;
-        if (item == 0 && lane == 0) tstamp[2 * mi] = global_ns();
         const uint32_t o_first = (uint32_t)(item / m.hnrays), rr_first = (uint32_t)(item % m.hnrays);
-        for (uint32_t j = 0; j < plan.K; j++) {
-            const bool live = item + j < n_items;
-            const uint32_t o = live ? o_first + (rr_first + j) / m.hnrays : 0u;
-            const uint32_t rr = live ? (rr_first + j) % m.hnrays : 0u;
-            // general geometry with shared rays (mgr_batch_create refuses the other kinds)
-            staged_trace<MODE, 0>(m, o, rr, cap, mine + staged_tile_bytes(MODE, plan.W), j, lane, status, live);
-        }
-        __syncwarp();
+        const uint32_t live = (uint32_t)(n_items - item < plan.K ? n_items - item : plan.K);
         const size_t at = (size_t)(stage_off[mi] - s0);
-        staged_solve<MODE, AP>(m, sl, cap, plan, mine, o_first, rr_first, m.hnrays, lane,
+        staged_solve<MODE, AP>(m, m.sorted_line, cap, plan, mine,
+                               rays + (ray_off[mi] - ray_off[m0]) + 2 * item * staged_half_bytes(MODE, cap), live,
+                               o_first, rr_first, m.hnrays, lane,
                                [&](uint32_t j, uint32_t o, uint32_t f, const LaneResult& r) {
                                    const size_t k = at + ((size_t)((rr_first + j) % m.hnrays) * m.P + o) * m.F + f;
                                    U[k] = r.u;
@@ -293,15 +323,23 @@ static cudaError_t launch_multi_variant(MgrBatch* b, uint32_t m0, uint32_t m1, b
     unsigned grid = 1;
     cudaError_t e;
     if (b->staged) {
-        const size_t bytes = b->staged_bytes[MODE == MODE_SPLIT ? 1 : 0];
-        const size_t smem = (size_t)nw * (batch_head_bytes(b->L_max) + bytes);
+        const uint64_t halves = 2 * (b->item_off[m1] - b->item_off[m0]);
+        auto tr = trace_multi_kernel<MODE>;
+        e = multi_grid(tr, 8, 8 * kDescBytes, sms, halves, &grid);
+        if (e != cudaSuccess) return e;
+        count_launch();
+        tr<<<grid, 256, 8 * kDescBytes, b->stream>>>(b->d_models, b->d_caps, m0, m1, b->d_item_off, b->d_ray_off,
+                                                     b->rays, b->d_t, n, b->status);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        const size_t bytes = b->staged_bytes[MODE];
+        const size_t smem = (size_t)nw * (kDescBytes + bytes);
         auto kern = fo2_multi_staged_kernel<MODE, AP, MINB>;
         e = multi_grid(kern, nw, smem, sms, b->group_off[m1] - b->group_off[m0], &grid);
         if (e != cudaSuccess) return e;
         count_launch();
         kern<<<grid, nw * 32, smem, b->stream>>>(b->d_models, b->d_plans, b->d_caps, m0, m1, b->d_group_off,
-                                                 b->d_stage_off, (uint32_t)bytes, b->L_max, b->stage_u,
-                                                 want_lam ? b->stage_ld : nullptr, b->d_t, n, b->status);
+                                                 b->d_stage_off, b->d_ray_off, b->rays, (uint32_t)bytes, b->stage_u,
+                                                 want_lam ? b->stage_ld : nullptr, b->status);
     } else {
         const size_t smem = (size_t)nw * batch_warp_bytes(b->cap, b->L_max);
         auto kern = fo2_multi_kernel<MODE, AP, MINB>;
@@ -332,7 +370,9 @@ static cudaError_t launch_batch_variant(MgrBatch* b, bool want_lam) {
     uint32_t m0 = 0;
     while (m0 < n) {
         uint32_t m1 = m0 + 1;
-        while (m1 < n && b->stage_off[m1 + 1] - b->stage_off[m0] <= b->stage_entries) m1++;
+        while (m1 < n && b->stage_off[m1 + 1] - b->stage_off[m0] <= b->stage_entries &&
+               (!b->staged || b->ray_off[m1 + 1] - b->ray_off[m0] <= b->ray_bytes))
+            m1++;
         cudaError_t e = launch_multi_variant<MODE, AP, MINB>(b, m0, m1, want_lam);
         if (e != cudaSuccess) return e;
         m0 = m1;
@@ -366,6 +406,8 @@ static void batch_release(MgrBatch* b) {
     cudaFree(b->d_plans);
     cudaFree(b->d_caps);
     cudaFree(b->d_group_off);
+    cudaFree(b->d_ray_off);
+    cudaFree(b->rays);
     cudaFree(b->stage_u);
     cudaFree(b->stage_ld);
     cudaFree(b->d_J);
@@ -452,23 +494,27 @@ int mgr_batch_create(MgrModel* const* models, uint32_t n_models, MgrBatch** out)
         stage_off[i + 1] = stage_off[i] + entries;
         largest = std::max(largest, entries);
     }
-    // the staged solve when every model qualifies and a warp's ray buffers are no larger than
-    // the general kernel's (they hold K ray pairs of the model's own longest ray)
+    // the staged solve when every model qualifies
     std::vector<StagedPlan> plans(n_models);
     std::vector<uint32_t> caps(n_models);
     b->group_off.assign(n_models + 1, 0);
+    b->ray_off.assign(n_models + 1, 0);
     b->staged = true;
+    uint64_t largest_rays = 1;
     for (uint32_t i = 0; i < n_models; i++) {
         const MgrModel* m = models[i];
         b->staged = b->staged && staged_ok(m);
         plans[i] = staged_plan(m->dm);
         caps[i] = m->half_cap;
         b->group_off[i + 1] = b->group_off[i] + ((uint64_t)m->dm.P * m->dm.hnrays + plans[i].K - 1) / plans[i].K;
-        b->staged_bytes[0] =
-            std::max(b->staged_bytes[0], staged_warp_bytes(MODE_FP64, caps[i], plans[i].K, plans[i].W));
-        b->staged_bytes[1] =
-            std::max(b->staged_bytes[1], staged_warp_bytes(MODE_SPLIT, caps[i], plans[i].K, plans[i].W));
+        // either precision's layout
+        const uint64_t bytes = (uint64_t)m->dm.P * staged_origin_bytes(MODE_FP64, caps[i], m->dm.hnrays);
+        b->ray_off[i + 1] = b->ray_off[i] + bytes;
+        largest_rays = std::max(largest_rays, bytes);
+        for (int mode : {MODE_FP64, MODE_SPLIT})
+            b->staged_bytes[mode] = std::max(b->staged_bytes[mode], (size_t)staged_tile_bytes(mode, plans[i].W));
     }
+    b->ray_bytes = b->staged ? std::min(b->ray_off[n_models], std::max(kBatchRayBytes, largest_rays)) : 0;
     b->n_items = offsets[n_models];
     b->origin_off = offsets;
     b->item_off = item_off;
@@ -489,6 +535,10 @@ int mgr_batch_create(MgrModel* const* models, uint32_t n_models, MgrBatch** out)
     if (e == cudaSuccess) e = cudaMemcpy(b->d_caps, caps.data(), n_models * sizeof(uint32_t), cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
         e = cudaMemcpy(b->d_group_off, b->group_off.data(), (n_models + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_ray_off, (n_models + 1) * sizeof(uint64_t));
+    if (e == cudaSuccess)
+        e = cudaMemcpy(b->d_ray_off, b->ray_off.data(), (n_models + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && b->ray_bytes) e = cudaMalloc(&b->rays, b->ray_bytes);
     if (e == cudaSuccess) e = cudaMalloc(&b->stage_u, b->stage_entries * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&b->stage_ld, b->stage_entries * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_J, n_models * sizeof(double*));

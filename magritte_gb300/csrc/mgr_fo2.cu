@@ -267,41 +267,41 @@ __global__ void __launch_bounds__(256, MINB)
 }
 
 // ---------------------------------------------------------------------------------
-// Formal solve, stage 1, staged (mgr_staged.cuh): one warp per K consecutive (origin, ray
-// pair) items, results as fo2_kernel's.
+// Formal solve, stage 1, staged (mgr_staged.cuh).  trace_rays_kernel: a warp per half ray of
+// the origins' pairs, slot 2 ((o - o_begin) nR + rr - rr0) + side.  fo2_staged_kernel: a warp
+// per K consecutive (origin, ray pair) items, results as fo2_kernel's.
 // ---------------------------------------------------------------------------------
-template <int MODE, int AP, int MINB, int GEO>
+template <int MODE, int GEO>
+__global__ void __launch_bounds__(256) trace_rays_kernel(const __grid_constant__ DevModel m, uint32_t cap,
+                                                         uint32_t o_begin, uint32_t rr0, uint32_t nR, uint64_t n_halves,
+                                                         unsigned char* __restrict__ rays, int* status) {
+    const int lane = threadIdx.x & 31;
+    const uint64_t k = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (k >= n_halves) return;
+    const uint64_t item = k >> 1;
+    staged_trace<MODE, GEO>(m, o_begin + (uint32_t)(item / nR), rr0 + (uint32_t)(item % nR), (int)(k & 1u), cap,
+                            rays + (size_t)k * staged_half_bytes(MODE, cap), lane, status);
+}
+
+template <int MODE, int AP, int MINB>
 __global__ void __launch_bounds__(256, MINB)
     fo2_staged_kernel(const __grid_constant__ DevModel m, uint32_t cap, StagedPlan plan, uint32_t o_begin,
-                      uint32_t o_end, uint32_t rr0, uint32_t nR, double* __restrict__ U, size_t u_stride, uint32_t u_o0,
-                      double* __restrict__ LD, size_t ld_stride, uint32_t ld_o0, const uint8_t* __restrict__ cls,
-                      uint32_t cls_id, int* status) {
+                      uint32_t o_end, uint32_t nR, unsigned char* __restrict__ rays, double* __restrict__ U,
+                      size_t u_stride, uint32_t u_o0, double* __restrict__ LD, size_t ld_stride, uint32_t ld_o0,
+                      int* status) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int nw = blockDim.x >> 5;
     const int w = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    double* sl = reinterpret_cast<double*>(smem);
-    const uint32_t Lpad = (m.L + 1) & ~1u;
-    unsigned char* mine = smem + (size_t)Lpad * 8 + (size_t)w * staged_warp_bytes(MODE, cap, plan.K, plan.W);
-    for (uint32_t i = threadIdx.x; i < m.L; i += blockDim.x) sl[i] = m.sorted_line[i];
-    __syncthreads();
+    unsigned char* mine = smem + (size_t)w * staged_tile_bytes(MODE, plan.W);
 
     const uint64_t n_items = (uint64_t)(o_end - o_begin) * nR;
     const uint64_t stride = (uint64_t)gridDim.x * nw * plan.K;
     for (uint64_t item = ((uint64_t)blockIdx.x * nw + w) * plan.K; item < n_items; item += stride) {
-        bool any = false;
         const uint32_t o_first = o_begin + (uint32_t)(item / nR), k_first = (uint32_t)(item % nR);
-        for (uint32_t j = 0; j < plan.K; j++) {
-            bool live = item + j < n_items;
-            const uint32_t o = live ? o_first + (k_first + j) / nR : 0u;
-            const uint32_t rr = live ? rr0 + (k_first + j) % nR : 0u;
-            if (live && cls && cls[(size_t)o * m.hnrays + rr] != cls_id) live = false;  // another class's launch
-            staged_trace<MODE, GEO>(m, o, rr, cap, mine + staged_tile_bytes(MODE, plan.W), j, lane, status, live);
-            any = any || live;
-        }
-        __syncwarp();
-        if (!any) continue;
-        staged_solve<MODE, AP>(m, sl, cap, plan, mine, o_first, k_first, nR, lane,
+        const uint32_t live = (uint32_t)(n_items - item < plan.K ? n_items - item : plan.K);
+        staged_solve<MODE, AP>(m, m.sorted_line, cap, plan, mine, rays + 2 * item * staged_half_bytes(MODE, cap), live,
+                               o_first, k_first, nR, lane,
                                [&](uint32_t j, uint32_t o, uint32_t f, const LaneResult& r) {
                                    const size_t k = (k_first + j) % nR;
                                    U[k * u_stride + (size_t)(o - u_o0) * m.F + f] = r.u;
@@ -700,14 +700,17 @@ static size_t fo2_bytes_per_origin(const MgrModel* model) {
     return (size_t)model->dm.hnrays * model->dm.F * sizeof(double);
 }
 
+static size_t fo2_ray_bytes(const MgrModel* model, uint32_t nR);
+
 size_t fo2_work_bytes(const MgrModel* model, uint32_t n_origins, bool stage_u, bool stage_ld) {
     const int k = (stage_u ? 1 : 0) + (stage_ld ? 1 : 0);
-    if (k == 0 || n_origins == 0) return 0;
-    const size_t per = fo2_bytes_per_origin(model) * k;
+    const size_t rays = staged_ok(model) ? fo2_ray_bytes(model, model->dm.hnrays) : 0;
+    if ((k == 0 && rays == 0) || n_origins == 0) return 0;
+    const size_t per = fo2_bytes_per_origin(model) * k + rays;
     size_t chunk = kFo2WorkBudget / per;
     if (chunk < 1) chunk = 1;
     if (chunk > n_origins) chunk = n_origins;
-    return chunk * per;
+    return chunk * per + 16;
 }
 
 // Whether the staged solve serves this model: its tiles hold one line's data, so the
@@ -750,24 +753,27 @@ StagedPlan staged_plan(const DevModel& m) {
     return best;
 }
 
-template <int MODE, int AP, int MINB, int GEO>
-static cudaError_t launch_staged_variant(MgrModel* model, uint32_t o_begin, uint32_t o_end, uint32_t rr0, uint32_t nR,
-                                         double* U, size_t us, uint32_t uo, double* LD, size_t ls, uint32_t lo,
-                                         const uint8_t* cls, uint32_t cls_id) {
+// Ray memory of one origin for the staged solve, in either precision's layout.
+static size_t fo2_ray_bytes(const MgrModel* model, uint32_t nR) {
+    return staged_origin_bytes(MODE_FP64, model->half_cap, nR);
+}
+
+template <int MODE, int AP, int MINB>
+static cudaError_t launch_staged_variant(MgrModel* model, uint32_t o_begin, uint32_t o_end, uint32_t nR,
+                                         unsigned char* rays, double* U, size_t us, uint32_t uo, double* LD, size_t ls,
+                                         uint32_t lo) {
     const DevModel& m = model->dm;
-    const uint32_t cap = cls ? model->class_cap[cls_id] : model->half_cap;
     int nw = (MODE == MODE_SPLIT) ? model->fo2_warps_split : model->fo2_warps_fp64;
     if (nw < 1 || nw > 8) nw = 8;
-    StagedPlan plan = staged_plan(m);
-    const uint32_t Lpad = (m.L + 1) & ~1u;
-    size_t smem = (size_t)Lpad * 8 + (size_t)nw * staged_warp_bytes(MODE, cap, plan.K, plan.W);
-    auto kern = fo2_staged_kernel<MODE, AP, MINB, GEO>;
+    const StagedPlan plan = staged_plan(m);
+    const size_t smem = (size_t)nw * staged_tile_bytes(MODE, plan.W);
+    auto kern = fo2_staged_kernel<MODE, AP, MINB>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nw * 32, smem);
     if (e != cudaSuccess) return e;
-    if (per_sm < 1) return cudaErrorInvalidConfiguration;  // the ray buffers do not fit in shared memory
+    if (per_sm < 1) return cudaErrorInvalidConfiguration;
     const uint64_t items = (uint64_t)(o_end - o_begin) * nR;
     uint64_t grid = (uint64_t)model->sm_count * per_sm;
     const uint64_t per_block = (uint64_t)nw * plan.K;
@@ -775,9 +781,35 @@ static cudaError_t launch_staged_variant(MgrModel* model, uint32_t o_begin, uint
     if (grid > need) grid = need;
     if (grid < 1) grid = 1;
     count_launch();
-    kern<<<(unsigned)grid, nw * 32, smem, model->stream>>>(m, cap, plan, o_begin, o_end, rr0, nR, U, us, uo, LD, ls, lo,
-                                                          cls, cls_id, model->status);
+    kern<<<(unsigned)grid, nw * 32, smem, model->stream>>>(m, model->half_cap, plan, o_begin, o_end, nR, rays, U, us, uo,
+                                                          LD, ls, lo, model->status);
     return cudaGetLastError();
+}
+
+template <int MODE>
+static cudaError_t launch_trace_rays(MgrModel* model, uint32_t o_begin, uint32_t o_end, uint32_t rr0, uint32_t nR,
+                                     unsigned char* rays) {
+    const DevModel& m = model->dm;
+    const uint64_t halves = (uint64_t)(o_end - o_begin) * nR * 2;
+    auto kern = (m.sph || m.adaptive) ? trace_rays_kernel<MODE, 1> : trace_rays_kernel<MODE, 0>;
+    count_launch();
+    kern<<<(unsigned)((halves + 7) / 8), 256, 0, model->stream>>>(m, model->half_cap, o_begin, rr0, nR, halves, rays,
+                                                                  model->status);
+    return cudaGetLastError();
+}
+
+// Walks and solves origins [o_begin, o_end) x ray pairs [rr0, rr0 + nR) with the half rays in
+// `rays` (fo2_ray_bytes per origin).
+template <int MODE, int AP>
+static cudaError_t launch_staged(MgrModel* model, uint32_t o_begin, uint32_t o_end, uint32_t rr0, uint32_t nR,
+                                 unsigned char* rays, double* U, size_t us, uint32_t uo, double* LD, size_t ls,
+                                 uint32_t lo) {
+    const cudaError_t e = launch_trace_rays<MODE>(model, o_begin, o_end, rr0, nR, rays);
+    if (e != cudaSuccess) return e;
+    const int minb = (MODE == MODE_SPLIT) ? model->fo2_minb_split : model->fo2_minb_fp64;
+    if (minb == 2) return launch_staged_variant<MODE, AP, 2>(model, o_begin, o_end, nR, rays, U, us, uo, LD, ls, lo);
+    if (minb == 4) return launch_staged_variant<MODE, AP, 4>(model, o_begin, o_end, nR, rays, U, us, uo, LD, ls, lo);
+    return launch_staged_variant<MODE, AP, 3>(model, o_begin, o_end, nR, rays, U, us, uo, LD, ls, lo);
 }
 
 // One launch of fo2_kernel over origins [o_begin, o_end) x ray pairs [rr0, rr0 + nR):
@@ -820,24 +852,15 @@ static cudaError_t launch_fo2_variant(MgrModel* model, uint32_t o_begin, uint32_
 // were 4 % slower).
 template <int MODE, int AP>
 static cudaError_t launch_fo2_minb(MgrModel* model, uint32_t o_begin, uint32_t o_end, uint32_t rr0, uint32_t nR,
-                                   double* U, size_t us, uint32_t uo, double* LD, size_t ls, uint32_t lo) {
+                                   unsigned char* rays, double* U, size_t us, uint32_t uo, double* LD, size_t ls,
+                                   uint32_t lo) {
+    if (rays) return launch_staged<MODE, AP>(model, o_begin, o_end, rr0, nR, rays, U, us, uo, LD, ls, lo);
     const int minb = (MODE == MODE_SPLIT) ? model->fo2_minb_split : model->fo2_minb_fp64;
     const bool any_geo = model->dm.sph || model->dm.adaptive;
     const uint8_t* cls = model->half_cap > kLenClassBound[2] ? model->pair_class : nullptr;
     for (int c = 0; c < (cls ? kLenClasses : 1); c++) {
         if (cls && model->class_cap[c] == 0) continue;
         cudaError_t e;
-        if (staged_ok(model)) {
-            if (any_geo) e = launch_staged_variant<MODE, AP, 3, 1>(model, o_begin, o_end, rr0, nR, U, us, uo, LD, ls, lo, cls, c);
-            else if (minb == 2)
-                e = launch_staged_variant<MODE, AP, 2, 0>(model, o_begin, o_end, rr0, nR, U, us, uo, LD, ls, lo, cls, c);
-            else if (minb == 4)
-                e = launch_staged_variant<MODE, AP, 4, 0>(model, o_begin, o_end, rr0, nR, U, us, uo, LD, ls, lo, cls, c);
-            else
-                e = launch_staged_variant<MODE, AP, 3, 0>(model, o_begin, o_end, rr0, nR, U, us, uo, LD, ls, lo, cls, c);
-            if (e != cudaSuccess) return e;
-            continue;
-        }
         // spherical symmetry and adaptive rays: the run-time geometry variant, one tile
         if (any_geo) e = launch_fo2_variant<MODE, AP, 3, false, 1>(model, o_begin, o_end, rr0, nR, U, us, uo, LD, ls, lo,
                                                                   nullptr, cls, c);
@@ -871,13 +894,14 @@ static cudaError_t launch_fo2_uv(MgrModel* model, uint32_t o_begin, uint32_t o_e
 
 template <int MODE>
 static cudaError_t launch_fo2_approx(MgrModel* model, uint32_t o_begin, uint32_t o_end, uint32_t rr0, uint32_t nR,
-                                     double* U, size_t us, uint32_t uo, double* LD, size_t ls, uint32_t lo) {
+                                     unsigned char* rays, double* U, size_t us, uint32_t uo, double* LD, size_t ls,
+                                     uint32_t lo) {
     switch (model->dm.approx) {
         case APPROX_ONELINE:
-            return launch_fo2_minb<MODE, APPROX_ONELINE>(model, o_begin, o_end, rr0, nR, U, us, uo, LD, ls, lo);
+            return launch_fo2_minb<MODE, APPROX_ONELINE>(model, o_begin, o_end, rr0, nR, rays, U, us, uo, LD, ls, lo);
         case APPROX_CLOSELINES:
-            return launch_fo2_minb<MODE, APPROX_CLOSELINES>(model, o_begin, o_end, rr0, nR, U, us, uo, LD, ls, lo);
-        default: return launch_fo2_minb<MODE, APPROX_NONE>(model, o_begin, o_end, rr0, nR, U, us, uo, LD, ls, lo);
+            return launch_fo2_minb<MODE, APPROX_CLOSELINES>(model, o_begin, o_end, rr0, nR, rays, U, us, uo, LD, ls, lo);
+        default: return launch_fo2_minb<MODE, APPROX_NONE>(model, o_begin, o_end, rr0, nR, rays, U, us, uo, LD, ls, lo);
     }
 }
 
@@ -949,7 +973,19 @@ cudaError_t launch_fo2_range(MgrModel* model, int precision, uint32_t o_begin, u
     const int k = (u ? 0 : 1) + (lam ? 1 : 0);
     const size_t per = fo2_bytes_per_origin(model);
     uint32_t chunk = o_end - o_begin;
-    if (k) {
+    // the staged solve where the work area takes the half rays of enough origins to fill the
+    // GPU (or of all of them); the general kernel traces into shared memory
+    bool staged = work && !v && !alo_off && staged_ok(model);
+    if (staged) {
+        const size_t fit = work_bytes > 16 ? (work_bytes - 16) / (per * k + fo2_ray_bytes(model, m.hnrays)) : 0;
+        if (fit >= chunk) {
+        } else if (fit * nR >= (uint64_t)model->sm_count * 32) {
+            chunk = (uint32_t)fit;
+        } else {
+            staged = false;
+        }
+    }
+    if (k && !staged) {
         const size_t fit = work ? work_bytes / (per * k) : 0;
         if (fit < 1) return cudaErrorInvalidValue;  // caller sizes the work area with fo2_work_bytes
         if (fit < chunk) chunk = (uint32_t)fit;
@@ -974,6 +1010,11 @@ cudaError_t launch_fo2_range(MgrModel* model, int precision, uint32_t o_begin, u
         }
         double* LD = lam ? next : nullptr;
         const size_t ls = (size_t)n * m.F;
+        unsigned char* rays = nullptr;
+        if (staged) {
+            double* end = next + (lam ? (size_t)nR * n * m.F : 0);
+            rays = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(end) + 15) & ~uintptr_t(15));
+        }
         cudaError_t e;
         if (alo_off)
             e = launch_fo2_alo(model, c0, c1, rr_begin, nR, U, us, uo, LD, ls, c0, alo_off, alo_nr);
@@ -983,8 +1024,8 @@ cudaError_t launch_fo2_range(MgrModel* model, int precision, uint32_t o_begin, u
                     : launch_fo2_uv<MODE_FP64>(model, c0, c1, rr_begin, nR, U, us, uo, LD, ls, c0, v);
         else
             e = (precision == MGR_PRECISION_SPLIT)
-                    ? launch_fo2_approx<MODE_SPLIT>(model, c0, c1, rr_begin, nR, U, us, uo, LD, ls, c0)
-                    : launch_fo2_approx<MODE_FP64>(model, c0, c1, rr_begin, nR, U, us, uo, LD, ls, c0);
+                    ? launch_fo2_approx<MODE_SPLIT>(model, c0, c1, rr_begin, nR, rays, U, us, uo, LD, ls, c0)
+                    : launch_fo2_approx<MODE_FP64>(model, c0, c1, rr_begin, nR, rays, U, us, uo, LD, ls, c0);
         if (e != cudaSuccess) return e;
         if (!J && !lam && !Jlin && !anis) continue;  // u (and v) only
         unsigned grid = n < (uint32_t)nsm * 16 ? n : (unsigned)nsm * 16;

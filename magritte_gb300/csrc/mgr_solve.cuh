@@ -412,14 +412,17 @@ __device__ int trace_half(const DevModel& m, uint32_t o, uint32_t r, uint32_t ca
         t.Zc = 0.0f;
         t.eZc = 0.0f;
     }
-    double Z = 0.0;  // exact Z after the last step whose Zn is known in FP64
-    // Steps chosen by the filter whose exact Zn and dZ are not computed yet: the last
-    // np steps; lane j holds the point of the j-th of them.
-    uint32_t pend = 0;
+    double Z = 0.0;  // exact Z after the last step that is not pending
+    // The last np steps are pending: lane j holds the point and edge of the j-th of them.
+    uint32_t pend = 0, pend_eid = 0;
     int np = 0;
     uint32_t crt = o;
     int count = 0;
-    // Exact Zn of the pending steps, one step per lane, then Z += Zn - Z in step order.
+    // Stores the pending steps, one step per lane: exact Zn, dZ, Doppler shift and the FP32
+    // copies.  Z after a step is the step's Zn unless Z + fl(Zn - Z) rounds away from it: the
+    // lanes take every step's distance from the previous Zn side by side, and the serial
+    // chain Z += Zn - Z runs only when one of the sums does not come back to its Zn (two
+    // FP64 warp instructions for up to 32 steps instead of two per step).
     auto flush = [&]() {
         if (np == 0) return;
         double Zn = 0.0;
@@ -427,11 +430,6 @@ __device__ int trace_half(const DevModel& m, uint32_t o, uint32_t r, uint32_t ca
             const double4_32a q = m.pos[pend];
             Zn = dot3_rn(dsub_rn(q.x, po.x), dsub_rn(q.y, po.y), dsub_rn(q.z, po.z), dx, dy, dz);
         }
-        const int base = count - np;
-        // Z after a step is the step's Zn unless Z + fl(Zn - Z) rounds away from it: take
-        // every step's distance from the previous Zn side by side, and the serial chain only
-        // when one of the sums does not come back to its Zn (two FP64 warp instructions for
-        // up to 32 steps instead of two per step).
         const double Zb = __shfl_up_sync(FULL_MASK, Zn, 1);
         const double Zprev = lane == 0 ? Z : Zb;
         double dz_lane = dsub_rn(Zn, Zprev);
@@ -439,33 +437,35 @@ __device__ int trace_half(const DevModel& m, uint32_t o, uint32_t r, uint32_t ca
         if (__all_sync(FULL_MASK, back || lane >= np)) {
             Z = __shfl_sync(FULL_MASK, Zn, np - 1);
         } else {
+#pragma unroll 1
             for (int j = 0; j < np; j++) {
                 const double dZl = dsub_rn(__shfl_sync(FULL_MASK, Zn, j), Z);
                 Z = dadd_rn(Z, dZl);
                 if (lane == j) dz_lane = dZl;
             }
         }
-        if (STORE && lane < np) store_dz<LAY>(m, h, base + lane, dz_lane);
+        if (STORE && lane < np) {
+            const int k = count - np + lane;
+            h.ids[k] = pend;
+            h.eid[k] = pend_eid;
+            store_dz<LAY>(m, h, k, dz_lane);
+            if (LAY == LAY_FULL) h.dzs[k] = (float)dz_lane * m.dz_scale;
+            store_shift<LAY>(h, k, FRAME ? shift_rest(m, r, pend, d) : shift_comoving(m, o, pend, d));
+        }
         np = 0;
     };
+#pragma unroll 1
     while (true) {
         uint32_t nxt = 0, eid = 0;
         float Zw = 0.0f, EZw = 0.0f;
         int found = (FILTER && m.edge_hl) ? warp_next_point_f32(m, t, crt, lane, nxt, eid, Zw, EZw) : -1;
-        bool exact = false;
-        double dZl = 0.0;
         if (found < 0) {
             flush();
             double bestZ;
             found = warp_next_point(m, po, dx, dy, dz, crt, Z, lane, nxt, bestZ, eid) ? 1 : 0;
-            if (found) {
-                exact = true;
-                dZl = dsub_rn(bestZ, Z);
-                Z = dadd_rn(Z, dZl);
-                if (FILTER) {
-                    Zw = (float)dmul_rn(Z, m.pos_scale);
-                    EZw = fmaf(2.0f * kU32, fabsf(Zw), 32.0f * kU32Sq);
-                }
+            if (FILTER && found) {
+                Zw = (float)dmul_rn(bestZ, m.pos_scale);
+                EZw = fmaf(2.0f * kU32, fabsf(Zw), 32.0f * kU32Sq);
             }
         }
         if (!found) {
@@ -481,15 +481,11 @@ __device__ int trace_half(const DevModel& m, uint32_t o, uint32_t r, uint32_t ca
             count = -1;
             break;
         }
-        if (STORE && lane == 0) {
-            h.ids[count] = nxt;
-            h.eid[count] = eid;
-            if (exact) store_dz<LAY>(m, h, count, dZl);
+        if (lane == np) {
+            pend = nxt;
+            pend_eid = eid;
         }
-        if (!exact) {
-            if (lane == np) pend = nxt;
-            np++;
-        }
+        np++;
         count++;
         if (FILTER) {
             t.Zc = Zw;
@@ -499,16 +495,8 @@ __device__ int trace_half(const DevModel& m, uint32_t o, uint32_t r, uint32_t ca
         if (m.p2b[nxt] != m.P) break;
         crt = nxt;
     }
-    if (count > 0) flush();
+    if (STORE && count > 0) flush();
     __syncwarp();
-    if (STORE && count > 0) {
-        // Per-step Doppler shifts and FP32 copies, one step per lane.
-        for (int s = lane; s < count; s += 32) {
-            store_shift<LAY>(h, s, FRAME ? shift_rest(m, r, h.ids[s], d) : shift_comoving(m, o, h.ids[s], d));
-            if (LAY == LAY_FULL) h.dzs[s] = (float)h.dZ[s] * m.dz_scale;
-        }
-        __syncwarp();
-    }
     return count;
 }
 
