@@ -48,6 +48,8 @@ struct MgrBatch {
     uint64_t* d_ray_off = nullptr;         // [n + 1]
     unsigned char* rays = nullptr;
     uint64_t ray_bytes = 0;
+    uint32_t* list = nullptr;              // ray pairs of a wave the staged solve gave up
+    size_t max_smem = 0;
     std::vector<uint64_t> item_off, stage_off, origin_off;  // host copies
     double* stage_u = nullptr;             // staging of u for one wave
     double* stage_ld = nullptr;            // staging of L_diag for one wave
@@ -122,8 +124,8 @@ template <int MODE, int AP, int MINB>
 __global__ void __launch_bounds__(256, MINB)
     fo2_multi_kernel(const DevModel* __restrict__ models, uint32_t m0, uint32_t m1,
                      const uint64_t* __restrict__ item_off, const uint64_t* __restrict__ stage_off, uint32_t cap,
-                     uint32_t L_max, double* __restrict__ U, double* __restrict__ LD,
-                     unsigned long long* __restrict__ tstamp, uint32_t n_models, int* status) {
+                     uint32_t L_max, const uint32_t* __restrict__ list, double* __restrict__ U,
+                     double* __restrict__ LD, unsigned long long* __restrict__ tstamp, uint32_t n_models, int* status) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int nw = blockDim.x >> 5;
     const int w = threadIdx.x >> 5;
@@ -135,11 +137,15 @@ __global__ void __launch_bounds__(256, MINB)
     carve_halves(base + batch_head_bytes(L_max), cap, bk, fw);
     if (threadIdx.x == 0) atomicMin(&tstamp[2 * n_models], global_ns());
 
-    const uint64_t i0 = item_off[m0], i1 = item_off[m1];
+    const uint64_t i0 = item_off[m0];
+    // list: only the items listed (list[0] of them, from list[1] on, counted from i0)
+    const uint64_t n = list ? (uint64_t)list[0] : item_off[m1] - i0;
     const uint64_t s0 = stage_off[m0];
     const uint64_t stride = (uint64_t)gridDim.x * nw;
     uint32_t mi = m0, desc_mi = 0xffffffffu;
-    for (uint64_t item = i0 + (uint64_t)blockIdx.x * nw + w; item < i1; item += stride) {
+    for (uint64_t q = (uint64_t)blockIdx.x * nw + w; q < n; q += stride) {
+        const uint64_t item = i0 + (list ? (uint64_t)list[1 + q] : q);
+        if (list) mi = model_of(item_off, m0, m1, item);
         // the item's model: items only grow within a warp
         while (item_off[mi + 1] <= item) mi++;
         if (mi != desc_mi) {
@@ -153,7 +159,7 @@ __global__ void __launch_bounds__(256, MINB)
         const uint64_t k = item - item_off[mi];
         const uint32_t o = (uint32_t)(k / m.hnrays);
         const uint32_t rr = (uint32_t)(k % m.hnrays);
-        if (k == 0 && lane == 0) tstamp[2 * mi] = global_ns();
+        if (k == 0 && lane == 0 && !list) tstamp[2 * mi] = global_ns();
         // general geometry with shared rays (mgr_batch_create refuses the other kinds)
         int nb = 0, nf = 0;
         trace_pair<true, 0, 0>(m, o, rr, m.antipod[rr], cap, bk, fw, lane, status, nb, nf);
@@ -214,7 +220,8 @@ __global__ void __launch_bounds__(256, MINB)
     fo2_multi_staged_kernel(const DevModel* __restrict__ models, const StagedPlan* __restrict__ plans,
                             const uint32_t* __restrict__ caps, uint32_t m0, uint32_t m1,
                             const uint64_t* __restrict__ group_off, const uint64_t* __restrict__ stage_off,
-                            const uint64_t* __restrict__ ray_off, unsigned char* __restrict__ rays, uint32_t warp_bytes,
+                            const uint64_t* __restrict__ ray_off, const uint64_t* __restrict__ item_off,
+                            unsigned char* __restrict__ rays, uint32_t* __restrict__ list, uint32_t warp_bytes,
                             double* __restrict__ U, double* __restrict__ LD, int* status) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int nw = blockDim.x >> 5;
@@ -245,15 +252,18 @@ __global__ void __launch_bounds__(256, MINB)
         const uint32_t o_first = (uint32_t)(item / m.hnrays), rr_first = (uint32_t)(item % m.hnrays);
         const uint32_t live = (uint32_t)(n_items - item < plan.K ? n_items - item : plan.K);
         const size_t at = (size_t)(stage_off[mi] - s0);
-        staged_solve<MODE, AP>(m, m.sorted_line, cap, plan, mine,
-                               rays + (ray_off[mi] - ray_off[m0]) + 2 * item * staged_half_bytes(MODE, cap), live,
-                               o_first, rr_first, m.hnrays, lane,
-                               [&](uint32_t j, uint32_t o, uint32_t f, const LaneResult& r) {
-                                   const size_t k = at + ((size_t)((rr_first + j) % m.hnrays) * m.P + o) * m.F + f;
-                                   U[k] = r.u;
-                                   if (LD) LD[k] = r.solved ? r.Ldiag : 0.0;
-                                   if (!isfinite(r.u)) atomicOr(status, ST_NONFINITE);
-                               });
+        const uint32_t again = staged_solve<MODE, AP>(
+            m, cap, plan, mine, rays + (ray_off[mi] - ray_off[m0]) + 2 * item * staged_half_bytes(MODE, cap), live,
+            o_first, rr_first, m.hnrays, lane,
+            [&](uint32_t j, uint32_t o, uint32_t f, const LaneResult& r, bool& bad) {
+                const size_t k = at + ((size_t)((rr_first + j) % m.hnrays) * m.P + o) * m.F + f;
+                U[k] = r.u;
+                if (LD) LD[k] = r.solved ? r.Ldiag : 0.0;
+                bad = bad || !isfinite(r.u);
+            });
+        if (lane == 0)
+            for (uint32_t j = 0; j < live; j++)
+                if ((again >> j) & 1u) list[1 + atomicAdd(list, 1u)] = (uint32_t)(item_off[mi] - item_off[m0] + item + j);
         __syncwarp();
     }
 }
@@ -327,6 +337,7 @@ static cudaError_t launch_multi_variant(MgrBatch* b, uint32_t m0, uint32_t m1, b
         auto tr = trace_multi_kernel<MODE>;
         e = multi_grid(tr, 8, 8 * kDescBytes, sms, halves, &grid);
         if (e != cudaSuccess) return e;
+        if ((e = cudaMemsetAsync(b->list, 0, sizeof(uint32_t), b->stream)) != cudaSuccess) return e;
         count_launch();
         tr<<<grid, 256, 8 * kDescBytes, b->stream>>>(b->d_models, b->d_caps, m0, m1, b->d_item_off, b->d_ray_off,
                                                      b->rays, b->d_t, n, b->status);
@@ -338,16 +349,23 @@ static cudaError_t launch_multi_variant(MgrBatch* b, uint32_t m0, uint32_t m1, b
         if (e != cudaSuccess) return e;
         count_launch();
         kern<<<grid, nw * 32, smem, b->stream>>>(b->d_models, b->d_plans, b->d_caps, m0, m1, b->d_group_off,
-                                                 b->d_stage_off, b->d_ray_off, b->rays, (uint32_t)bytes, b->stage_u,
+                                                 b->d_stage_off, b->d_ray_off, b->d_item_off, b->rays, b->list,
+                                                 (uint32_t)bytes, b->stage_u,
                                                  want_lam ? b->stage_ld : nullptr, b->status);
-    } else {
-        const size_t smem = (size_t)nw * batch_warp_bytes(b->cap, b->L_max);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    {
+        // every item, or after the staged solve the items it gave up
+        int gw = nw;
+        while (b->staged && gw > 1 && (size_t)gw * batch_warp_bytes(b->cap, b->L_max) > b->max_smem) gw /= 2;
+        const size_t smem = (size_t)gw * batch_warp_bytes(b->cap, b->L_max);
         auto kern = fo2_multi_kernel<MODE, AP, MINB>;
-        e = multi_grid(kern, nw, smem, sms, b->item_off[m1] - b->item_off[m0], &grid);
+        e = multi_grid(kern, gw, smem, sms, b->item_off[m1] - b->item_off[m0], &grid);
         if (e != cudaSuccess) return e;
         count_launch();
-        kern<<<grid, nw * 32, smem, b->stream>>>(b->d_models, m0, m1, b->d_item_off, b->d_stage_off, b->cap, b->L_max,
-                                                 b->stage_u, want_lam ? b->stage_ld : nullptr, b->d_t, n, b->status);
+        kern<<<grid, gw * 32, smem, b->stream>>>(b->d_models, m0, m1, b->d_item_off, b->d_stage_off, b->cap, b->L_max,
+                                                 b->staged ? b->list : nullptr, b->stage_u,
+                                                 want_lam ? b->stage_ld : nullptr, b->d_t, n, b->status);
     }
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -408,6 +426,7 @@ static void batch_release(MgrBatch* b) {
     cudaFree(b->d_group_off);
     cudaFree(b->d_ray_off);
     cudaFree(b->rays);
+    cudaFree(b->list);
     cudaFree(b->stage_u);
     cudaFree(b->stage_ld);
     cudaFree(b->d_J);
@@ -514,6 +533,7 @@ int mgr_batch_create(MgrModel* const* models, uint32_t n_models, MgrBatch** out)
         for (int mode : {MODE_FP64, MODE_SPLIT})
             b->staged_bytes[mode] = std::max(b->staged_bytes[mode], (size_t)staged_tile_bytes(mode, plans[i].W));
     }
+    b->staged = b->staged && item_off[n_models] < 0xffffffffu;
     b->ray_bytes = b->staged ? std::min(b->ray_off[n_models], std::max(kBatchRayBytes, largest_rays)) : 0;
     b->n_items = offsets[n_models];
     b->origin_off = offsets;
@@ -539,6 +559,7 @@ int mgr_batch_create(MgrModel* const* models, uint32_t n_models, MgrBatch** out)
     if (e == cudaSuccess)
         e = cudaMemcpy(b->d_ray_off, b->ray_off.data(), (n_models + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && b->ray_bytes) e = cudaMalloc(&b->rays, b->ray_bytes);
+    if (e == cudaSuccess && b->staged) e = cudaMalloc(&b->list, (item_off[n_models] + 1) * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMalloc(&b->stage_u, b->stage_entries * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&b->stage_ld, b->stage_entries * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_J, n_models * sizeof(double*));
@@ -561,6 +582,12 @@ int mgr_batch_create(MgrModel* const* models, uint32_t n_models, MgrBatch** out)
     const size_t per_warp = batch_need_bytes(b);
     int max_smem = 0;
     cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
+    b->max_smem = (size_t)max_smem;
+    if (b->staged && batch_warp_bytes(b->cap, b->L_max) > b->max_smem) {
+        batch_release(b);
+        set_error("mgr_batch_create: the longest ray of the batch does not fit one warp's shared memory");
+        return MGR_ERR_CAPACITY;
+    }
     while (b->warps > 1 && (size_t)b->warps * per_warp > (size_t)max_smem) b->warps /= 2;
     if ((size_t)b->warps * per_warp > (size_t)max_smem) {
         batch_release(b);

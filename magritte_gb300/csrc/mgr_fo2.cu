@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(256, MINB)
     fo2_kernel(DevModel m, uint32_t cap, uint32_t o_begin, uint32_t o_end, uint32_t rr0, uint32_t nR,
                double* __restrict__ U, size_t u_stride, uint32_t u_o0, double* __restrict__ LD, size_t ld_stride,
                uint32_t ld_o0, double* __restrict__ V, const uint8_t* __restrict__ cls, uint32_t cls_id,
-               int* status) {
+               const uint32_t* __restrict__ list, int* status) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int nw = blockDim.x >> 5;
     const int w = threadIdx.x >> 5;
@@ -240,9 +240,11 @@ __global__ void __launch_bounds__(256, MINB)
     for (uint32_t i = threadIdx.x; i < m.L; i += blockDim.x) sl[i] = m.sorted_line[i];
     __syncthreads();
 
-    const uint64_t n_items = (uint64_t)(o_end - o_begin) * nR;
+    // list: only the items listed (list[0] of them, from list[1] on)
+    const uint64_t n_items = list ? (uint64_t)list[0] : (uint64_t)(o_end - o_begin) * nR;
     const uint64_t stride = (uint64_t)gridDim.x * nw;
-    for (uint64_t item = (uint64_t)blockIdx.x * nw + w; item < n_items; item += stride) {
+    for (uint64_t k = (uint64_t)blockIdx.x * nw + w; k < n_items; k += stride) {
+        const uint64_t item = list ? (uint64_t)list[1 + k] : k;
         const uint32_t o = o_begin + (uint32_t)(item / nR);
         const uint32_t rr = rr0 + (uint32_t)(item % nR);
         if (cls && cls[(size_t)o * m.hnrays + rr] != cls_id) continue;  // another length class's launch
@@ -288,7 +290,7 @@ __global__ void __launch_bounds__(256, MINB)
     fo2_staged_kernel(const __grid_constant__ DevModel m, uint32_t cap, StagedPlan plan, uint32_t o_begin,
                       uint32_t o_end, uint32_t nR, unsigned char* __restrict__ rays, double* __restrict__ U,
                       size_t u_stride, uint32_t u_o0, double* __restrict__ LD, size_t ld_stride, uint32_t ld_o0,
-                      int* status) {
+                      uint32_t* __restrict__ list, int* status) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int nw = blockDim.x >> 5;
     const int w = threadIdx.x >> 5;
@@ -300,14 +302,19 @@ __global__ void __launch_bounds__(256, MINB)
     for (uint64_t item = ((uint64_t)blockIdx.x * nw + w) * plan.K; item < n_items; item += stride) {
         const uint32_t o_first = o_begin + (uint32_t)(item / nR), k_first = (uint32_t)(item % nR);
         const uint32_t live = (uint32_t)(n_items - item < plan.K ? n_items - item : plan.K);
-        staged_solve<MODE, AP>(m, m.sorted_line, cap, plan, mine, rays + 2 * item * staged_half_bytes(MODE, cap), live,
-                               o_first, k_first, nR, lane,
-                               [&](uint32_t j, uint32_t o, uint32_t f, const LaneResult& r) {
-                                   const size_t k = (k_first + j) % nR;
-                                   U[k * u_stride + (size_t)(o - u_o0) * m.F + f] = r.u;
-                                   if (LD) LD[k * ld_stride + (size_t)(o - ld_o0) * m.F + f] = r.solved ? r.Ldiag : 0.0;
-                                   if (!isfinite(r.u)) atomicOr(status, ST_NONFINITE);
-                               });
+        // a non-finite value may come from an operand that gives the pair up: the general kernel
+        // decides about those
+        const uint32_t again = staged_solve<MODE, AP>(
+            m, cap, plan, mine, rays + 2 * item * staged_half_bytes(MODE, cap), live, o_first, k_first, nR, lane,
+            [&](uint32_t j, uint32_t o, uint32_t f, const LaneResult& r, bool& bad) {
+                const size_t k = (k_first + j) % nR;
+                U[k * u_stride + (size_t)(o - u_o0) * m.F + f] = r.u;
+                if (LD) LD[k * ld_stride + (size_t)(o - ld_o0) * m.F + f] = r.solved ? r.Ldiag : 0.0;
+                bad = bad || !isfinite(r.u);
+            });
+        if (lane == 0)
+            for (uint32_t j = 0; j < live; j++)
+                if ((again >> j) & 1u) list[1 + atomicAdd(list, 1u)] = (uint32_t)item + j;
         __syncwarp();
     }
 }
@@ -710,7 +717,7 @@ size_t fo2_work_bytes(const MgrModel* model, uint32_t n_origins, bool stage_u, b
     size_t chunk = kFo2WorkBudget / per;
     if (chunk < 1) chunk = 1;
     if (chunk > n_origins) chunk = n_origins;
-    return chunk * per + 16;
+    return chunk * per + 32;
 }
 
 // Whether the staged solve serves this model: its tiles hold one line's data, so the
@@ -753,15 +760,16 @@ StagedPlan staged_plan(const DevModel& m) {
     return best;
 }
 
-// Ray memory of one origin for the staged solve, in either precision's layout.
+// Memory of one origin for the staged solve: its half rays in either precision's layout and
+// its share of the list of ray pairs given up.
 static size_t fo2_ray_bytes(const MgrModel* model, uint32_t nR) {
-    return staged_origin_bytes(MODE_FP64, model->half_cap, nR);
+    return staged_origin_bytes(MODE_FP64, model->half_cap, nR) + (size_t)nR * sizeof(uint32_t);
 }
 
 template <int MODE, int AP, int MINB>
 static cudaError_t launch_staged_variant(MgrModel* model, uint32_t o_begin, uint32_t o_end, uint32_t nR,
-                                         unsigned char* rays, double* U, size_t us, uint32_t uo, double* LD, size_t ls,
-                                         uint32_t lo) {
+                                         unsigned char* rays, uint32_t* list, double* U, size_t us, uint32_t uo,
+                                         double* LD, size_t ls, uint32_t lo) {
     const DevModel& m = model->dm;
     int nw = (MODE == MODE_SPLIT) ? model->fo2_warps_split : model->fo2_warps_fp64;
     if (nw < 1 || nw > 8) nw = 8;
@@ -782,7 +790,7 @@ static cudaError_t launch_staged_variant(MgrModel* model, uint32_t o_begin, uint
     if (grid < 1) grid = 1;
     count_launch();
     kern<<<(unsigned)grid, nw * 32, smem, model->stream>>>(m, model->half_cap, plan, o_begin, o_end, nR, rays, U, us, uo,
-                                                          LD, ls, lo, model->status);
+                                                          LD, ls, lo, list, model->status);
     return cudaGetLastError();
 }
 
@@ -798,20 +806,6 @@ static cudaError_t launch_trace_rays(MgrModel* model, uint32_t o_begin, uint32_t
     return cudaGetLastError();
 }
 
-// Walks and solves origins [o_begin, o_end) x ray pairs [rr0, rr0 + nR) with the half rays in
-// `rays` (fo2_ray_bytes per origin).
-template <int MODE, int AP>
-static cudaError_t launch_staged(MgrModel* model, uint32_t o_begin, uint32_t o_end, uint32_t rr0, uint32_t nR,
-                                 unsigned char* rays, double* U, size_t us, uint32_t uo, double* LD, size_t ls,
-                                 uint32_t lo) {
-    const cudaError_t e = launch_trace_rays<MODE>(model, o_begin, o_end, rr0, nR, rays);
-    if (e != cudaSuccess) return e;
-    const int minb = (MODE == MODE_SPLIT) ? model->fo2_minb_split : model->fo2_minb_fp64;
-    if (minb == 2) return launch_staged_variant<MODE, AP, 2>(model, o_begin, o_end, nR, rays, U, us, uo, LD, ls, lo);
-    if (minb == 4) return launch_staged_variant<MODE, AP, 4>(model, o_begin, o_end, nR, rays, U, us, uo, LD, ls, lo);
-    return launch_staged_variant<MODE, AP, 3>(model, o_begin, o_end, nR, rays, U, us, uo, LD, ls, lo);
-}
-
 // One launch of fo2_kernel over origins [o_begin, o_end) x ray pairs [rr0, rr0 + nR):
 // every pair (cls null, buffers sized for the model's longest half ray) or the pairs of
 // length class cls_id (buffers sized for that class's longest half ray).
@@ -819,7 +813,7 @@ template <int MODE, int AP, int MINB, bool UV = false, int GEO = 0>
 static cudaError_t launch_fo2_variant(MgrModel* model, uint32_t o_begin, uint32_t o_end, uint32_t rr0, uint32_t nR,
                                       double* U, size_t u_stride, uint32_t u_o0, double* LD, size_t ld_stride,
                                       uint32_t ld_o0, double* V = nullptr, const uint8_t* cls = nullptr,
-                                      uint32_t cls_id = 0) {
+                                      uint32_t cls_id = 0, const uint32_t* list = nullptr) {
     const DevModel& m = model->dm;
     const uint32_t cap = cls ? model->class_cap[cls_id] : model->half_cap;
     int nw = (MODE == MODE_SPLIT) ? model->fo2_warps_split : model->fo2_warps_fp64;
@@ -840,8 +834,34 @@ static cudaError_t launch_fo2_variant(MgrModel* model, uint32_t o_begin, uint32_
     if (grid < 1) grid = 1;
     count_launch();
     kern<<<(unsigned)grid, nw * 32, smem, model->stream>>>(m, cap, o_begin, o_end, rr0, nR, U, u_stride, u_o0, LD,
-                                                          ld_stride, ld_o0, V, cls, cls_id, model->status);
+                                                          ld_stride, ld_o0, V, cls, cls_id, list, model->status);
     return cudaGetLastError();
+}
+
+// Walks and solves origins [o_begin, o_end) x ray pairs [rr0, rr0 + nR) with the half rays in
+// `rays` and, behind them, the list of ray pairs given up, which the general kernel solves.
+template <int MODE, int AP>
+static cudaError_t launch_staged(MgrModel* model, uint32_t o_begin, uint32_t o_end, uint32_t rr0, uint32_t nR,
+                                 unsigned char* rays, double* U, size_t us, uint32_t uo, double* LD, size_t ls,
+                                 uint32_t lo) {
+    uint32_t* list = reinterpret_cast<uint32_t*>(
+        rays + (size_t)(o_end - o_begin) * staged_origin_bytes(MODE, model->half_cap, nR));
+    cudaError_t e = cudaMemsetAsync(list, 0, sizeof(uint32_t), model->stream);
+    if (e == cudaSuccess) e = launch_trace_rays<MODE>(model, o_begin, o_end, rr0, nR, rays);
+    if (e != cudaSuccess) return e;
+    const int minb = (MODE == MODE_SPLIT) ? model->fo2_minb_split : model->fo2_minb_fp64;
+    if (minb == 2)
+        e = launch_staged_variant<MODE, AP, 2>(model, o_begin, o_end, nR, rays, list, U, us, uo, LD, ls, lo);
+    else if (minb == 4)
+        e = launch_staged_variant<MODE, AP, 4>(model, o_begin, o_end, nR, rays, list, U, us, uo, LD, ls, lo);
+    else
+        e = launch_staged_variant<MODE, AP, 3>(model, o_begin, o_end, nR, rays, list, U, us, uo, LD, ls, lo);
+    if (e != cudaSuccess) return e;
+    if (model->dm.sph || model->dm.adaptive)
+        return launch_fo2_variant<MODE, AP, 3, false, 1>(model, o_begin, o_end, rr0, nR, U, us, uo, LD, ls, lo, nullptr,
+                                                         nullptr, 0, list);
+    return launch_fo2_variant<MODE, AP, 3>(model, o_begin, o_end, rr0, nR, U, us, uo, LD, ls, lo, nullptr, nullptr, 0,
+                                           list);
 }
 
 // The formal solve's launches.  Models whose longest half ray is over 128 steps (9 KB
@@ -975,9 +995,9 @@ cudaError_t launch_fo2_range(MgrModel* model, int precision, uint32_t o_begin, u
     uint32_t chunk = o_end - o_begin;
     // the staged solve where the work area takes the half rays of enough origins to fill the
     // GPU (or of all of them); the general kernel traces into shared memory
-    bool staged = work && !v && !alo_off && staged_ok(model);
+    bool staged = work && !v && !alo_off && staged_ok(model) && (uint64_t)chunk * nR < 0xffffffffu;
     if (staged) {
-        const size_t fit = work_bytes > 16 ? (work_bytes - 16) / (per * k + fo2_ray_bytes(model, m.hnrays)) : 0;
+        const size_t fit = work_bytes > 32 ? (work_bytes - 32) / (per * k + fo2_ray_bytes(model, m.hnrays)) : 0;
         if (fit >= chunk) {
         } else if (fit * nR >= (uint64_t)model->sm_count * 32) {
             chunk = (uint32_t)fit;
