@@ -77,6 +77,7 @@ static int read_status(MgrModel* model) {
 static int ensure_scratch(MgrModel* m, double** p, size_t* have, size_t bytes) {
     if (*have >= bytes) return MGR_OK;
     if (*p) cudaFree(*p);
+    ali_shard_changed(m);  // a captured ALI iteration holds the old address
     *p = nullptr;
     *have = 0;
     void* q = nullptr;

@@ -13,7 +13,9 @@
 #include <algorithm>
 #include <vector>
 
+#include "mgr_ali.h"
 #include "mgr_image.cuh"
+#include "mgr_staged.cuh"
 
 namespace mgr {
 
@@ -60,7 +62,8 @@ __global__ void __launch_bounds__(256) image_kernel(DevModel m, uint32_t cap, ui
 
 template <int MODE, int AP, bool TAU>
 __global__ void __launch_bounds__(256) image_new_kernel(DevModel m, ImagePlane ip, uint32_t cap,
-                                                        double* __restrict__ I, int* status) {
+                                                        double* __restrict__ I, const uint32_t* __restrict__ list,
+                                                        int* status) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int nw = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double* sl = reinterpret_cast<double*>(smem);
@@ -69,8 +72,10 @@ __global__ void __launch_bounds__(256) image_new_kernel(DevModel m, ImagePlane i
     carve_halves(smem + (size_t)Lpad * 8 + (size_t)w * half_bytes_per_warp(cap), cap, bk, fw);
     for (uint32_t i = threadIdx.x; i < m.L; i += blockDim.x) sl[i] = m.sorted_line[i];
     __syncthreads();
-    const uint32_t npix = ip.nx * ip.ny;
-    for (uint32_t px = blockIdx.x * nw + w; px < npix; px += gridDim.x * nw) {
+    // list: only the pixels listed (list[0] of them, from list[1] on)
+    const uint32_t npix = list ? list[0] : ip.nx * ip.ny;
+    for (uint32_t k = blockIdx.x * nw + w; k < npix; k += gridDim.x * nw) {
+        const uint32_t px = list ? list[1 + k] : k;
         double org[3];
         pixel_origin(ip, ip.ImX[px], ip.ImY[px], org);
         double Z;
@@ -90,6 +95,63 @@ __global__ void __launch_bounds__(256) image_new_kernel(DevModel m, ImagePlane i
                 if (!isfinite(v)) atomicOr(status, ST_NONFINITE);
             }
         }
+        __syncwarp();
+    }
+}
+
+// ---------------------------------------------------------------------------------
+// New imager, staged (mgr_staged.cuh): image_trace_kernel walks a warp per pixel into global
+// memory, image_staged_kernel eliminates; pixels it gives up go to image_new_kernel.
+// ---------------------------------------------------------------------------------
+template <int MODE>
+__global__ void __launch_bounds__(256) image_trace_kernel(const __grid_constant__ DevModel m, ImagePlane ip,
+                                                          uint32_t cap, uint32_t px0, uint32_t px1,
+                                                          unsigned char* __restrict__ rays, int* status) {
+    constexpr int LAY = (MODE == MODE_SPLIT) ? LAY_SPLIT : LAY_FP64;
+    const int lane = threadIdx.x & 31;
+    const uint32_t px = px0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (px >= px1) return;
+    unsigned char* base = rays + (size_t)(px - px0) * staged_half_bytes(MODE, cap);
+    HalfSmem h = staged_half<MODE>(base, cap);
+    double org[3];
+    pixel_origin(ip, ip.ImX[px], ip.ImY[px], org);
+    double Z;
+    const uint32_t start = pixel_start(m, org, ip, lane, Z);
+    const int n = trace_image<true, LAY>(m, org, ip, start, Z, cap, h, lane, status);
+    if (lane == 0) {
+        HalfHead<MODE>* hd = reinterpret_cast<HalfHead<MODE>*>(base);
+        const double sh0 = image_shift(m, org, ip, start, Z);
+        if constexpr (MODE == MODE_SPLIT) {
+            set_dsh0(h, sh0);
+            hd->dsh0 = h.dsh0;
+            hd->dsl0 = h.dsl0;
+        } else {
+            hd->shift0 = sh0;
+        }
+        hd->n = n;
+        hd->start = start;
+    }
+}
+
+template <int MODE, int AP, int MINB>
+__global__ void __launch_bounds__(256, MINB)
+    image_staged_kernel(const __grid_constant__ DevModel m, uint32_t cap, uint32_t px0, uint32_t px1,
+                        unsigned char* __restrict__ rays, double* __restrict__ I, uint32_t* __restrict__ list) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int nw = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned char* mine = smem + (size_t)w * staged_tile_bytes(MODE, 4);
+    for (uint32_t px = px0 + blockIdx.x * nw + w; px < px1; px += gridDim.x * nw) {
+        unsigned char* half = rays + (size_t)(px - px0) * staged_half_bytes(MODE, cap);
+        const HalfHead<MODE>* hd = reinterpret_cast<const HalfHead<MODE>*>(half);
+        if (hd->n < 0) continue;  // status recorded by the trace
+        // rays without an interior point and non-finite values are the general kernel's
+        bool again = hd->n == 0;
+        if (!again)
+            again = staged_image<MODE, AP>(m, cap, mine, half, hd->start, lane, [&](uint32_t f, double v, bool& bad) {
+                I[(size_t)px * m.F + f] = v;
+                bad = bad || !isfinite(v);
+            });
+        if (again && lane == 0) list[1 + atomicAdd(list, 1u)] = px;
         __syncwarp();
     }
 }
@@ -134,8 +196,58 @@ static cudaError_t launch_image_t(MgrModel* model, uint32_t rr, double* I) {
     return cudaGetLastError();
 }
 
+// Half rays of a pass of the staged imager at most.
+constexpr size_t kImageRayBytes = size_t(1) << 30;
+
+// The model's work area grown to `bytes`; false (and the area as it was) when it cannot be.
+static bool grow_work(MgrModel* model, size_t bytes) {
+    if (model->work_bytes >= bytes) return true;
+    void* q = nullptr;
+    if (cudaMalloc(&q, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (model->work) cudaFree(model->work);  // waits for the work that uses it
+    ali_shard_changed(model);                // a captured ALI iteration holds the old address
+    model->work = static_cast<double*>(q);
+    model->work_bytes = bytes;
+    return true;
+}
+
 template <int MODE, int AP, bool TAU>
 static cudaError_t launch_image_new_t(MgrModel* model, const ImagePlane& ip, uint32_t cap, double* I) {
+    // Intensities of models whose lines are apart: the staged solve where its rays fit the work
+    // area (an image of 151 x 97 pixels x 41 frequencies, FP64, 20k points: see the kernel)
+    const uint32_t npix = ip.nx * ip.ny;
+    const size_t hb = staged_half_bytes(MODE, cap), list_bytes = (size_t)(npix + 1) * sizeof(uint32_t);
+    const size_t pass = std::max<size_t>(1, std::min<size_t>(npix, kImageRayBytes / hb));
+    const size_t list_at = (pass * hb + 15) & ~size_t(15);
+    const bool staged = !TAU && (model->dm.L == 1 || (AP == APPROX_CLOSELINES && model->lines_apart)) &&
+                        grow_work(model, list_at + list_bytes);
+    uint32_t* list = nullptr;
+    if (staged) {
+        unsigned char* rays = reinterpret_cast<unsigned char*>(model->work);
+        list = reinterpret_cast<uint32_t*>(rays + list_at);
+        cudaError_t e = cudaMemsetAsync(list, 0, sizeof(uint32_t), model->stream);
+        auto kern = image_staged_kernel<MODE, AP, MODE == MODE_SPLIT ? 4 : 2>;
+        const int nw = 4;
+        const size_t tile = nw * staged_tile_bytes(MODE, 4);
+        int per_sm = 0;
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nw * 32, tile);
+        if (e != cudaSuccess) return e;
+        const unsigned full = (unsigned)model->sm_count * (per_sm > 0 ? per_sm : 1);
+        for (size_t p0 = 0; p0 < npix; p0 += pass) {
+            const uint32_t px0 = (uint32_t)p0, px1 = (uint32_t)std::min<size_t>(npix, p0 + pass), n = px1 - px0;
+            count_launch();
+            image_trace_kernel<MODE><<<(n + 7) / 8, 256, 0, model->stream>>>(model->dm, ip, cap, px0, px1, rays,
+                                                                            model->status);
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            count_launch();
+            kern<<<std::min(full, (n + nw - 1) / nw), nw * 32, tile, model->stream>>>(model->dm, cap, px0, px1, rays, I,
+                                                                                      list);
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        }
+    }
     size_t smem;
     unsigned grid;
     auto kern = image_new_kernel<MODE, AP, TAU>;
@@ -143,7 +255,7 @@ static cudaError_t launch_image_new_t(MgrModel* model, const ImagePlane& ip, uin
     if (e != cudaSuccess) return e;
     const int nw = (int)((smem - (size_t)((model->dm.L + 1) & ~1u) * 8) / half_bytes_per_warp(cap));
     count_launch();
-    kern<<<grid, nw * 32, smem, model->stream>>>(model->dm, ip, cap, I, model->status);
+    kern<<<grid, nw * 32, smem, model->stream>>>(model->dm, ip, cap, I, list, model->status);
     return cudaGetLastError();
 }
 

@@ -97,7 +97,7 @@ static __host__ __device__ __forceinline__ double image_shift(const DevModel& m,
 // shifts 1 + v . d of a motionless observer.  Returns the steps stored, 0 if the ray
 // met no interior point (the reference then keeps only the start point), -1 on
 // capacity overflow.
-template <bool STORE>
+template <bool STORE, int LAY = LAY_FULL>
 static __device__ int trace_image(const DevModel& m, const double* org, const ImagePlane& ip, uint32_t start, double Z,
                            uint32_t cap, HalfSmem h, int lane, int* status) {
     const double dx = ip.d[0], dy = ip.d[1], dz = ip.d[2];
@@ -122,11 +122,9 @@ static __device__ int trace_image(const DevModel& m, const double* org, const Im
             if (STORE && lane == 0) {
                 h.ids[count] = nxt;
                 h.eid[count] = sph_eid(crt, nxt);
-                h.dZ[count] = dZl;
-                const double sh = image_shift(m, org, ip, nxt, Z);
-                h.shift[count] = sh;
-                store_dsh(h, count, sh);
-                h.dzs[count] = (float)dZl * m.dz_scale;
+                store_dz<LAY>(m, h, count, dZl);
+                store_shift<LAY>(h, count, image_shift(m, org, ip, nxt, Z));
+                if (LAY == LAY_FULL) h.dzs[count] = (float)dZl * m.dz_scale;
             }
             count++;
             if (m.p2b[nxt] != m.P) {
@@ -185,7 +183,7 @@ static __device__ int trace_image(const DevModel& m, const double* org, const Im
         if (STORE && lane == 0) {
             h.ids[count] = nxt;
             h.eid[count] = cum + besti;
-            h.dZ[count] = dZl;
+            store_dz<LAY>(m, h, count, dZl);
         }
         count++;
         const bool interior = m.p2b[nxt] == m.P;
@@ -204,10 +202,8 @@ static __device__ int trace_image(const DevModel& m, const double* org, const Im
     if (STORE && count > 0) {
         for (int s = lane; s < count; s += 32) {
             const double4_32a v = m.vel[h.ids[s]];
-            const double sh = dadd_rn(1.0, dot3_rn(v.x, v.y, v.z, dx, dy, dz));
-            h.shift[s] = sh;
-            store_dsh(h, s, sh);
-            h.dzs[s] = (float)h.dZ[s] * m.dz_scale;
+            store_shift<LAY>(h, s, dadd_rn(1.0, dot3_rn(v.x, v.y, v.z, dx, dy, dz)));
+            if (LAY == LAY_FULL) h.dzs[s] = (float)h.dZ[s] * m.dz_scale;
         }
         __syncwarp();
     }

@@ -8,6 +8,7 @@
 // u, v and the per-direction ALO factors; stage 2 sums J and the ALO diagonal per
 // origin in the reference's order (ray pair outer, quadrature point inner, forward
 // then backward direction).
+#include "mgr_ali.h"
 #include "mgr_internal.h"
 #include "mgr_solve.cuh"
 
@@ -242,6 +243,7 @@ int mgr_formal_solve_sc0_device(MgrModel* model, int precision, double* J_dev, d
     const size_t wb = sc0_work_bytes(model, model->dm.P, u_dev == nullptr, lambda_diag_dev != nullptr);
     if (model->work_bytes < wb) {
         if (model->work) cudaFree(model->work);
+        ali_shard_changed(model);  // a captured ALI iteration holds the old address
         model->work = nullptr;
         model->work_bytes = 0;
         void* q = nullptr;
