@@ -936,7 +936,7 @@ extern "C" int mgr_emu_image_new_adjoint(const MgrModelDesc* d, const double* ra
     int rc = for_each_pixel(d, x, raydir, nx, ny, ip, [&](uint32_t px, uint32_t start, const HalfSmem& bk, int nb) {
         size_t pairs = 1;
         for (int s = 0; s < nb; s++) pairs += m.nint_all[bk.eid[s]];
-        if (scratch.size() < 3 * pairs) scratch.resize(3 * pairs);
+        if (scratch.size() < 4 * pairs) scratch.resize(4 * pairs);
         const LaneScratch scr{scratch.data(), 1, (uint32_t)pairs};
         const AdjAcc acc{AdjGrads{g_em, g_op, g_iw, g_Sp, g_vel, {ip.d[0], ip.d[1], ip.d[2]}}, m.L};
         for (uint32_t f = 0; f < m.F; f++) {
@@ -1010,7 +1010,7 @@ extern "C" int mgr_emu_fo2_adjoint(const MgrModelDesc* d, const double* gJ, doub
         size_t pairs = 2;
         for (int s = 0; s < nb; s++) pairs += m.nint_all[bk.eid[s]];
         for (int s = 0; s < nf; s++) pairs += m.nint_all[fw.eid[s]];
-        if (scratch.size() < 4 * pairs) scratch.resize(4 * pairs);
+        if (scratch.size() < 5 * pairs) scratch.resize(5 * pairs);
         const Fo2Scratch scr{scratch.data(), 1, (uint32_t)pairs};
         const double* db = ray_dir(m, o, rr);
         const double* df = ray_dir(m, o, ar);

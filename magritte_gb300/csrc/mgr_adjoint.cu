@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(256) image_adj_kernel(DevModel m, ImagePlane i
     for (uint32_t i = threadIdx.x; i < m.L; i += blockDim.x) sl[i] = m.sorted_line[i];
     __syncthreads();
     const size_t slot = (size_t)blockIdx.x * nw + w;
-    LaneScratch scr{scratch + slot * (size_t)scratch_pairs * 3 * 32 + lane, 32, scratch_pairs};
+    LaneScratch scr{scratch + slot * (size_t)scratch_pairs * 4 * 32 + lane, 32, scratch_pairs};
     const AdjAcc acc{g, m.L};
     const uint32_t npix = ip.nx * ip.ny;
     for (uint32_t px = blockIdx.x * nw + w; px < npix; px += gridDim.x * nw) {
@@ -347,7 +347,7 @@ int mgr_image_new_adjoint_device(MgrModel* model, const double* raydir, uint32_t
     auto run = [&](auto kern) -> cudaError_t {
         cudaError_t r = pixel_launch_shape(model, kern, cap, npix, &nw, &smem, &grid);
         if (r != cudaSuccess) return r;
-        const size_t need = (size_t)grid * nw * pairs * 3 * 32 * sizeof(double);
+        const size_t need = (size_t)grid * nw * pairs * 4 * 32 * sizeof(double);
         if (model->adj_scratch_bytes < need) {  // grown on demand, kept for the next call
             cudaFree(model->adj_scratch);
             model->adj_scratch = nullptr;

@@ -29,16 +29,19 @@ MGR_HD double gauss_s(double iw, double diff) {
     return iw * INVERSE_SQRT_PI * exp(-x * x);
 }
 
-// a^(1-f) b^f as a (b / a)^f (interpolate_log)
+// a^(1-f) b^f as a (b / a)^f (interpolate_log).  The power, and the erf difference below, are
+// out of line: inlined at their dozen sites they made the adjoint kernels several times the
+// instruction cache (instruction fetch was 30 of 50 cycles per issue).
+static __host__ __device__ __noinline__ double ilog_between_s(double a, double b, double f) { return a * pow(b / a, f); }
 MGR_HD double ilog_s(double a, double b, double f) {
     if (f == 0.0) return a;
     if (f == 1.0) return b;
-    return a * pow(b / a, f);
+    return ilog_between_s(a, b, f);
 }
 
 // erf(a) - erf(b) without cancellation when a and b lie on the same side of 0
 // (differences of erfc there, which keeps its relative precision in the wings).
-MGR_HD double erf_diff_s(double a, double b) {
+static __host__ __device__ __noinline__ double erf_diff_s(double a, double b) {
     if (a > 0.0 && b > 0.0) return erfc(b) - erfc(a);
     if (a < 0.0 && b < 0.0) return erfc(-a) - erfc(-b);
     return erf(a) - erf(b);
@@ -98,6 +101,38 @@ struct AdjAcc {
         base[(size_t)p * L + l] += v;
 #endif
     }
+    // Adds six contributions whose targets (null: none) the warp's lanes agree on.  The lanes
+    // halve the values they carry with the lanes they sum over, so the warp spends 9 FP64
+    // additions instead of 30, and six lanes issue the atomics.
+    MGR_HD void add6(double* const t[6], const double v[6]) const {
+#ifdef __CUDA_ARCH__
+        const int lane = threadIdx.x & 31;
+        double w[8] = {v[0], v[1], v[2], v[3], v[4], v[5], 0.0, 0.0};
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const int off = 16 >> k, half = 4 >> k;
+            const bool up = (lane & off) != 0;
+#pragma unroll
+            for (int j = 0; j < half; j++) {
+                const double send = up ? w[j] : w[j + half];
+                const double keep = up ? w[j + half] : w[j];
+                w[j] = keep + __shfl_xor_sync(FULL_MASK, send, off);
+            }
+        }
+        w[0] += __shfl_xor_sync(FULL_MASK, w[0], 2);
+        w[0] += __shfl_xor_sync(FULL_MASK, w[0], 1);
+        const int k = ((lane & 16) >> 2) | ((lane & 8) >> 2) | ((lane & 4) >> 2);
+        double* to = k == 0 ? t[0] : k == 1 ? t[1] : k == 2 ? t[2] : k == 3 ? t[3] : k == 4 ? t[4] : k == 5 ? t[5] : nullptr;
+        if ((lane & 3) == 0 && to && w[0] != 0.0) atomicAdd(to, w[0]);
+#else
+        for (int k = 0; k < 6; k++)
+            if (t[k]) *t[k] += v[k];
+#endif
+    }
+    MGR_HD double* at(int kind, uint32_t p, uint32_t l) const {
+        double* base = kind == ADJ_EM ? g.em : kind == ADJ_OP ? g.op : kind == ADJ_IW ? g.iw : g.Sp;
+        return base + (size_t)p * L + l;
+    }
     MGR_HD void add_shift(uint32_t p, double v) const {
 #ifdef __CUDA_ARCH__
         for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(FULL_MASK, v, off);
@@ -129,7 +164,7 @@ MGR_HD uint32_t line_of(const DevModel& m, uint32_t s) {
 // Element emissivity and opacity (eta_chi_fp64, smooth).
 template <int AP>
 MGR_HD void elem_s(const DevModel& m, const double* sl, double nu, const Elem& e, double& eta, double& chi) {
-    const double freq = nu * e.shift;
+    const double freq = dmul_rn(nu, e.shift);
     uint32_t lo, hi;
     elem_bracket<AP>(m, sl, freq, e.nr, lo, hi);
     const size_t b1 = (size_t)e.nr * m.L, b2 = (size_t)e.ni * m.L;
@@ -151,7 +186,7 @@ MGR_HD void elem_s(const DevModel& m, const double* sl, double nu, const Elem& e
 template <int AP>
 MGR_HD void elem_s_adj(const DevModel& m, const double* sl, double nu, const Elem& e, double g_eta, double g_chi,
                        const AdjAcc& acc, double& g_shift) {
-    const double freq = nu * e.shift;
+    const double freq = dmul_rn(nu, e.shift);
     uint32_t lo, hi;
     elem_bracket<AP>(m, sl, freq, e.nr, lo, hi);
     uint32_t wlo = lo, whi = hi;
@@ -172,23 +207,24 @@ MGR_HD void elem_s_adj(const DevModel& m, const double* sl, double nu, const Ele
             const double g_emE = g_eta * prof, g_opE = g_chi * prof;
             const double g_iwE = gprof * prof * (1.0 / iw - 2.0 * x * diff);
             g_shift += gprof * prof * (-2.0 * x * iw) * nu;
-            gem_nr = g_emE * (1.0 - f) * emE / m.em[b1 + l];
-            gop_nr = g_opE * (1.0 - f) * opE / m.op[b1 + l];
-            giw_nr = g_iwE * (1.0 - f);
+            gem_nr = g_emE;
+            gop_nr = g_opE;
+            giw_nr = g_iwE;
             if (f != 0.0) {
+                gem_nr = g_emE * (1.0 - f) * emE / m.em[b1 + l];
+                gop_nr = g_opE * (1.0 - f) * opE / m.op[b1 + l];
+                giw_nr = g_iwE * (1.0 - f);
                 gem_ni = g_emE * f * emE / m.em[b2 + l];
                 gop_ni = g_opE * f * opE / m.op[b2 + l];
                 giw_ni = g_iwE * f;
             }
         }
-        acc.add(ADJ_EM, e.nr, l, gem_nr);
-        acc.add(ADJ_OP, e.nr, l, gop_nr);
-        acc.add(ADJ_IW, e.nr, l, giw_nr);
-        if (f != 0.0) {
-            acc.add(ADJ_EM, e.ni, l, gem_ni);
-            acc.add(ADJ_OP, e.ni, l, gop_ni);
-            acc.add(ADJ_IW, e.ni, l, giw_ni);
-        }
+        const bool two = f != 0.0;
+        double* const to[6] = {acc.at(ADJ_EM, e.nr, l), acc.at(ADJ_OP, e.nr, l), acc.at(ADJ_IW, e.nr, l),
+                               two ? acc.at(ADJ_EM, e.ni, l) : nullptr, two ? acc.at(ADJ_OP, e.ni, l) : nullptr,
+                               two ? acc.at(ADJ_IW, e.ni, l) : nullptr};
+        const double v[6] = {gem_nr, gop_nr, giw_nr, gem_ni, gop_ni, giw_ni};
+        acc.add6(to, v);
     }
 }
 
@@ -208,8 +244,10 @@ MGR_HD void pair_bracket(const DevModel& m, const double* sl, double cf, double 
     }
 }
 
-// One line's optical depth over a large-shift pair (dtau_single_line_fp64, smooth).
-MGR_HD double ld_s(const DevModel& m, const Elem& lo, const Elem& hi, uint32_t l, double cf, double nf, double dz) {
+// One line's optical depth over a large-shift pair (dtau_single_line_fp64, smooth).  E: its erf
+// difference, taken when `known`, else stored.
+MGR_HD double ld_s(const DevModel& m, const Elem& lo, const Elem& hi, uint32_t l, double cf, double nf, double dz,
+                   double& E, bool known) {
     const size_t c1 = (size_t)lo.nr * m.L, c2 = (size_t)lo.ni * m.L;
     const size_t n1 = (size_t)hi.nr * m.L, n2 = (size_t)hi.ni * m.L;
     const double linefreq = m.line[l];
@@ -222,7 +260,8 @@ MGR_HD double ld_s(const DevModel& m, const Elem& lo, const Elem& hi, uint32_t l
     const double next_pos = (linefreq - nf) * avg_iw;
     const double curr_pos = (linefreq - cf) * avg_iw;
     const double diff_pos = next_pos - curr_pos;
-    const double erfterm = (nop + cop) / 2.0 / diff_pos / 2.0 * erf_diff_s(next_pos, curr_pos);
+    if (!known) E = erf_diff_s(next_pos, curr_pos);
+    const double erfterm = (nop + cop) * 0.25 / diff_pos * E;
     return dz * (avg_iw * erfterm + m.min_opacity);
 }
 
@@ -232,7 +271,7 @@ struct LdAdj {
     double g_iwc, g_iwn, g_cop, g_nop, g_cf, g_nf;
 };
 MGR_HD LdAdj ld_s_adj(const DevModel& m, const Elem& lo, const Elem& hi, uint32_t l, double cf, double nf, double dz,
-                      double gld) {
+                      double gld, double E) {
     const size_t c1 = (size_t)lo.nr * m.L, c2 = (size_t)lo.ni * m.L;
     const size_t n1 = (size_t)hi.nr * m.L, n2 = (size_t)hi.ni * m.L;
     const double linefreq = m.line[l];
@@ -257,13 +296,13 @@ MGR_HD LdAdj ld_s_adj(const DevModel& m, const Elem& lo, const Elem& hi, uint32_
     const double cp = (linefreq - cf) * avg;
     const double dp = np - cp;
     const double avg_op = (nop + cop) / 2.0;
-    const double E = erf_diff_s(np, cp);
-    const double erfterm = avg_op / dp / 2.0 * E;
+    const double half_rdp = 0.5 / dp;
+    const double erfterm = avg_op * half_rdp * E;
     const double g_erfterm = gld * dz * avg;
     double gavg = gld * dz * erfterm;
-    const double g_avg_op = g_erfterm * E / (2.0 * dp);
-    const double gE = g_erfterm * avg_op / (2.0 * dp);
-    const double gdp = -g_erfterm * erfterm / dp;
+    const double g_avg_op = g_erfterm * E * half_rdp;
+    const double gE = g_erfterm * avg_op * half_rdp;
+    const double gdp = -2.0 * g_erfterm * erfterm * half_rdp;
     const double two_rsqpi = 2.0 * INVERSE_SQRT_PI;
     double gnp = gE * two_rsqpi * exp(-np * np) + gdp;
     double gcp = -gE * two_rsqpi * exp(-cp * cp) - gdp;
@@ -281,7 +320,9 @@ struct PairS {
     bool large;
     double dtau, Slo, Shi;
     double eta_o, chi_o, eta_i, chi_i;  // trapezoid branch
-    double sum_dtau, sum_c, sum_n;       // large branch, before the clamp
+    double sum_dtau;                     // large branch, before the clamp
+    double E;                            // large branch with one line in reach: its erf difference
+    bool one;                            // large branch with one line in reach
 };
 
 template <int AP>
@@ -291,42 +332,70 @@ MGR_HD bool pair_large(const DevModel& m, const Elem& outer, const Elem& inner) 
     return dshift_abs > (a < b ? a : b);
 }
 
+// A sweep's element between two pairs: emissivity and opacity, once evaluated.
+struct ElemVal {
+    double eta, chi;
+    bool ok;
+};
+
+// oc / ic: the outer / inner element's values if already known (evaluated and stored
+// otherwise, trapezoid branch).  E: the pair's erf difference if known (one line in reach).
 template <int AP>
-MGR_HD PairS pair_s(const DevModel& m, const double* sl, double nu, const Elem& outer, const Elem& inner, double dz) {
+MGR_HD PairS pair_s(const DevModel& m, const double* sl, double nu, const Elem& outer, const Elem& inner, double dz,
+                    ElemVal& oc, ElemVal& ic, const double* E = nullptr) {
     PairS r{};
     r.large = pair_large<AP>(m, outer, inner);
     if (!r.large) {
-        elem_s<AP>(m, sl, nu, outer, r.eta_o, r.chi_o);
-        elem_s<AP>(m, sl, nu, inner, r.eta_i, r.chi_i);
+        for (int k = 0; k < 2; k++) {  // one site of elem_s
+            ElemVal& v = k ? ic : oc;
+            if (v.ok) continue;
+            elem_s<AP>(m, sl, nu, k ? inner : outer, v.eta, v.chi);
+            v.ok = true;
+        }
+        r.eta_o = oc.eta;
+        r.chi_o = oc.chi;
+        r.eta_i = ic.eta;
+        r.chi_i = ic.chi;
         r.Slo = r.eta_o / r.chi_o;
         r.Shi = r.eta_i / r.chi_i;
         r.dtau = 0.5 * (r.chi_o + r.chi_i) * dz;
         return r;
     }
-    const double cf = nu * outer.shift, nf = nu * inner.shift;
+    // Rounded products, here and in elem_s: fused into (nu shift - line) in the forward pass or in
+    // the adjoint alone, a position moves by 1e-10 of a width, and an adjoint whose state and
+    // recomputed pairs differ by that is off by 2e-10 to 6e-10 in every gradient (it was, against
+    // the restatement on the CPU; 1e-14 now).
+    const double cf = dmul_rn(nu, outer.shift), nf = dmul_rn(nu, inner.shift);
     uint32_t a, b;
     pair_bracket<AP>(m, sl, cf, nf, outer.nr, inner.nr, a, b);
     const size_t c1 = (size_t)outer.nr * m.L, c2 = (size_t)outer.ni * m.L;
     const size_t n1 = (size_t)inner.nr * m.L, n2 = (size_t)inner.ni * m.L;
-    double sd = 0.0, sc = 0.0, sn = 0.0;
+    r.one = b == a + 1;
+    if (E) r.E = *E;
+    double sd = 0.0, sc = 0.0, sn = 0.0, lsc = 0.0, lsn = 0.0;
     for (uint32_t s = a; s < b; s++) {
         const uint32_t l = line_of<AP>(m, s);
-        const double ld = ld_s(m, outer, inner, l, cf, nf, dz);
+        const double ld = ld_s(m, outer, inner, l, cf, nf, dz, r.E, E && r.one);
+        lsc = ilog_s(m.Sp[c1 + l], m.Sp[c2 + l], outer.fac);
+        lsn = ilog_s(m.Sp[n1 + l], m.Sp[n2 + l], inner.fac);
         sd += ld;
-        sc += ld * ilog_s(m.Sp[c1 + l], m.Sp[c2 + l], outer.fac);
-        sn += ld * ilog_s(m.Sp[n1 + l], m.Sp[n2 + l], inner.fac);
+        sc += ld * lsc;
+        sn += ld * lsn;
     }
     r.sum_dtau = sd;
-    r.sum_c = sc;
-    r.sum_n = sn;
     double d = sd;
     if (AP != APPROX_NONE) {
         const double bound_min_dtau = m.min_opacity * dz;
         if (-bound_min_dtau < d) d = (bound_min_dtau > d) ? bound_min_dtau : d;
     }
     r.dtau = d;
-    r.Slo = sc / d;
-    r.Shi = sn / d;
+    if (r.one && d == sd) {  // (ld S) / ld
+        r.Slo = lsc;
+        r.Shi = lsn;
+    } else {
+        r.Slo = sc / d;
+        r.Shi = sn / d;
+    }
     return r;
 }
 
@@ -337,10 +406,15 @@ MGR_HD void pair_large_adj(const DevModel& m, const double* sl, double nu, const
                            double dz, const PairS& f, double g_dt, double g_Slo, double g_Shi, const AdjAcc& acc,
                            double& g_sh_o, double& g_sh_i) {
     const double d = f.dtau;
-    const double gd = g_dt - g_Slo * f.Slo / d - g_Shi * f.Shi / d;
-    const double gsc = g_Slo / d, gsn = g_Shi / d;
-    const double gsd = (d == f.sum_dtau) ? gd : 0.0;  // a clamped dtau does not move
-    const double cf = nu * outer.shift, nf = nu * inner.shift;
+    // one line in reach and no clamp: the sources are the line's own, S = (ld S) / ld
+    const bool own = f.one && d == f.sum_dtau;
+    double gsd = 0.0, gsc = 0.0, gsn = 0.0;
+    if (!own) {
+        gsc = g_Slo / d;
+        gsn = g_Shi / d;
+        if (d == f.sum_dtau) gsd = g_dt - gsc * f.Slo - gsn * f.Shi;  // a clamped dtau does not move
+    }
+    const double cf = dmul_rn(nu, outer.shift), nf = dmul_rn(nu, inner.shift);
     uint32_t a, b;
     pair_bracket<AP>(m, sl, cf, nf, outer.nr, inner.nr, a, b);
     uint32_t wa = a, wb = b;
@@ -353,39 +427,53 @@ MGR_HD void pair_large_adj(const DevModel& m, const double* sl, double nu, const
         // per point: [outer nr, outer ni, inner nr, inner ni]
         double gop[4] = {0.0, 0.0, 0.0, 0.0}, giw[4] = {0.0, 0.0, 0.0, 0.0}, gsp[4] = {0.0, 0.0, 0.0, 0.0};
         if (s >= a && s < b) {
-            const double ld = ld_s(m, outer, inner, l, cf, nf, dz);
             const double lsc = ilog_s(m.Sp[c1 + l], m.Sp[c2 + l], fo);
             const double lsn = ilog_s(m.Sp[n1 + l], m.Sp[n2 + l], fi);
-            const double gld = gsd + gsc * lsc + gsn * lsn;
-            const double glsc = gsc * ld, glsn = gsn * ld;
-            const LdAdj r = ld_s_adj(m, outer, inner, l, cf, nf, dz, gld);
+            double gld = g_dt, glsc = g_Slo, glsn = g_Shi, E = f.E;
+            if (!own) {
+                const double ld = ld_s(m, outer, inner, l, cf, nf, dz, E, f.one);
+                gld = gsd + gsc * lsc + gsn * lsn;
+                glsc = gsc * ld;
+                glsn = gsn * ld;
+            }
+            const LdAdj r = ld_s_adj(m, outer, inner, l, cf, nf, dz, gld, E);
             g_sh_o += r.g_cf * nu;
             g_sh_i += r.g_nf * nu;
-            const double cop = ilog_s(m.op[c1 + l], m.op[c2 + l], fo);
-            const double nop = ilog_s(m.op[n1 + l], m.op[n2 + l], fi);
-            gop[0] = r.g_cop * (1.0 - fo) * cop / m.op[c1 + l];
-            gop[2] = r.g_nop * (1.0 - fi) * nop / m.op[n1 + l];
-            giw[0] = r.g_iwc * (1.0 - fo);
-            giw[2] = r.g_iwn * (1.0 - fi);
-            gsp[0] = glsc * (1.0 - fo) * lsc / m.Sp[c1 + l];
-            gsp[2] = glsn * (1.0 - fi) * lsn / m.Sp[n1 + l];
+            gop[0] = r.g_cop;
+            gop[2] = r.g_nop;
+            giw[0] = r.g_iwc;
+            giw[2] = r.g_iwn;
+            gsp[0] = glsc;
+            gsp[2] = glsn;
             if (fo != 0.0) {
+                const double cop = ilog_s(m.op[c1 + l], m.op[c2 + l], fo);
+                gop[0] = r.g_cop * (1.0 - fo) * cop / m.op[c1 + l];
+                giw[0] = r.g_iwc * (1.0 - fo);
+                gsp[0] = glsc * (1.0 - fo) * lsc / m.Sp[c1 + l];
                 gop[1] = r.g_cop * fo * cop / m.op[c2 + l];
                 giw[1] = r.g_iwc * fo;
                 gsp[1] = glsc * fo * lsc / m.Sp[c2 + l];
             }
             if (fi != 0.0) {
+                const double nop = ilog_s(m.op[n1 + l], m.op[n2 + l], fi);
+                gop[2] = r.g_nop * (1.0 - fi) * nop / m.op[n1 + l];
+                giw[2] = r.g_iwn * (1.0 - fi);
+                gsp[2] = glsn * (1.0 - fi) * lsn / m.Sp[n1 + l];
                 gop[3] = r.g_nop * fi * nop / m.op[n2 + l];
                 giw[3] = r.g_iwn * fi;
                 gsp[3] = glsn * fi * lsn / m.Sp[n2 + l];
             }
         }
-        const uint32_t pts[4] = {outer.nr, outer.ni, inner.nr, inner.ni};
-        for (int j = 0; j < 4; j++) {
-            if ((j == 1 && fo == 0.0) || (j == 3 && fi == 0.0)) continue;
-            acc.add(ADJ_OP, pts[j], l, gop[j]);
-            acc.add(ADJ_IW, pts[j], l, giw[j]);
-            acc.add(ADJ_SP, pts[j], l, gsp[j]);
+        // the elements' first points, then the second points of subdivided steps
+        for (int j = 0; j < 2; j++) {
+            if (j == 1 && fo == 0.0 && fi == 0.0) continue;
+            const bool to_o = j == 0 || fo != 0.0, to_i = j == 0 || fi != 0.0;
+            const uint32_t po = j ? outer.ni : outer.nr, pi = j ? inner.ni : inner.nr;
+            double* const to[6] = {to_o ? acc.at(ADJ_OP, po, l) : nullptr, to_o ? acc.at(ADJ_IW, po, l) : nullptr,
+                                   to_o ? acc.at(ADJ_SP, po, l) : nullptr, to_i ? acc.at(ADJ_OP, pi, l) : nullptr,
+                                   to_i ? acc.at(ADJ_IW, pi, l) : nullptr, to_i ? acc.at(ADJ_SP, pi, l) : nullptr};
+            const double v[6] = {gop[j], giw[j], gsp[j], gop[2 + j], giw[2 + j], gsp[2 + j]};
+            acc.add6(to, v);
         }
     }
 }
@@ -396,13 +484,13 @@ MGR_HD void elem_shift_adj(const Elem& e, double g_shift, const AdjAcc& acc) {
     if (e.fac != 0.0) acc.add_shift(e.ni, g_shift * e.fac);
 }
 
-// Scratch of one lane: elimination state after pair k, (F, Su, dtau) at
-// scr[(3 k + j) * stride].
+// Scratch of one lane: elimination state after pair k, (F, Su, dtau, erf difference) at
+// scr[(4 k + j) * stride].
 struct LaneScratch {
     double* p;
     int stride;
     uint32_t cap;  // pairs
-    MGR_HD double& at(uint32_t k, int j) const { return p[(size_t)(3 * k + j) * stride]; }
+    MGR_HD double& at(uint32_t k, int j) const { return p[(size_t)(4 * k + j) * stride]; }
 };
 
 // Smooth forward of one pixel ray for one frequency (image_lane with nb > 0, nf = 0):
@@ -423,6 +511,7 @@ MGR_HD double image_lane_s(const DevModel& m, const double* sl, uint32_t o, doub
     iter_next<MODE_FP64>(m, bk, o, kAllLines, it, prev);
     const double Ib = bdy_s(m, prev.nr, nu * prev.shift, dummy);
     double F = 0.0, Su = 0.0, dt_prev = 0.0, S_last = 0.0;
+    ElemVal v_prev{0.0, 0.0, false};
     uint32_t k = 0;
     bool done = false;
     while (!done) {
@@ -431,7 +520,9 @@ MGR_HD double image_lane_s(const DevModel& m, const double* sl, uint32_t o, doub
             cur = cen;
             done = true;
         }
-        const PairS ps = pair_s<AP>(m, sl, nu, prev, cur, prev.dzin);
+        ElemVal v_cur{0.0, 0.0, false};
+        const PairS ps = pair_s<AP>(m, sl, nu, prev, cur, prev.dzin, v_prev, v_cur);
+        v_prev = v_cur;
         const double dt = ps.dtau;
         if (k == 0) {
             // first row, Su = (S + 2 Ib/dt) / (1 + 2/dt + 2/dt^2) and F = (1 + 2/dt) dt^2/2,
@@ -454,6 +545,7 @@ MGR_HD double image_lane_s(const DevModel& m, const double* sl, uint32_t o, doub
             scr->at(k, 0) = F;
             scr->at(k, 1) = Su;
             scr->at(k, 2) = dt;
+            scr->at(k, 3) = ps.E;
         }
         dt_prev = dt;
         S_last = ps.Shi;
@@ -503,10 +595,14 @@ MGR_HD bool image_lane_adj(const DevModel& m, const double* sl, uint32_t o, doub
     double carry_eta = 0.0, carry_chi = 0.0;  // adjoint of the inner element's eta/chi from the pair outside it
     bool have_carry = false;
     double g_sh_inner_carry = 0.0;  // shift adjoint of the inner element from the pair outside it
+    ElemVal v_inner{0.0, 0.0, false};
     for (uint32_t kk = M; kk-- > 0;) {
         iter_up_next<MODE_FP64>(m, bk, o, kAllLines, it, outer);
         const double dz = outer.dzin;
-        const PairS ps = pair_s<AP>(m, sl, nu, outer, inner, dz);
+        const double E = scr.at(kk, 3);
+        ElemVal v_outer{0.0, 0.0, false};
+        const PairS ps = pair_s<AP>(m, sl, nu, outer, inner, dz, v_outer, v_inner, &E);
+        v_inner = v_outer;
         double gSlo = 0.0, gShi = 0.0;
         if (kk == M - 1) {
             const double N = Su_last + ps.Shi * (0.5 * dtl * dtl) + Ibl * dtl;

@@ -3,14 +3,14 @@
 // Solver::solve_feautrier_order_2, solver.tpp:458-540), plus the device-pointer update
 // of the model's frequencies that an autograd wrapper needs between calls.
 //
-// Both kernels run one warp per origin (grid-stride over the origins, or over a list
-// of them).  The warp walks the ray pairs in order, tracing both halves into shared
-// memory; for each line it runs the lanes over that line's quadrature points (so all
-// lanes share the ray's elements, which the adjoint's warp sums need), and J(o, f) is
-// accumulated in shared memory in the reference's ray-pair order.  The backward keeps
-// each lane's per-pair elimination state in a scratch array of the warp's slot
-// (recomputed, not saved by the forward) and adds its derivatives with one atomic per
-// warp and entry.
+// Both kernels run one warp per (origin, ray pair), over every origin or a list of them: a
+// warp per origin left a 1k-point model on 8 warps an SM, each walking its ray pairs one
+// after another.  The warp traces both halves into shared memory; for each line it runs the
+// lanes over that line's quadrature points (so all lanes share the ray's elements, which the
+// adjoint's warp sums need).  The forward stages u and a second kernel sums J(o, f) in the
+// reference's ray-pair order.  The backward keeps each lane's per-pair elimination state in a
+// scratch array of the warp's slot (recomputed, not saved by the forward) and adds its
+// derivatives with one atomic per warp and entry.
 #include <algorithm>
 #include <vector>
 
@@ -19,50 +19,52 @@
 
 namespace mgr {
 
+// u of the listed origins i0 .. i1 - 1 (every origin without a list) along every ray pair:
+// U[((i - i0) * hnrays + rr) * F + f].
 template <int AP>
 __global__ void __launch_bounds__(256) fo2_s_kernel(DevModel m, uint32_t cap, const uint32_t* __restrict__ olist,
-                                                    uint32_t n_o, double* __restrict__ J, int* status) {
+                                                    uint32_t i0, uint32_t i1, double* __restrict__ U, int* status) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int nw = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t Lpad = (m.L + 1) & ~1u, Fpad = (m.F + 1) & ~1u;
+    const uint32_t Lpad = (m.L + 1) & ~1u;
     double* sl = reinterpret_cast<double*>(smem);
-    double* Jacc = sl + Lpad + (size_t)w * Fpad;
     HalfSmem bk, fw;
-    carve_halves(smem + ((size_t)Lpad + (size_t)nw * Fpad) * 8 + (size_t)w * half_bytes_per_warp(cap), cap, bk, fw);
+    carve_halves(smem + (size_t)Lpad * 8 + (size_t)w * half_bytes_per_warp(cap), cap, bk, fw);
     for (uint32_t i = threadIdx.x; i < m.L; i += blockDim.x) sl[i] = m.sorted_line[i];
     __syncthreads();
-    for (uint32_t item = blockIdx.x * nw + w; item < n_o; item += gridDim.x * nw) {
-        const uint32_t o = olist ? olist[item] : item;
-        for (uint32_t f = lane; f < m.F; f += 32) Jacc[f] = 0.0;
-        __syncwarp();
-        bool ok = true;
-        for (uint32_t rr = 0; rr < m.hnrays; rr++) {
-            int nb = 0, nf = 0;
-            trace_pair<true, 0, 1>(m, o, rr, m.antipod[rr], cap, bk, fw, lane, status, nb, nf);
-            if (nb < 0 || nf < 0) {
-                ok = false;  // status recorded by the trace
-                break;
-            }
-            const double wt = 2.0 * ray_w(m, o, rr);
-            for (uint32_t l = 0; l < m.L; l++)
-                for (uint32_t q0 = 0; q0 < m.Q; q0 += 32) {
-                    const uint32_t q = q0 + lane;
-                    if (q < m.Q) {
-                        const uint32_t f = m.lq2f[(size_t)l * m.Q + q];
-                        const LaneS r = solve_lane_s<AP>(m, sl, o, m.nu[(size_t)o * m.F + f], l, bk, nb, fw, nf,
-                                                         nullptr);
-                        Jacc[f] += r.u * wt;
-                    }
+    const uint64_t n = (uint64_t)(i1 - i0) * m.hnrays;
+    for (uint64_t item = (uint64_t)blockIdx.x * nw + w; item < n; item += (uint64_t)gridDim.x * nw) {
+        const uint32_t i = i0 + (uint32_t)(item / m.hnrays), rr = (uint32_t)(item % m.hnrays);
+        const uint32_t o = olist ? olist[i] : i;
+        int nb = 0, nf = 0;
+        trace_pair<true, 0, 1>(m, o, rr, m.antipod[rr], cap, bk, fw, lane, status, nb, nf);
+        if (nb < 0 || nf < 0) continue;  // status recorded by the trace
+        for (uint32_t l = 0; l < m.L; l++)
+            for (uint32_t q0 = 0; q0 < m.Q; q0 += 32) {
+                const uint32_t q = q0 + lane;
+                if (q < m.Q) {
+                    const uint32_t f = m.lq2f[(size_t)l * m.Q + q];
+                    const LaneS r = solve_lane_s<AP>(m, sl, o, m.nu[(size_t)o * m.F + f], l, bk, nb, fw, nf, nullptr);
+                    U[(size_t)item * m.F + f] = r.u;
                 }
-            __syncwarp();
-        }
-        if (ok)
-            for (uint32_t f = lane; f < m.F; f += 32) {
-                const double v = Jacc[f];
-                J[(size_t)o * m.F + f] = v;
-                if (!isfinite(v)) atomicOr(status, ST_NONFINITE);
             }
         __syncwarp();
+    }
+}
+
+// J of the origins, summed over the ray pairs in order.
+__global__ void __launch_bounds__(256) fo2_s_sum_kernel(DevModel m, const uint32_t* __restrict__ olist, uint32_t i0,
+                                                        uint32_t i1, const double* __restrict__ U,
+                                                        double* __restrict__ J, int* status) {
+    const uint64_t n = (uint64_t)(i1 - i0) * m.F;
+    for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t i = i0 + (uint32_t)(k / m.F), f = (uint32_t)(k % m.F);
+        const uint32_t o = olist ? olist[i] : i;
+        double v = 0.0;
+        for (uint32_t rr = 0; rr < m.hnrays; rr++)
+            v += U[((size_t)(i - i0) * m.hnrays + rr) * m.F + f] * (2.0 * ray_w(m, o, rr));
+        J[(size_t)o * m.F + f] = v;
+        if (!isfinite(v)) atomicOr(status, ST_NONFINITE);
     }
 }
 
@@ -73,74 +75,68 @@ __global__ void __launch_bounds__(256) fo2_adj_kernel(DevModel m, uint32_t cap, 
                                                       uint32_t scratch_pairs, int* status) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int nw = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t Lpad = (m.L + 1) & ~1u, Fpad = (m.F + 1) & ~1u;
+    const uint32_t Lpad = (m.L + 1) & ~1u;
     double* sl = reinterpret_cast<double*>(smem);
-    double* gnu_acc = sl + Lpad + (size_t)w * Fpad;
     HalfSmem bk, fw;
-    carve_halves(smem + ((size_t)Lpad + (size_t)nw * Fpad) * 8 + (size_t)w * half_bytes_per_warp(cap), cap, bk, fw);
+    carve_halves(smem + (size_t)Lpad * 8 + (size_t)w * half_bytes_per_warp(cap), cap, bk, fw);
     for (uint32_t i = threadIdx.x; i < m.L; i += blockDim.x) sl[i] = m.sorted_line[i];
     __syncthreads();
     const size_t slot = (size_t)blockIdx.x * nw + w;
-    const Fo2Scratch scr{scratch + slot * (size_t)scratch_pairs * 4 * 32 + lane, 32, scratch_pairs};
-    for (uint32_t item = blockIdx.x * nw + w; item < n_o; item += gridDim.x * nw) {
-        const uint32_t o = olist ? olist[item] : item;
+    const Fo2Scratch scr{scratch + slot * (size_t)scratch_pairs * 5 * 32 + lane, 32, scratch_pairs};
+    const uint64_t n = (uint64_t)n_o * m.hnrays;
+    for (uint64_t item = (uint64_t)blockIdx.x * nw + w; item < n; item += (uint64_t)gridDim.x * nw) {
+        const uint32_t i = (uint32_t)(item / m.hnrays), rr = (uint32_t)(item % m.hnrays);
+        const uint32_t o = olist ? olist[i] : i;
         // origins without a derivative of the loss contribute nothing
         bool any = false;
         for (uint32_t f = lane; f < m.F; f += 32) any |= gJ[(size_t)o * m.F + f] != 0.0;
         if (!__any_sync(FULL_MASK, any)) continue;
-        for (uint32_t f = lane; f < m.F; f += 32) gnu_acc[f] = 0.0;
-        __syncwarp();
         double vo[3] = {0.0, 0.0, 0.0};
-        for (uint32_t rr = 0; rr < m.hnrays; rr++) {
-            const uint32_t ar = m.antipod[rr];
-            int nb = 0, nf = 0;
-            trace_pair<true, 0, 1>(m, o, rr, ar, cap, bk, fw, lane, status, nb, nf);
-            if (nb < 0 || nf < 0) break;
-            const double* db = ray_dir(m, o, rr);
-            const double* df = ray_dir(m, o, ar);
-            AdjGrads gb = g, gf = g;
-            for (int k = 0; k < 3; k++) {
-                gb.d[k] = db[k];
-                gf.d[k] = df[k];
-            }
-            const AdjAcc acc_b{gb, m.L}, acc_f{gf, m.L};
-            const double wt = 2.0 * ray_w(m, o, rr);
-            for (uint32_t l = 0; l < m.L; l++)
-                for (uint32_t q0 = 0; q0 < m.Q; q0 += 32) {
-                    const uint32_t q = q0 + lane;
-                    const uint32_t f = m.lq2f[(size_t)l * m.Q + (q < m.Q ? q : m.Q - 1)];
-                    const double gu = q < m.Q ? gJ[(size_t)o * m.F + f] * wt : 0.0;
-                    if (!__any_sync(FULL_MASK, gu != 0.0)) continue;
-                    double gvb = 0.0, gvf = 0.0, gn = 0.0;
-                    if (!solve_lane_s_adj<AP>(m, sl, o, m.nu[(size_t)o * m.F + f], l, bk, nb, fw, nf, gu, scr,
-                                              acc_b, acc_f, gvb, gvf, gn)) {
-                        if (lane == 0) atomicOr(status, ST_CAPACITY);
-                        continue;
-                    }
-                    for (int k = 0; k < 3; k++) vo[k] += gvb * db[k] + gvf * df[k];
-                    if (q < m.Q) gnu_acc[f] += gn;
-                    __syncwarp();
-                }
+        const uint32_t ar = m.antipod[rr];
+        int nb = 0, nf = 0;
+        trace_pair<true, 0, 1>(m, o, rr, ar, cap, bk, fw, lane, status, nb, nf);
+        if (nb < 0 || nf < 0) continue;
+        const double* db = ray_dir(m, o, rr);
+        const double* df = ray_dir(m, o, ar);
+        AdjGrads gb = g, gf = g;
+        for (int k = 0; k < 3; k++) {
+            gb.d[k] = db[k];
+            gf.d[k] = df[k];
         }
+        const AdjAcc acc_b{gb, m.L}, acc_f{gf, m.L};
+        const double wt = 2.0 * ray_w(m, o, rr);
+        for (uint32_t l = 0; l < m.L; l++)
+            for (uint32_t q0 = 0; q0 < m.Q; q0 += 32) {
+                const uint32_t q = q0 + lane;
+                const uint32_t f = m.lq2f[(size_t)l * m.Q + (q < m.Q ? q : m.Q - 1)];
+                const double gu = q < m.Q ? gJ[(size_t)o * m.F + f] * wt : 0.0;
+                if (!__any_sync(FULL_MASK, gu != 0.0)) continue;
+                double gvb = 0.0, gvf = 0.0, gn = 0.0;
+                if (!solve_lane_s_adj<AP>(m, sl, o, m.nu[(size_t)o * m.F + f], l, bk, nb, fw, nf, gu, scr, acc_b, acc_f,
+                                          gvb, gvf, gn)) {
+                    if (lane == 0) atomicOr(status, ST_CAPACITY);
+                    continue;
+                }
+                for (int k = 0; k < 3; k++) vo[k] += gvb * db[k] + gvf * df[k];
+                if (q < m.Q && gn != 0.0) atomicAdd(g_nu + (size_t)o * m.F + f, gn);
+                __syncwarp();
+            }
         for (int k = 0; k < 3; k++) {
             double v = vo[k];
             for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(FULL_MASK, v, off);
             if (lane == 0 && v != 0.0) atomicAdd(g.vel + 3 * (size_t)o + k, v);
         }
         __syncwarp();
-        for (uint32_t f = lane; f < m.F; f += 32) g_nu[(size_t)o * m.F + f] += gnu_acc[f];
-        __syncwarp();
     }
 }
 
-// Launch shape of the per-origin kernels: CTAs of up to 8 warps whose ray buffers and
-// per-warp frequency accumulators fit in shared memory.
+// Launch shape of the kernels: CTAs of up to 8 warps whose ray buffers fit in shared memory.
 template <typename K>
 static cudaError_t origin_launch_shape(MgrModel* model, K kern, uint32_t cap, uint64_t items, int* nw_out,
                                        size_t* smem_out, unsigned* grid_out) {
-    const uint32_t Lpad = (model->dm.L + 1) & ~1u, Fpad = (model->dm.F + 1) & ~1u;
+    const uint32_t Lpad = (model->dm.L + 1) & ~1u;
     int nw = 8;
-    auto bytes = [&](int n) { return ((size_t)Lpad + (size_t)n * Fpad) * 8 + (size_t)n * half_bytes_per_warp(cap); };
+    auto bytes = [&](int n) { return (size_t)Lpad * 8 + (size_t)n * half_bytes_per_warp(cap); };
     while (nw > 1 && bytes(nw) > 200 * 1024) nw /= 2;
     const size_t smem = bytes(nw);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -158,6 +154,9 @@ static cudaError_t origin_launch_shape(MgrModel* model, K kern, uint32_t cap, ui
     *grid_out = (unsigned)grid;
     return cudaSuccess;
 }
+
+// Staged u of a pass of the smooth forward at most.
+constexpr size_t kSmoothStageBytes = size_t(1) << 30;
 
 static int check_smooth_model(MgrModel* model, const char* who) {
     if (!model->line_disc) {
@@ -221,12 +220,30 @@ int mgr_formal_solve_fo2_smooth_device(MgrModel* model, const uint32_t* origins_
     int nw;
     size_t smem;
     unsigned grid;
+    // u staged in the work area, for as many origins at a time as a pass of kSmoothStageBytes
+    // (or the area there is) holds
+    const size_t per = (size_t)model->dm.hnrays * model->dm.F * sizeof(double);
+    const size_t want = std::min<size_t>(n_o, std::max<size_t>(1, kSmoothStageBytes / per)) * per;
+    if (!grow_work(model, want) && model->work_bytes < per)
+        return cuda_fail(cudaErrorMemoryAllocation, "mgr_formal_solve_fo2_smooth_device: staging");
+    const uint32_t pass = (uint32_t)std::min<size_t>(n_o, model->work_bytes / per);
     auto run = [&](auto kern) -> cudaError_t {
-        cudaError_t r = origin_launch_shape(model, kern, cap, n_o, &nw, &smem, &grid);
-        if (r != cudaSuccess) return r;
-        count_launch();
-        kern<<<grid, nw * 32, smem, model->stream>>>(model->dm, cap, origins_dev, n_o, J_dev, model->status);
-        return cudaGetLastError();
+        for (uint32_t i0 = 0; i0 < n_o; i0 += pass) {
+            const uint32_t i1 = n_o - i0 > pass ? i0 + pass : n_o;
+            cudaError_t r = origin_launch_shape(model, kern, cap, (uint64_t)(i1 - i0) * model->dm.hnrays, &nw, &smem,
+                                                &grid);
+            if (r != cudaSuccess) return r;
+            count_launch();
+            kern<<<grid, nw * 32, smem, model->stream>>>(model->dm, cap, origins_dev, i0, i1, model->work, model->status);
+            if ((r = cudaGetLastError()) != cudaSuccess) return r;
+            const uint64_t threads = (uint64_t)(i1 - i0) * model->dm.F;
+            const uint64_t blocks = std::min<uint64_t>((threads + 255) / 256, (uint64_t)model->sm_count * 16);
+            count_launch();
+            fo2_s_sum_kernel<<<(unsigned)blocks, 256, 0, model->stream>>>(model->dm, origins_dev, i0, i1, model->work,
+                                                                          J_dev, model->status);
+            if ((r = cudaGetLastError()) != cudaSuccess) return r;
+        }
+        return cudaSuccess;
     };
     cudaError_t e = (model->dm.approx == APPROX_CLOSELINES) ? run(fo2_s_kernel<APPROX_CLOSELINES>)
                                                              : run(fo2_s_kernel<APPROX_NONE>);
@@ -263,9 +280,9 @@ int mgr_formal_solve_fo2_adjoint_device(MgrModel* model, const uint32_t* origins
     size_t smem;
     unsigned grid;
     auto run = [&](auto kern) -> cudaError_t {
-        cudaError_t r = origin_launch_shape(model, kern, cap, n_o, &nw, &smem, &grid);
+        cudaError_t r = origin_launch_shape(model, kern, cap, (uint64_t)n_o * model->dm.hnrays, &nw, &smem, &grid);
         if (r != cudaSuccess) return r;
-        const size_t need = (size_t)grid * nw * pairs * 4 * 32 * sizeof(double);
+        const size_t need = (size_t)grid * nw * pairs * 5 * 32 * sizeof(double);
         if (model->adj_scratch_bytes < need) {  // grown on demand, kept for the next call
             cudaFree(model->adj_scratch);
             model->adj_scratch = nullptr;

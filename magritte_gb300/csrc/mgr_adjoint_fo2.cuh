@@ -27,13 +27,13 @@
 
 namespace mgr {
 
-// Per-pair scratch of one lane: (F, Su, dtau, row source) of pair k at
-// p[(4 k + j) * stride]; the backward half's pairs come first, then the forward half's.
+// Per-pair scratch of one lane: (F, Su, dtau, row source, erf difference) of pair k at
+// p[(5 k + j) * stride]; the backward half's pairs come first, then the forward half's.
 struct Fo2Scratch {
     double* p;
     int stride;
     uint32_t cap;  // pairs
-    MGR_HD double& at(uint32_t k, int j) const { return p[(size_t)(4 * k + j) * stride]; }
+    MGR_HD double& at(uint32_t k, int j) const { return p[(size_t)(5 * k + j) * stride]; }
 };
 
 // End state of one half's elimination toward the origin.
@@ -63,6 +63,7 @@ MGR_HD HalfS half_s(const DevModel& m, const double* sl, uint32_t o, double nu, 
     double dummy;
     const double Ib = bdy_s(m, prev.nr, nu * prev.shift, dummy);
     double F = 0.0, Su = 0.0, dt_prev = 0.0, S_carry = 0.0;
+    ElemVal v_prev{0.0, 0.0, false};
     uint32_t k = 0;
     bool done = false;
     while (!done) {
@@ -71,7 +72,9 @@ MGR_HD HalfS half_s(const DevModel& m, const double* sl, uint32_t o, double nu, 
             cur = cen;
             done = true;
         }
-        const PairS ps = pair_s<AP>(m, sl, nu, prev, cur, prev.dzin);
+        ElemVal v_cur{0.0, 0.0, false};
+        const PairS ps = pair_s<AP>(m, sl, nu, prev, cur, prev.dzin, v_prev, v_cur);
+        v_prev = v_cur;
         const double dt = ps.dtau;
         const double S_row = (side == 0 || k == 0) ? ps.Slo : S_carry;
         if (k == 0) {
@@ -93,6 +96,7 @@ MGR_HD HalfS half_s(const DevModel& m, const double* sl, uint32_t o, double nu, 
             scr->at(k0 + k, 1) = Su;
             scr->at(k0 + k, 2) = dt;
             scr->at(k0 + k, 3) = S_row;
+            scr->at(k0 + k, 4) = ps.E;
         }
         dt_prev = dt;
         S_carry = ps.Shi;
@@ -192,10 +196,14 @@ MGR_HD void half_s_adj(const DevModel& m, const double* sl, uint32_t o, double n
     bool have_carry = false;
     double g_sh_carry = 0.0;  // inner element's shift adjoint from the pair outside it
     double gShi_pend = gSin;  // adjoint of the current pair's inner source (next row's or the origin's)
+    ElemVal v_inner{0.0, 0.0, false};
     for (uint32_t kk = n; kk-- > 0;) {
         iter_up_next<MODE_FP64>(m, h, o, l, it, outer);
         const double dz = outer.dzin;
-        const PairS ps = pair_s<AP>(m, sl, nu, outer, inner, dz);
+        const double E = scr.at(k0 + kk, 4);
+        ElemVal v_outer{0.0, 0.0, false};
+        const PairS ps = pair_s<AP>(m, sl, nu, outer, inner, dz, v_outer, v_inner, &E);
+        v_inner = v_outer;
         const double dt = scr.at(k0 + kk, 2);
         const double S_row = scr.at(k0 + kk, 3);
         double g_dt_k, gSrow, g_sh_o = 0.0;

@@ -200,7 +200,7 @@ static cudaError_t launch_image_t(MgrModel* model, uint32_t rr, double* I) {
 constexpr size_t kImageRayBytes = size_t(1) << 30;
 
 // The model's work area grown to `bytes`; false (and the area as it was) when it cannot be.
-static bool grow_work(MgrModel* model, size_t bytes) {
+bool grow_work(MgrModel* model, size_t bytes) {
     if (model->work_bytes >= bytes) return true;
     void* q = nullptr;
     if (cudaMalloc(&q, bytes) != cudaSuccess) {

@@ -169,6 +169,8 @@ cudaError_t launch_fo2_range(MgrModel* model, int precision, uint32_t o_begin, u
                              double* lam, double* work, size_t work_bytes, uint32_t rr_begin = 0,
                              uint32_t rr_end = 0xffffffffu, double* Jlin = nullptr, double* anis = nullptr,
                              double* v = nullptr, double* alo_off = nullptr, uint32_t* alo_nr = nullptr);
+// The model's work area grown to `bytes`; false (and the area as it was) when it cannot be.
+bool grow_work(MgrModel* model, size_t bytes);
 cudaError_t launch_trace_export(MgrModel* model, uint32_t o, uint32_t rr, uint32_t l, uint32_t capacity,
                                 uint32_t* d_meta, uint32_t* d_nr, uint32_t* d_ni, double* d_fac, double* d_shift,
                                 double* d_dZ);
