@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(128)
         const size_t stride = (size_t)m.P * m.F;
         reduce_J_origin(m, o, 0, m.hnrays, Um, stride, 0, Jout[mi], threadIdx.x, blockDim.x);
         if (LD && Lout[mi])
-            reduce_lam_origin(m, o, 0, m.hnrays, LD + (stage_off[mi] - s0), stride, 0, Lout[mi], w, nw, lane);
+            reduce_lam_origin(m, o, 0, m.hnrays, LD + (stage_off[mi] - s0), nullptr, stride, 0, Lout[mi], w, nw, lane);
         __syncthreads();
         if (threadIdx.x == 0) {
             __threadfence();

@@ -498,7 +498,7 @@ __global__ void __launch_bounds__(128) fo2_reduce_kernel(DevModel m, uint32_t o_
                 }
             }
         }
-        if (lam) reduce_lam_origin(m, o, rr0, nR, LD, ld_stride, ld_o0, lam, w, nw, lane);
+        if (lam) reduce_lam_origin(m, o, rr0, nR, LD, nullptr, ld_stride, ld_o0, lam, w, nw, lane);
     }
 }
 

@@ -17,37 +17,58 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// Threads t = 0 .. nt-1 over the frequencies.
+// Both sums run over values that are already in L2 or stream from memory; what bound them was
+// the FP64 pipe (one warp instruction per 16 cycles and SM), six multiplications and an
+// addition per ALO element.  The factors that do not depend on the ray pair stand outside the
+// sums over it: one multiplication-addition per element of either sum.
+// ray_w(o, rr0 + k) as a pointer over k
+__device__ __forceinline__ const double* ray_weights(const DevModel& m, uint32_t o, uint32_t rr0) {
+    return m.rayw + (m.adaptive ? (size_t)o * m.nrays : (size_t)0) + rr0;
+}
+
+// Threads t = 0 .. nt-1 over the frequencies.  2 w u is summed as w u, doubled at the end: exact.
 __device__ __forceinline__ void reduce_J_origin(const DevModel& m, uint32_t o, uint32_t rr0, uint32_t nR,
                                                 const double* __restrict__ U, size_t u_stride, uint32_t u_o0,
                                                 double* __restrict__ J, int t, int nt) {
+    const double* wr = ray_weights(m, o, rr0);
     for (uint32_t f = (uint32_t)t; f < m.F; f += (uint32_t)nt) {
         const double* Uo = U + (size_t)(o - u_o0) * m.F + f;
         double s = 0.0;
-        for (uint32_t k = 0; k < nR; k++) s += Uo[(size_t)k * u_stride] * 2.0 * ray_w(m, o, rr0 + k);
-        J[(size_t)o * m.F + f] = s;
+#pragma unroll 8
+        for (uint32_t k = 0; k < nR; k++) s = fma(Uo[(size_t)k * u_stride], wr[k], s);
+        J[(size_t)o * m.F + f] = s * 2.0;
     }
 }
 
-// Warps w = 0 .. nw-1 over the lines, lanes over the quadrature points.
+// Warps w = 0 .. nw-1 over the lines, lanes over the quadrature points.  X: one array of
+// L_diag, weighted 2 w (X2 null), or the two directions' factors of the short
+// characteristics, each weighted w (lambda_element_sc0; 0 where no pair was solved).
 __device__ __forceinline__ void reduce_lam_origin(const DevModel& m, uint32_t o, uint32_t rr0, uint32_t nR,
-                                                  const double* __restrict__ LD, size_t ld_stride, uint32_t ld_o0,
-                                                  double* __restrict__ lam, int w, int nw, int lane) {
+                                                  const double* __restrict__ X, const double* __restrict__ X2,
+                                                  size_t x_stride, uint32_t x_o0, double* __restrict__ lam, int w,
+                                                  int nw, int lane) {
+    const double* wr = ray_weights(m, o, rr0);
     for (uint32_t l = (uint32_t)w; l < m.L; l += (uint32_t)nw) {
-        // lane q: the ray-independent factors of quadrature point q, then its elements
-        // over the ray pairs in order
+        // lane q: its elements over the ray pairs in order, then the ray-independent factors
         const uint32_t* l2f = m.lq2f + (size_t)l * m.Q;
         double s = 0.0;
         for (uint32_t q0 = 0; q0 < m.Q; q0 += 32) {
             const uint32_t q = q0 + lane;
             const uint32_t f = q < m.Q ? l2f[q] : 0xffffffffu;
             if (f == 0xffffffffu || !m.in_line[f]) continue;
-            const LambdaFactors k = lambda_factors(m, m.sorted_line, o, f);
+            const double* Xo = X + (size_t)(o - x_o0) * m.F + f;
             double part = 0.0;
-            for (uint32_t rr = rr0; rr < rr0 + nR; rr++)
-                part += lambda_element(k, ray_w(m, o, rr),
-                                       LD[(size_t)(rr - rr0) * ld_stride + (size_t)(o - ld_o0) * m.F + f]);
-            s += part;
+            if (X2) {
+                const double* X2o = X2 + (size_t)(o - x_o0) * m.F + f;
+#pragma unroll 4
+                for (uint32_t k = 0; k < nR; k++)
+                    part = fma(Xo[(size_t)k * x_stride] + X2o[(size_t)k * x_stride], wr[k], part);
+            } else {
+#pragma unroll 8
+                for (uint32_t k = 0; k < nR; k++) part = fma(Xo[(size_t)k * x_stride], wr[k], part);
+                part *= 2.0;
+            }
+            s += lambda_element_sc0(lambda_factors(m, m.sorted_line, o, f), part, 1.0);
         }
         s = warp_sum(s);
         if (lane == 0) lam[(size_t)o * m.L + l] = s;

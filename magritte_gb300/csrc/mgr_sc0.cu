@@ -10,6 +10,7 @@
 // then backward direction).
 #include "mgr_ali.h"
 #include "mgr_internal.h"
+#include "mgr_reduce.cuh"
 #include "mgr_solve.cuh"
 
 namespace mgr {
@@ -75,43 +76,9 @@ __global__ void __launch_bounds__(128) sc0_reduce_kernel(DevModel m, uint32_t o_
     const int nw = blockDim.x >> 5;
     const int w = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    const uint32_t R = m.hnrays;
     for (uint32_t o = o_begin + blockIdx.x; o < o_end; o += gridDim.x) {
-        for (uint32_t f = threadIdx.x; f < m.F; f += blockDim.x) {
-            const double* Uo = U + (size_t)(o - u_o0) * m.F + f;
-            double s = 0.0;
-            for (uint32_t rr = 0; rr < R; rr++) s += (ray_w(m, o, rr) * 2.0) * Uo[(size_t)rr * u_stride];
-            J[(size_t)o * m.F + f] = s;
-        }
-        if (!lam) continue;
-        for (uint32_t l = w; l < m.L; l += nw) {
-            const uint32_t* l2f = m.lq2f + (size_t)l * m.Q;
-            double s = 0.0;
-            for (uint32_t rr = 0; rr < R; rr++) {
-                const size_t xo = (size_t)rr * x_stride + (size_t)(o - x_o0) * m.F;
-                for (uint32_t q0 = 0; q0 < m.Q; q0 += 32) {
-                    const uint32_t q = q0 + lane;
-                    const uint32_t f = q < m.Q ? l2f[q] : 0xffffffffu;
-                    double ef = 0.0, eb = 0.0;
-                    bool add = false;
-                    if (f != 0xffffffffu && m.in_line[f]) {
-                        const double xf = XF[xo + f], xb = XB[xo + f];
-                        add = (xf != 0.0) || (xb != 0.0);  // solved pairs only (update_Lambda per direction)
-                        if (add) {
-                            const LambdaFactors k = lambda_factors(m, m.sorted_line, o, f);
-                            ef = lambda_element_sc0(k, ray_w(m, o, rr), xf);
-                            eb = lambda_element_sc0(k, ray_w(m, o, rr), xb);
-                        }
-                    }
-                    const uint32_t nq = min(32u, m.Q - q0);
-                    for (uint32_t j = 0; j < nq; j++) {
-                        s += __shfl_sync(FULL_MASK, ef, j);
-                        s += __shfl_sync(FULL_MASK, eb, j);
-                    }
-                }
-            }
-            if (lane == 0) lam[(size_t)o * m.L + l] = s;
-        }
+        reduce_J_origin(m, o, 0, m.hnrays, U, u_stride, u_o0, J, threadIdx.x, blockDim.x);
+        if (lam) reduce_lam_origin(m, o, 0, m.hnrays, XF, XB, x_stride, x_o0, lam, w, nw, lane);
     }
 }
 
