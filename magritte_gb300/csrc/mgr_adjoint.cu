@@ -177,7 +177,8 @@ static int adj_plane(MgrModel* model, const char* who, const double* raydir, uin
     uint32_t* dmax = nullptr;
     cudaError_t e = cudaMalloc(d_xy, 2 * hx.size() * 8);
     if (e == cudaSuccess) e = cudaMalloc(&dmax, sizeof(uint32_t));
-    if (e == cudaSuccess) e = image_plane_upload(model, ip, hx, hy, *d_xy, dmax, cap);
+    if (e == cudaSuccess) e = image_plane_upload(model, ip, hx, hy, *d_xy, dmax);
+    if (e == cudaSuccess) e = image_size(model, ip, dmax, cap);
     cudaFree(dmax);
     if (e != cudaSuccess) {
         cudaFree(*d_xy);

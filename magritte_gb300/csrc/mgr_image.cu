@@ -106,7 +106,8 @@ __global__ void __launch_bounds__(256) image_new_kernel(DevModel m, ImagePlane i
 template <int MODE>
 __global__ void __launch_bounds__(256) image_trace_kernel(const __grid_constant__ DevModel m, ImagePlane ip,
                                                           uint32_t cap, uint32_t px0, uint32_t px1,
-                                                          unsigned char* __restrict__ rays, int* status) {
+                                                          unsigned char* __restrict__ rays,
+                                                          uint32_t* __restrict__ d_max, int* status) {
     constexpr int LAY = (MODE == MODE_SPLIT) ? LAY_SPLIT : LAY_FP64;
     const int lane = threadIdx.x & 31;
     const uint32_t px = px0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -117,8 +118,9 @@ __global__ void __launch_bounds__(256) image_trace_kernel(const __grid_constant_
     pixel_origin(ip, ip.ImX[px], ip.ImY[px], org);
     double Z;
     const uint32_t start = pixel_start(m, org, ip, lane, Z);
-    const int n = trace_image<true, LAY>(m, org, ip, start, Z, cap, h, lane, status);
+    const int n = trace_image<true, LAY, true>(m, org, ip, start, Z, cap, h, lane, status);
     if (lane == 0) {
+        if (n > 0) atomicMax(d_max, (uint32_t)n);
         HalfHead<MODE>* hd = reinterpret_cast<HalfHead<MODE>*>(base);
         const double sh0 = image_shift(m, org, ip, start, Z);
         if constexpr (MODE == MODE_SPLIT) {
@@ -143,9 +145,9 @@ __global__ void __launch_bounds__(256, MINB)
     for (uint32_t px = px0 + blockIdx.x * nw + w; px < px1; px += gridDim.x * nw) {
         unsigned char* half = rays + (size_t)(px - px0) * staged_half_bytes(MODE, cap);
         const HalfHead<MODE>* hd = reinterpret_cast<const HalfHead<MODE>*>(half);
-        if (hd->n < 0) continue;  // status recorded by the trace
-        // rays without an interior point and non-finite values are the general kernel's
-        bool again = hd->n == 0;
+        // rays without an interior point, longer than cap, and non-finite values are the
+        // general kernel's
+        bool again = hd->n == 0 || hd->n > (int)cap;
         if (!again)
             again = staged_image<MODE, AP>(m, cap, mine, half, hd->start, lane, [&](uint32_t f, double v, bool& bad) {
                 I[(size_t)px * m.F + f] = v;
@@ -199,7 +201,6 @@ static cudaError_t launch_image_t(MgrModel* model, uint32_t rr, double* I) {
 // Half rays of a pass of the staged imager at most.
 constexpr size_t kImageRayBytes = size_t(1) << 30;
 
-// The model's work area grown to `bytes`; false (and the area as it was) when it cannot be.
 bool grow_work(MgrModel* model, size_t bytes) {
     if (model->work_bytes >= bytes) return true;
     void* q = nullptr;
@@ -214,10 +215,32 @@ bool grow_work(MgrModel* model, size_t bytes) {
     return true;
 }
 
+// *cap: the steps of the longest pixel ray, recorded in d_max.
+static cudaError_t image_max_steps(MgrModel* model, const uint32_t* d_max, uint32_t* cap) {
+    uint32_t n = 0;
+    cudaError_t e = cudaMemcpyAsync(&n, d_max, sizeof(uint32_t), cudaMemcpyDeviceToHost, model->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(model->stream);
+    *cap = std::max(n, 1u);
+    return e;
+}
+
+cudaError_t image_size(MgrModel* model, const ImagePlane& ip, uint32_t* d_max, uint32_t* cap) {
+    const size_t npix = (size_t)ip.nx * ip.ny;
+    const unsigned blocks = (unsigned)std::min<size_t>((npix * 32 + 255) / 256, (size_t)model->sm_count * 16);
+    count_launch();
+    image_size_kernel<<<blocks ? blocks : 1, 256, 0, model->stream>>>(model->dm, ip, d_max, model->status);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? image_max_steps(model, d_max, cap) : e;
+}
+
 template <int MODE, int AP, bool TAU>
-static cudaError_t launch_image_new_t(MgrModel* model, const ImagePlane& ip, uint32_t cap, double* I) {
+static cudaError_t launch_image_new_t(MgrModel* model, const ImagePlane& ip, uint32_t* d_max, double* I) {
     // Intensities of models whose lines are apart: the staged solve where its rays fit the work
     // area (an image of 151 x 97 pixels x 41 frequencies, FP64, 20k points: see the kernel)
+    // Room for half rays a quarter longer than the formal solve's longest: nearly every pixel's
+    // fits without a walk to size it first (0.63 ms; 3.20 -> 2.57 ms without it), the others are
+    // listed.
+    uint32_t cap = model->half_cap + model->half_cap / 4 + 8;
     const uint32_t npix = ip.nx * ip.ny;
     const size_t hb = staged_half_bytes(MODE, cap), list_bytes = (size_t)(npix + 1) * sizeof(uint32_t);
     const size_t pass = std::max<size_t>(1, std::min<size_t>(npix, kImageRayBytes / hb));
@@ -240,7 +263,7 @@ static cudaError_t launch_image_new_t(MgrModel* model, const ImagePlane& ip, uin
             const uint32_t px0 = (uint32_t)p0, px1 = (uint32_t)std::min<size_t>(npix, p0 + pass), n = px1 - px0;
             count_launch();
             image_trace_kernel<MODE><<<(n + 7) / 8, 256, 0, model->stream>>>(model->dm, ip, cap, px0, px1, rays,
-                                                                            model->status);
+                                                                            d_max, model->status);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
             count_launch();
             kern<<<std::min(full, (n + nw - 1) / nw), nw * 32, tile, model->stream>>>(model->dm, cap, px0, px1, rays, I,
@@ -251,7 +274,8 @@ static cudaError_t launch_image_new_t(MgrModel* model, const ImagePlane& ip, uin
     size_t smem;
     unsigned grid;
     auto kern = image_new_kernel<MODE, AP, TAU>;
-    cudaError_t e = launch_warp_kernel(model, kern, cap, (uint64_t)ip.nx * ip.ny, &smem, &grid);
+    cudaError_t e = staged ? image_max_steps(model, d_max, &cap) : image_size(model, ip, d_max, &cap);
+    if (e == cudaSuccess) e = launch_warp_kernel(model, kern, cap, (uint64_t)ip.nx * ip.ny, &smem, &grid);
     if (e != cudaSuccess) return e;
     const int nw = (int)((smem - (size_t)((model->dm.L + 1) & ~1u) * 8) / half_bytes_per_warp(cap));
     count_launch();
@@ -266,9 +290,9 @@ static cudaError_t dispatch_image(MgrModel* model, uint32_t rr, double* I) {
 }
 
 template <int MODE, bool TAU = false>
-static cudaError_t dispatch_image_new(MgrModel* model, const ImagePlane& ip, uint32_t cap, double* I) {
-    if (model->dm.approx == APPROX_NONE) return launch_image_new_t<MODE, APPROX_NONE, TAU>(model, ip, cap, I);
-    return launch_image_new_t<MODE, APPROX_CLOSELINES, TAU>(model, ip, cap, I);
+static cudaError_t dispatch_image_new(MgrModel* model, const ImagePlane& ip, uint32_t* d_max, double* I) {
+    if (model->dm.approx == APPROX_NONE) return launch_image_new_t<MODE, APPROX_NONE, TAU>(model, ip, d_max, I);
+    return launch_image_new_t<MODE, APPROX_CLOSELINES, TAU>(model, ip, d_max, I);
 }
 
 // Image::set_coordinates_all_model_points, 3D (image.cpp:154-219).
@@ -286,23 +310,13 @@ int image_plane_setup(MgrModel* model, const char* who, const double* raydir, ui
 }
 
 cudaError_t image_plane_upload(MgrModel* model, ImagePlane& ip, const std::vector<double>& hx,
-                               const std::vector<double>& hy, double* d_xy, uint32_t* d_max, uint32_t* cap) {
+                               const std::vector<double>& hy, double* d_xy, uint32_t* d_max) {
     const size_t npix = hx.size();
     cudaError_t e = cudaMemcpyAsync(d_xy, hx.data(), npix * 8, cudaMemcpyHostToDevice, model->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_xy + npix, hy.data(), npix * 8, cudaMemcpyHostToDevice, model->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(d_max, 0, sizeof(uint32_t), model->stream);
     ip.ImX = d_xy;
     ip.ImY = d_xy + npix;
-    *cap = 0;
-    if (e == cudaSuccess) {
-        count_launch();
-        const unsigned blocks = (unsigned)std::min<size_t>((npix * 32 + 255) / 256, (size_t)model->sm_count * 16);
-        image_size_kernel<<<blocks ? blocks : 1, 256, 0, model->stream>>>(model->dm, ip, d_max, model->status);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(cap, d_max, sizeof(uint32_t), cudaMemcpyDeviceToHost, model->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(model->stream);
-    if (*cap < 1) *cap = 1;
     return e;
 }
 
@@ -383,18 +397,17 @@ static int image_new_impl(MgrModel* model, int precision, const double* raydir, 
     const size_t npix = (size_t)nx * ny;
     double *dxy = nullptr, *dI = nullptr;
     uint32_t* dmax = nullptr;
-    uint32_t cap = 0;
     cudaError_t e = cudaMalloc(&dxy, 2 * npix * 8);
     if (e == cudaSuccess) e = cudaMalloc(&dI, npix * dm.F * 8);
     if (e == cudaSuccess) e = cudaMalloc(&dmax, sizeof(uint32_t));
-    if (e == cudaSuccess) e = image_plane_upload(model, ip, hx, hy, dxy, dmax, &cap);
+    if (e == cudaSuccess) e = image_plane_upload(model, ip, hx, hy, dxy, dmax);
     if (e == cudaSuccess) {
         if (tau)
-            e = (precision == MGR_PRECISION_SPLIT) ? dispatch_image_new<MODE_SPLIT, true>(model, ip, cap, dI)
-                                                   : dispatch_image_new<MODE_FP64, true>(model, ip, cap, dI);
+            e = (precision == MGR_PRECISION_SPLIT) ? dispatch_image_new<MODE_SPLIT, true>(model, ip, dmax, dI)
+                                                   : dispatch_image_new<MODE_FP64, true>(model, ip, dmax, dI);
         else
-            e = (precision == MGR_PRECISION_SPLIT) ? dispatch_image_new<MODE_SPLIT>(model, ip, cap, dI)
-                                                   : dispatch_image_new<MODE_FP64>(model, ip, cap, dI);
+            e = (precision == MGR_PRECISION_SPLIT) ? dispatch_image_new<MODE_SPLIT>(model, ip, dmax, dI)
+                                                   : dispatch_image_new<MODE_FP64>(model, ip, dmax, dI);
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(I, dI, npix * dm.F * 8, cudaMemcpyDeviceToHost, model->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(model->stream);

@@ -96,8 +96,9 @@ static __host__ __device__ __forceinline__ double image_shift(const DevModel& m,
 // boundary point through the model until it leaves on the far side; rest-frame
 // shifts 1 + v . d of a motionless observer.  Returns the steps stored, 0 if the ray
 // met no interior point (the reference then keeps only the start point), -1 on
-// capacity overflow.
-template <bool STORE, int LAY = LAY_FULL>
+// capacity overflow; with OVER the walk counts on instead, storing cap steps, and a result
+// above cap means that the ray isn't there.
+template <bool STORE, int LAY = LAY_FULL, bool OVER = false>
 static __device__ int trace_image(const DevModel& m, const double* org, const ImagePlane& ip, uint32_t start, double Z,
                            uint32_t cap, HalfSmem h, int lane, int* status) {
     const double dx = ip.d[0], dy = ip.d[1], dz = ip.d[2];
@@ -113,13 +114,13 @@ static __device__ int trace_image(const DevModel& m, const double* org, const Im
             uint32_t nxt;
             double dZl;
             if (!next_point_sph(m, Rcos, Rsin2, crt, Z, nxt, dZl)) break;
-            if (STORE && (uint32_t)count >= cap) {
+            if (STORE && !OVER && (uint32_t)count >= cap) {
                 if (lane == 0) atomicOr(status, ST_CAPACITY);
                 count = -1;
                 break;
             }
             Z = dadd_rn(Z, dZl);
-            if (STORE && lane == 0) {
+            if (STORE && lane == 0 && (!OVER || (uint32_t)count < cap)) {
                 h.ids[count] = nxt;
                 h.eid[count] = sph_eid(crt, nxt);
                 store_dz<LAY>(m, h, count, dZl);
@@ -172,7 +173,7 @@ static __device__ int trace_image(const DevModel& m, const double* org, const Im
             }
         }
         if (besti == 0xffffffffu) break;  // no next point: the walk ends here
-        if (STORE && (uint32_t)count >= cap) {
+        if (STORE && !OVER && (uint32_t)count >= cap) {
             if (lane == 0) atomicOr(status, ST_CAPACITY);
             count = -1;
             break;
@@ -180,7 +181,7 @@ static __device__ int trace_image(const DevModel& m, const double* org, const Im
         const uint32_t nxt = (uint32_t)__double_as_longlong(m.edge[cum + besti].w);
         const double dZl = dsub_rn(bestZ, Z);
         Z = dadd_rn(Z, dZl);
-        if (STORE && lane == 0) {
+        if (STORE && lane == 0 && (!OVER || (uint32_t)count < cap)) {
             h.ids[count] = nxt;
             h.eid[count] = cum + besti;
             store_dz<LAY>(m, h, count, dZl);
@@ -199,7 +200,7 @@ static __device__ int trace_image(const DevModel& m, const double* org, const Im
     }
     __syncwarp();
     if (count > 0 && !accessed) count = 0;
-    if (STORE && count > 0) {
+    if (STORE && count > 0 && (!OVER || (uint32_t)count <= cap)) {
         for (int s = lane; s < count; s += 32) {
             const double4_32a v = m.vel[h.ids[s]];
             store_shift<LAY>(h, s, dadd_rn(1.0, dot3_rn(v.x, v.y, v.z, dx, dy, dz)));
@@ -365,8 +366,11 @@ int image_plane_setup(MgrModel* model, const char* who, const double* raydir, ui
                       ImagePlane& ip, std::vector<double>& hx, std::vector<double>& hy);
 
 // Uploads the pixel coordinates into d_xy [2*nx*ny] (device, owned by the caller), points
-// ip.ImX / ip.ImY at them and sizes the longest pixel ray (trace steps) into *cap.
+// ip.ImX / ip.ImY at them and clears d_max.
 cudaError_t image_plane_upload(MgrModel* model, ImagePlane& ip, const std::vector<double>& hx,
-                               const std::vector<double>& hy, double* d_xy, uint32_t* d_max, uint32_t* cap);
+                               const std::vector<double>& hy, double* d_xy, uint32_t* d_max);
+
+// *cap: the steps of the longest pixel ray, by walking them all.
+cudaError_t image_size(MgrModel* model, const ImagePlane& ip, uint32_t* d_max, uint32_t* cap);
 
 }  // namespace mgr
