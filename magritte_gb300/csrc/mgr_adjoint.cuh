@@ -40,10 +40,11 @@ MGR_HD double ilog_s(double a, double b, double f) {
 }
 
 // erf(a) - erf(b) without cancellation when a and b lie on the same side of 0
-// (differences of erfc there, which keeps its relative precision in the wings).
+// (differences of erfc there, which keeps its relative precision in the wings; one site for
+// both sides: a warp's frequencies usually lie on both).
 static __host__ __device__ __noinline__ double erf_diff_s(double a, double b) {
-    if (a > 0.0 && b > 0.0) return erfc(b) - erfc(a);
-    if (a < 0.0 && b < 0.0) return erfc(-a) - erfc(-b);
+    const bool above = a > 0.0 && b > 0.0;
+    if (above || (a < 0.0 && b < 0.0)) return erfc(above ? b : -a) - erfc(above ? a : -b);
     return erf(a) - erf(b);
 }
 
@@ -161,45 +162,56 @@ MGR_HD uint32_t line_of(const DevModel& m, uint32_t s) {
     return (AP == APPROX_CLOSELINES) ? m.sorted_map[s] : s;
 }
 
+// A sweep's element, once evaluated: emissivity, opacity and source, the lines that contribute,
+// and the profile of the last of them.
+struct ElemVal {
+    double eta, chi, S, prof;
+    uint32_t lo, hi;
+    bool ok;
+};
+
 // Element emissivity and opacity (eta_chi_fp64, smooth).
 template <int AP>
-MGR_HD void elem_s(const DevModel& m, const double* sl, double nu, const Elem& e, double& eta, double& chi) {
+MGR_HD void elem_s(const DevModel& m, const double* sl, double nu, const Elem& e, ElemVal& v) {
     const double freq = dmul_rn(nu, e.shift);
-    uint32_t lo, hi;
-    elem_bracket<AP>(m, sl, freq, e.nr, lo, hi);
+    elem_bracket<AP>(m, sl, freq, e.nr, v.lo, v.hi);
     const size_t b1 = (size_t)e.nr * m.L, b2 = (size_t)e.ni * m.L;
-    eta = 0.0;
-    chi = m.min_opacity;
-    for (uint32_t s = lo; s < hi; s++) {
+    v.eta = 0.0;
+    v.chi = m.min_opacity;
+    v.prof = 0.0;
+#pragma unroll 1
+    for (uint32_t s = v.lo; s < v.hi; s++) {
         const uint32_t l = line_of<AP>(m, s);
         const double diff = freq - m.line[l];
         const double iw = interpolate_linear(m.iw[b1 + l], m.iw[b2 + l], e.fac);
-        const double prof = gauss_s(iw, diff);
-        eta += prof * ilog_s(m.em[b1 + l], m.em[b2 + l], e.fac);
-        chi += prof * ilog_s(m.op[b1 + l], m.op[b2 + l], e.fac);
+        v.prof = gauss_s(iw, diff);
+        v.eta += v.prof * ilog_s(m.em[b1 + l], m.em[b2 + l], e.fac);
+        v.chi += v.prof * ilog_s(m.op[b1 + l], m.op[b2 + l], e.fac);
     }
+    v.S = v.eta / v.chi;
+    v.ok = true;
 }
 
 // Adjoint of elem_s: d(loss)/d(eta), d(loss)/d(chi) of the element -> per-point
 // line data and the element's shift (returned in g_shift, to be split over its two
 // points by the caller).
 template <int AP>
-MGR_HD void elem_s_adj(const DevModel& m, const double* sl, double nu, const Elem& e, double g_eta, double g_chi,
+MGR_HD void elem_s_adj(const DevModel& m, double nu, const Elem& e, const ElemVal& v, double g_eta, double g_chi,
                        const AdjAcc& acc, double& g_shift) {
     const double freq = dmul_rn(nu, e.shift);
-    uint32_t lo, hi;
-    elem_bracket<AP>(m, sl, freq, e.nr, lo, hi);
+    const uint32_t lo = v.lo, hi = v.hi;
     uint32_t wlo = lo, whi = hi;
     warp_range(wlo, whi);
     const size_t b1 = (size_t)e.nr * m.L, b2 = (size_t)e.ni * m.L;
     const double f = e.fac;
+#pragma unroll 1
     for (uint32_t s = wlo; s < whi; s++) {
         const uint32_t l = line_of<AP>(m, s);
         double gem_nr = 0.0, gem_ni = 0.0, gop_nr = 0.0, gop_ni = 0.0, giw_nr = 0.0, giw_ni = 0.0;
         if (s >= lo && s < hi) {
             const double diff = freq - m.line[l];
             const double iw = interpolate_linear(m.iw[b1 + l], m.iw[b2 + l], f);
-            const double prof = gauss_s(iw, diff);
+            const double prof = (hi == lo + 1) ? v.prof : gauss_s(iw, diff);
             const double x = iw * diff;
             const double emE = ilog_s(m.em[b1 + l], m.em[b2 + l], f);
             const double opE = ilog_s(m.op[b1 + l], m.op[b2 + l], f);
@@ -223,8 +235,8 @@ MGR_HD void elem_s_adj(const DevModel& m, const double* sl, double nu, const Ele
         double* const to[6] = {acc.at(ADJ_EM, e.nr, l), acc.at(ADJ_OP, e.nr, l), acc.at(ADJ_IW, e.nr, l),
                                two ? acc.at(ADJ_EM, e.ni, l) : nullptr, two ? acc.at(ADJ_OP, e.ni, l) : nullptr,
                                two ? acc.at(ADJ_IW, e.ni, l) : nullptr};
-        const double v[6] = {gem_nr, gop_nr, giw_nr, gem_ni, gop_ni, giw_ni};
-        acc.add6(to, v);
+        const double g[6] = {gem_nr, gop_nr, giw_nr, gem_ni, gop_ni, giw_ni};
+        acc.add6(to, g);
     }
 }
 
@@ -319,10 +331,10 @@ MGR_HD LdAdj ld_s_adj(const DevModel& m, const Elem& lo, const Elem& hi, uint32_
 struct PairS {
     bool large;
     double dtau, Slo, Shi;
-    double eta_o, chi_o, eta_i, chi_i;  // trapezoid branch
-    double sum_dtau;                     // large branch, before the clamp
-    double E;                            // large branch with one line in reach: its erf difference
-    bool one;                            // large branch with one line in reach
+    double chi_o, chi_i;  // trapezoid branch
+    double sum_dtau;      // large branch, before the clamp
+    double E;             // large branch with one line in reach: its erf difference
+    uint32_t a, b;        // large branch: the lines in reach
 };
 
 template <int AP>
@@ -332,32 +344,24 @@ MGR_HD bool pair_large(const DevModel& m, const Elem& outer, const Elem& inner) 
     return dshift_abs > (a < b ? a : b);
 }
 
-// A sweep's element between two pairs: emissivity and opacity, once evaluated.
-struct ElemVal {
-    double eta, chi;
-    bool ok;
-};
-
 // oc / ic: the outer / inner element's values if already known (evaluated and stored
-// otherwise, trapezoid branch).  E: the pair's erf difference if known (one line in reach).
+// otherwise, trapezoid branch).  E, dt: in the reverse sweep, the pair's erf difference (of one
+// line in reach) and its optical depth as the forward pass left them.
 template <int AP>
 MGR_HD PairS pair_s(const DevModel& m, const double* sl, double nu, const Elem& outer, const Elem& inner, double dz,
-                    ElemVal& oc, ElemVal& ic, const double* E = nullptr) {
+                    ElemVal& oc, ElemVal& ic, const double* E = nullptr, const double* dt = nullptr) {
     PairS r{};
     r.large = pair_large<AP>(m, outer, inner);
     if (!r.large) {
         for (int k = 0; k < 2; k++) {  // one site of elem_s
             ElemVal& v = k ? ic : oc;
             if (v.ok) continue;
-            elem_s<AP>(m, sl, nu, k ? inner : outer, v.eta, v.chi);
-            v.ok = true;
+            elem_s<AP>(m, sl, nu, k ? inner : outer, v);
         }
-        r.eta_o = oc.eta;
         r.chi_o = oc.chi;
-        r.eta_i = ic.eta;
         r.chi_i = ic.chi;
-        r.Slo = r.eta_o / r.chi_o;
-        r.Shi = r.eta_i / r.chi_i;
+        r.Slo = oc.S;
+        r.Shi = ic.S;
         r.dtau = 0.5 * (r.chi_o + r.chi_i) * dz;
         return r;
     }
@@ -370,12 +374,25 @@ MGR_HD PairS pair_s(const DevModel& m, const double* sl, double nu, const Elem& 
     pair_bracket<AP>(m, sl, cf, nf, outer.nr, inner.nr, a, b);
     const size_t c1 = (size_t)outer.nr * m.L, c2 = (size_t)outer.ni * m.L;
     const size_t n1 = (size_t)inner.nr * m.L, n2 = (size_t)inner.ni * m.L;
-    r.one = b == a + 1;
+    r.a = a;
+    r.b = b;
+    const bool one = b == a + 1;
     if (E) r.E = *E;
+    const double bound_min_dtau = m.min_opacity * dz;
+    // one line in reach and the depth not the clamp's (or the bare floor's, where the line adds
+    // nothing): the depth is the line's own, the sources are its own
+    if (dt && one && (AP == APPROX_NONE || *dt != bound_min_dtau || *E == 0.0)) {
+        const uint32_t l = line_of<AP>(m, a);
+        r.dtau = r.sum_dtau = *dt;
+        r.Slo = ilog_s(m.Sp[c1 + l], m.Sp[c2 + l], outer.fac);
+        r.Shi = ilog_s(m.Sp[n1 + l], m.Sp[n2 + l], inner.fac);
+        return r;
+    }
     double sd = 0.0, sc = 0.0, sn = 0.0, lsc = 0.0, lsn = 0.0;
+#pragma unroll 1
     for (uint32_t s = a; s < b; s++) {
         const uint32_t l = line_of<AP>(m, s);
-        const double ld = ld_s(m, outer, inner, l, cf, nf, dz, r.E, E && r.one);
+        const double ld = ld_s(m, outer, inner, l, cf, nf, dz, r.E, E && one);
         lsc = ilog_s(m.Sp[c1 + l], m.Sp[c2 + l], outer.fac);
         lsn = ilog_s(m.Sp[n1 + l], m.Sp[n2 + l], inner.fac);
         sd += ld;
@@ -385,11 +402,10 @@ MGR_HD PairS pair_s(const DevModel& m, const double* sl, double nu, const Elem& 
     r.sum_dtau = sd;
     double d = sd;
     if (AP != APPROX_NONE) {
-        const double bound_min_dtau = m.min_opacity * dz;
         if (-bound_min_dtau < d) d = (bound_min_dtau > d) ? bound_min_dtau : d;
     }
     r.dtau = d;
-    if (r.one && d == sd) {  // (ld S) / ld
+    if (one && d == sd) {  // (ld S) / ld
         r.Slo = lsc;
         r.Shi = lsn;
     } else {
@@ -402,12 +418,13 @@ MGR_HD PairS pair_s(const DevModel& m, const double* sl, double nu, const Elem& 
 // Adjoint of a large-shift pair: d(loss)/d(dtau, Slo, Shi) -> per-point line data and
 // the two elements' shifts.
 template <int AP>
-MGR_HD void pair_large_adj(const DevModel& m, const double* sl, double nu, const Elem& outer, const Elem& inner,
+MGR_HD void pair_large_adj(const DevModel& m, double nu, const Elem& outer, const Elem& inner,
                            double dz, const PairS& f, double g_dt, double g_Slo, double g_Shi, const AdjAcc& acc,
                            double& g_sh_o, double& g_sh_i) {
     const double d = f.dtau;
     // one line in reach and no clamp: the sources are the line's own, S = (ld S) / ld
-    const bool own = f.one && d == f.sum_dtau;
+    const uint32_t a = f.a, b = f.b;
+    const bool one = b == a + 1, own = one && d == f.sum_dtau;
     double gsd = 0.0, gsc = 0.0, gsn = 0.0;
     if (!own) {
         gsc = g_Slo / d;
@@ -415,8 +432,6 @@ MGR_HD void pair_large_adj(const DevModel& m, const double* sl, double nu, const
         if (d == f.sum_dtau) gsd = g_dt - gsc * f.Slo - gsn * f.Shi;  // a clamped dtau does not move
     }
     const double cf = dmul_rn(nu, outer.shift), nf = dmul_rn(nu, inner.shift);
-    uint32_t a, b;
-    pair_bracket<AP>(m, sl, cf, nf, outer.nr, inner.nr, a, b);
     uint32_t wa = a, wb = b;
     warp_range(wa, wb);
     const size_t c1 = (size_t)outer.nr * m.L, c2 = (size_t)outer.ni * m.L;
@@ -431,7 +446,7 @@ MGR_HD void pair_large_adj(const DevModel& m, const double* sl, double nu, const
             const double lsn = ilog_s(m.Sp[n1 + l], m.Sp[n2 + l], fi);
             double gld = g_dt, glsc = g_Slo, glsn = g_Shi, E = f.E;
             if (!own) {
-                const double ld = ld_s(m, outer, inner, l, cf, nf, dz, E, f.one);
+                const double ld = ld_s(m, outer, inner, l, cf, nf, dz, E, one);
                 gld = gsd + gsc * lsc + gsn * lsn;
                 glsc = gsc * ld;
                 glsn = gsn * ld;
@@ -465,6 +480,7 @@ MGR_HD void pair_large_adj(const DevModel& m, const double* sl, double nu, const
             }
         }
         // the elements' first points, then the second points of subdivided steps
+#pragma unroll 1
         for (int j = 0; j < 2; j++) {
             if (j == 1 && fo == 0.0 && fi == 0.0) continue;
             const bool to_o = j == 0 || fo != 0.0, to_i = j == 0 || fi != 0.0;
@@ -510,8 +526,8 @@ MGR_HD double image_lane_s(const DevModel& m, const double* sl, uint32_t o, doub
     iter_begin<MODE_FP64>(m, bk, o, kAllLines, nb, it);
     iter_next<MODE_FP64>(m, bk, o, kAllLines, it, prev);
     const double Ib = bdy_s(m, prev.nr, nu * prev.shift, dummy);
-    double F = 0.0, Su = 0.0, dt_prev = 0.0, S_last = 0.0;
-    ElemVal v_prev{0.0, 0.0, false};
+    double F = 0.0, FI = 0.0, Su = 0.0, dt_prev = 0.0, S_last = 0.0;  // FI = 1 / (1 + F)
+    ElemVal v_prev{};
     uint32_t k = 0;
     bool done = false;
     while (!done) {
@@ -520,7 +536,7 @@ MGR_HD double image_lane_s(const DevModel& m, const double* sl, uint32_t o, doub
             cur = cen;
             done = true;
         }
-        ElemVal v_cur{0.0, 0.0, false};
+        ElemVal v_cur{};
         const PairS ps = pair_s<AP>(m, sl, nu, prev, cur, prev.dzin, v_prev, v_cur);
         v_prev = v_cur;
         const double dt = ps.dtau;
@@ -529,13 +545,15 @@ MGR_HD double image_lane_s(const DevModel& m, const double* sl, uint32_t o, doub
             // multiplied through by dt^2/2 (no 1/dt: well conditioned for thin pairs)
             const double h = dt * (0.5 * dt + 1.0);
             F = h;
-            Su = (ps.Slo * (0.5 * dt * dt) + Ib * dt) / (1.0 + h);
+            FI = 1.0 / (1.0 + F);
+            Su = (ps.Slo * (0.5 * dt * dt) + Ib * dt) * FI;
         } else {
             // elimination row with q = A iC = dt / dt_prev
             const double q = dt / dt_prev;
             const double iC = 0.5 * (dt_prev + dt) * dt;
-            F = q * (F / (1.0 + F)) + iC;
-            Su = (q * Su + ps.Slo * iC) / (1.0 + F);
+            F = q * (F * FI) + iC;
+            FI = 1.0 / (1.0 + F);
+            Su = (q * Su + ps.Slo * iC) * FI;
         }
         if (scr) {
             if (k >= scr->cap) {
@@ -592,17 +610,18 @@ MGR_HD bool image_lane_adj(const DevModel& m, const double* sl, uint32_t o, doub
     ElemIter it;
     iter_up_begin<MODE_FP64>(m, bk, o, kAllLines, nb, it);
     Elem inner = cen, outer;
+    double FIk = 1.0 / (1.0 + F_last);
     double carry_eta = 0.0, carry_chi = 0.0;  // adjoint of the inner element's eta/chi from the pair outside it
     bool have_carry = false;
     double g_sh_inner_carry = 0.0;  // shift adjoint of the inner element from the pair outside it
-    ElemVal v_inner{0.0, 0.0, false};
+    ElemVal v_inner{};
     for (uint32_t kk = M; kk-- > 0;) {
         iter_up_next<MODE_FP64>(m, bk, o, kAllLines, it, outer);
         const double dz = outer.dzin;
         const double E = scr.at(kk, 3);
-        ElemVal v_outer{0.0, 0.0, false};
-        const PairS ps = pair_s<AP>(m, sl, nu, outer, inner, dz, v_outer, v_inner, &E);
-        v_inner = v_outer;
+        ElemVal v_outer{};
+        const double dt = scr.at(kk, 2);
+        const PairS ps = pair_s<AP>(m, sl, nu, outer, inner, dz, v_outer, v_inner, &E, &dt);
         double gSlo = 0.0, gShi = 0.0;
         if (kk == M - 1) {
             const double N = Su_last + ps.Shi * (0.5 * dtl * dtl) + Ibl * dtl;
@@ -616,36 +635,34 @@ MGR_HD bool image_lane_adj(const DevModel& m, const double* sl, uint32_t o, doub
             gdt += gN * (ps.Shi * dtl + Ibl) + gh * (dtl + 1.0);
             acc.add_shift(o, gIbl * dB * nu);  // Ibl = B(nu shift(start))
         }
-        const double dt = ps.dtau;
         double g_dt_k;
         double g_sh_o = 0.0, g_sh_i = g_sh_inner_carry;
         if (kk > 0) {
             // pair kk: F_k = q G' + iC, Su_k = Z / (1 + F_k), G' = F'/(1 + F'),
             // Z = q Su' + S iC, q = dt / dto, iC = (dto + dt) dt / 2
             const double Fp = scr.at(kk - 1, 0), Sup = scr.at(kk - 1, 1), dto = scr.at(kk - 1, 2);
-            const double Fk = scr.at(kk, 0);
-            const double q = dt / dto;
+                        const double q = dt / dto;
             const double iC = 0.5 * (dto + dt) * dt;
-            const double FIp = 1.0 / (1.0 + Fp);
+            const double FIp = 1.0 / (1.0 + Fp);  // the next pair's FIk
             const double G = Fp * FIp;
-            const double FIk = 1.0 / (1.0 + Fk);
             const double Z = q * Sup + ps.Slo * iC;
             const double gZ = gSu * FIk;
             const double gFt = gF - gSu * Z * FIk * FIk;
             const double gq = gFt * G + gZ * Sup;
             const double giC = gFt + gZ * ps.Slo;
             gSlo = gZ * iC;
-            g_dt_k = gdt + gq / dto + giC * (0.5 * dto + dt);
+            const double gqd = gq / dto;
+            g_dt_k = gdt + gqd + giC * (0.5 * dto + dt);
             // hand the state adjoint to pair kk - 1
             gF = gFt * q * FIp * FIp;
             gSu = gZ * q;
-            gdt = -gq * q / dto + giC * 0.5 * dt;
+            gdt = giC * 0.5 * dt - gqd * q;
+            FIk = FIp;
         } else {
             // pair 0: F_0 = h, Su_0 = N0 / (1 + h), N0 = S0 dt^2/2 + Ib dt, h = dt (dt/2 + 1)
             double dBf;
             const double Ib = bdy_s(m, outer.nr, nu * outer.shift, dBf);
-            const double h = dt * (0.5 * dt + 1.0);
-            const double FI0 = 1.0 / (1.0 + h);
+            const double FI0 = FIk;  // F_0 = h
             const double N0 = ps.Slo * (0.5 * dt * dt) + Ib * dt;
             const double gN0 = gSu * FI0;
             const double gh = gF - gSu * N0 * FI0 * FI0;
@@ -656,27 +673,27 @@ MGR_HD bool image_lane_adj(const DevModel& m, const double* sl, uint32_t o, doub
         }
         // ---- pair adjoint ----
         if (ps.large) {
-            pair_large_adj<AP>(m, sl, nu, outer, inner, dz, ps, g_dt_k, gSlo, gShi, acc, g_sh_o, g_sh_i);
+            pair_large_adj<AP>(m, nu, outer, inner, dz, ps, g_dt_k, gSlo, gShi, acc, g_sh_o, g_sh_i);
             // the inner element's eta/chi adjoint from the pair outside it is complete
-            if (have_carry) elem_s_adj<AP>(m, sl, nu, inner, carry_eta, carry_chi, acc, g_sh_i);
+            if (have_carry) elem_s_adj<AP>(m, nu, inner, v_inner, carry_eta, carry_chi, acc, g_sh_i);
             carry_eta = carry_chi = 0.0;
             have_carry = false;
         } else {
-            const double ce = carry_eta + gShi / ps.chi_i;
-            const double cc = carry_chi + 0.5 * dz * g_dt_k - gShi * ps.Shi / ps.chi_i;
-            elem_s_adj<AP>(m, sl, nu, inner, ce, cc, acc, g_sh_i);
-            carry_eta = gSlo / ps.chi_o;
-            carry_chi = 0.5 * dz * g_dt_k - gSlo * ps.Slo / ps.chi_o;
+            const double ti = gShi / ps.chi_i, to = gSlo / ps.chi_o, half = 0.5 * dz * g_dt_k;
+            elem_s_adj<AP>(m, nu, inner, v_inner, carry_eta + ti, carry_chi + half - ti * ps.Shi, acc, g_sh_i);
+            carry_eta = to;
+            carry_chi = half - to * ps.Slo;
             have_carry = true;
         }
         elem_shift_adj(inner, g_sh_i, acc);
         if (kk == 0) {
             // element 0 (the far end) is complete
-            if (have_carry) elem_s_adj<AP>(m, sl, nu, outer, carry_eta, carry_chi, acc, g_sh_o);
+            if (have_carry) elem_s_adj<AP>(m, nu, outer, v_outer, carry_eta, carry_chi, acc, g_sh_o);
             elem_shift_adj(outer, g_sh_o, acc);
         }
         g_sh_inner_carry = g_sh_o;
         inner = outer;
+        v_inner = v_outer;
     }
     (void)dummy;
     return true;

@@ -62,8 +62,8 @@ MGR_HD HalfS half_s(const DevModel& m, const double* sl, uint32_t o, double nu, 
     iter_next<MODE_FP64>(m, h, o, l, it, prev);
     double dummy;
     const double Ib = bdy_s(m, prev.nr, nu * prev.shift, dummy);
-    double F = 0.0, Su = 0.0, dt_prev = 0.0, S_carry = 0.0;
-    ElemVal v_prev{0.0, 0.0, false};
+    double F = 0.0, FI = 0.0, Su = 0.0, dt_prev = 0.0, S_carry = 0.0;  // FI = 1 / (1 + F)
+    ElemVal v_prev{};
     uint32_t k = 0;
     bool done = false;
     while (!done) {
@@ -72,7 +72,7 @@ MGR_HD HalfS half_s(const DevModel& m, const double* sl, uint32_t o, double nu, 
             cur = cen;
             done = true;
         }
-        ElemVal v_cur{0.0, 0.0, false};
+        ElemVal v_cur{};
         const PairS ps = pair_s<AP>(m, sl, nu, prev, cur, prev.dzin, v_prev, v_cur);
         v_prev = v_cur;
         const double dt = ps.dtau;
@@ -80,12 +80,14 @@ MGR_HD HalfS half_s(const DevModel& m, const double* sl, uint32_t o, double nu, 
         if (k == 0) {
             const double h0 = dt * (0.5 * dt + 1.0);
             F = h0;
-            Su = (S_row * (0.5 * dt * dt) + Ib * dt) / (1.0 + h0);
+            FI = 1.0 / (1.0 + F);
+            Su = (S_row * (0.5 * dt * dt) + Ib * dt) * FI;
         } else {
             const double q = dt / dt_prev;
             const double iC = 0.5 * (dt_prev + dt) * dt;
-            F = q * (F / (1.0 + F)) + iC;
-            Su = (q * Su + S_row * iC) / (1.0 + F);
+            F = q * (F * FI) + iC;
+            FI = 1.0 / (1.0 + F);
+            Su = (q * Su + S_row * iC) * FI;
         }
         if (scr) {
             if (k0 + k >= scr->cap) {
@@ -131,8 +133,11 @@ MGR_HD LaneS solve_lane_s(const DevModel& m, const double* sl, uint32_t o, doubl
         r.u = bdy_s(m, o, nu, dummy);
         return r;
     }
-    r.top = half_s<AP>(m, sl, o, nu, bk, nb, l, 0, scr, 0);
-    r.bot = half_s<AP>(m, sl, o, nu, fw, nf, l, 1, scr, r.top.n);
+    // one site of the sweep, here and of its reverse: instruction fetch bounds these kernels
+#pragma unroll 1
+    for (int side = 0; side < 2; side++)
+        (side ? r.bot : r.top) =
+            half_s<AP>(m, sl, o, nu, side ? fw : bk, side ? nf : nb, l, side, scr, side ? r.top.n : 0u);
     r.ovf = r.top.ovf || r.bot.ovf;
     if (r.ovf) {
         r.u = 0.0;
@@ -164,10 +169,10 @@ MGR_HD LaneS solve_lane_s(const DevModel& m, const double* sl, uint32_t o, doubl
 // Shift adjoint of an element of a formal-solve ray onto the velocities (comoving
 // shift 1 + (v[p] - v[o]) . n of the element's two points, interpolated with weights
 // 1 - fac / fac; the origin's own shift is exactly 1) and onto the lane's frequency
-// (the element's frequency is nu * shift).  gvo collects the origin's share along n.
-MGR_HD void shift_adj_comoving(const Elem& e, double g, uint32_t o, double nu, const AdjAcc& acc, double& gvo,
-                               double& g_nu) {
-    g_nu += g * e.shift / nu;
+// (the element's frequency is nu * shift; gs is nu times that).  gvo collects the origin's share along n.
+MGR_HD void shift_adj_comoving(const Elem& e, double g, uint32_t o, const AdjAcc& acc, double& gvo,
+                               double& gs) {
+    gs += g * e.shift;
     if (e.nr == o) return;  // the origin element
     const double w_nr = 1.0 - e.fac;
     acc.add_shift(e.nr, g * w_nr);
@@ -192,44 +197,44 @@ MGR_HD void half_s_adj(const DevModel& m, const double* sl, uint32_t o, double n
     ElemIter it;
     iter_up_begin<MODE_FP64>(m, h, o, l, nsteps, it);
     Elem inner = cen, outer;
+    double gs = 0.0;  // nu times the frequency derivative
+    double FIk = 1.0 / (1.0 + scr.at(k0 + n - 1, 0));
     double carry_eta = 0.0, carry_chi = 0.0;  // inner element's eta / chi adjoint from the pair outside it
     bool have_carry = false;
     double g_sh_carry = 0.0;  // inner element's shift adjoint from the pair outside it
     double gShi_pend = gSin;  // adjoint of the current pair's inner source (next row's or the origin's)
-    ElemVal v_inner{0.0, 0.0, false};
+    ElemVal v_inner{};
     for (uint32_t kk = n; kk-- > 0;) {
         iter_up_next<MODE_FP64>(m, h, o, l, it, outer);
         const double dz = outer.dzin;
         const double E = scr.at(k0 + kk, 4);
-        ElemVal v_outer{0.0, 0.0, false};
-        const PairS ps = pair_s<AP>(m, sl, nu, outer, inner, dz, v_outer, v_inner, &E);
-        v_inner = v_outer;
+        ElemVal v_outer{};
         const double dt = scr.at(k0 + kk, 2);
+        const PairS ps = pair_s<AP>(m, sl, nu, outer, inner, dz, v_outer, v_inner, &E, &dt);
         const double S_row = scr.at(k0 + kk, 3);
         double g_dt_k, gSrow, g_sh_o = 0.0;
         if (kk > 0) {
             const double Fp = scr.at(k0 + kk - 1, 0), Sup = scr.at(k0 + kk - 1, 1), dto = scr.at(k0 + kk - 1, 2);
-            const double Fk = scr.at(k0 + kk, 0);
             const double q = dt / dto;
             const double iC = 0.5 * (dto + dt) * dt;
-            const double FIp = 1.0 / (1.0 + Fp);
+            const double FIp = 1.0 / (1.0 + Fp);  // the next pair's FIk
             const double G = Fp * FIp;
-            const double FIk = 1.0 / (1.0 + Fk);
             const double Z = q * Sup + S_row * iC;
             const double gZ = gSu * FIk;
             const double gFt = gF - gSu * Z * FIk * FIk;
             const double gq = gFt * G + gZ * Sup;
             const double giC = gFt + gZ * S_row;
             gSrow = gZ * iC;
-            g_dt_k = gdt + gq / dto + giC * (0.5 * dto + dt);
+            const double gqd = gq / dto;
+            g_dt_k = gdt + gqd + giC * (0.5 * dto + dt);
             gF = gFt * q * FIp * FIp;
             gSu = gZ * q;
-            gdt = -gq * q / dto + giC * 0.5 * dt;
+            gdt = giC * 0.5 * dt - gqd * q;
+            FIk = FIp;
         } else {
             double dBf;
             const double Ib = bdy_s(m, outer.nr, nu * outer.shift, dBf);
-            const double h0 = dt * (0.5 * dt + 1.0);
-            const double FI0 = 1.0 / (1.0 + h0);
+            const double FI0 = FIk;  // F_0 = dt (dt / 2 + 1)
             const double N0 = S_row * (0.5 * dt * dt) + Ib * dt;
             const double gN0 = gSu * FI0;
             const double gh = gF - gSu * N0 * FI0 * FI0;
@@ -242,26 +247,27 @@ MGR_HD void half_s_adj(const DevModel& m, const double* sl, uint32_t o, double n
         gShi_pend = (side == 1 && kk > 0) ? gSrow : 0.0;
         double g_sh_i = g_sh_carry;
         if (ps.large) {
-            pair_large_adj<AP>(m, sl, nu, outer, inner, dz, ps, g_dt_k, gSlo, gShi, acc, g_sh_o, g_sh_i);
-            if (have_carry) elem_s_adj<AP>(m, sl, nu, inner, carry_eta, carry_chi, acc, g_sh_i);
+            pair_large_adj<AP>(m, nu, outer, inner, dz, ps, g_dt_k, gSlo, gShi, acc, g_sh_o, g_sh_i);
+            if (have_carry) elem_s_adj<AP>(m, nu, inner, v_inner, carry_eta, carry_chi, acc, g_sh_i);
             carry_eta = carry_chi = 0.0;
             have_carry = false;
         } else {
-            const double ce = carry_eta + gShi / ps.chi_i;
-            const double cc = carry_chi + 0.5 * dz * g_dt_k - gShi * ps.Shi / ps.chi_i;
-            elem_s_adj<AP>(m, sl, nu, inner, ce, cc, acc, g_sh_i);
-            carry_eta = gSlo / ps.chi_o;
-            carry_chi = 0.5 * dz * g_dt_k - gSlo * ps.Slo / ps.chi_o;
+            const double ti = gShi / ps.chi_i, to = gSlo / ps.chi_o, half = 0.5 * dz * g_dt_k;
+            elem_s_adj<AP>(m, nu, inner, v_inner, carry_eta + ti, carry_chi + half - ti * ps.Shi, acc, g_sh_i);
+            carry_eta = to;
+            carry_chi = half - to * ps.Slo;
             have_carry = true;
         }
-        shift_adj_comoving(inner, g_sh_i, o, nu, acc, gvo, g_nu);
+        shift_adj_comoving(inner, g_sh_i, o, acc, gvo, gs);
         if (kk == 0) {
-            if (have_carry) elem_s_adj<AP>(m, sl, nu, outer, carry_eta, carry_chi, acc, g_sh_o);
-            shift_adj_comoving(outer, g_sh_o, o, nu, acc, gvo, g_nu);
+            if (have_carry) elem_s_adj<AP>(m, nu, outer, v_outer, carry_eta, carry_chi, acc, g_sh_o);
+            shift_adj_comoving(outer, g_sh_o, o, acc, gvo, gs);
         }
         g_sh_carry = g_sh_o;
         inner = outer;
+        v_inner = v_outer;
     }
+    g_nu += gs / nu;
 }
 
 // Adjoint of solve_lane_s for d(loss)/d(u) = gu of one lane: the forward into the
@@ -330,8 +336,11 @@ MGR_HD bool solve_lane_s_adj(const DevModel& m, const double* sl, uint32_t o, do
         g_nu += gN * e * dB;
         gTdt = gN * (T.S_in * e + Ib) + gh * (e + 1.0);
     }
-    half_s_adj<AP>(m, sl, o, nu, bk, nb, l, 0, scr, 0, T.n, gTF, gTSu, gTdt, gTSin, acc_b, gvo_b, g_nu);
-    half_s_adj<AP>(m, sl, o, nu, fw, nf, l, 1, scr, T.n, B.n, gBF, gBSu, gBdt, gBSin, acc_f, gvo_f, g_nu);
+#pragma unroll 1
+    for (int side = 0; side < 2; side++)
+        half_s_adj<AP>(m, sl, o, nu, side ? fw : bk, side ? nf : nb, l, side, scr, side ? T.n : 0u, side ? B.n : T.n,
+                       side ? gBF : gTF, side ? gBSu : gTSu, side ? gBdt : gTdt, side ? gBSin : gTSin,
+                       side ? acc_f : acc_b, side ? gvo_f : gvo_b, g_nu);
     return true;
 }
 
