@@ -461,7 +461,7 @@ int mgr_model_create(const MgrModelDesc* d, MgrModel** out) {
         {
             float4* ehl = nullptr;
             float4* phl = nullptr;
-            if ((e = dalloc(m, &ehl, 2 * (E ? E : 1))) != cudaSuccess) break;
+            if ((e = dalloc(m, &ehl, 2 * (E + 32))) != cudaSuccess) break;
             if ((e = dalloc(m, &phl, 2 * (size_t)P)) != cudaSuccess) break;
             dm.edge_hl = unit_rays ? ehl : nullptr;
             dm.pos_hl = phl;

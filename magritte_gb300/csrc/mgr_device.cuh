@@ -9,7 +9,8 @@
 //     single-precision libm calls (expf, erff, logf, powf, expm1f).
 //   * MGR_PRECISION_SPLIT evaluates profiles, opacities, sources and optical depths in
 //     FP32 (frequencies as FP32 offsets from the line centre, so no catastrophic
-//     cancellation), and keeps the Feautrier elimination in FP64.
+//     cancellation), and keeps the Feautrier elimination in FP64, or in double-float rows
+//     (mgr_staged.cuh).
 #pragma once
 #include <cfloat>
 #include <cstdint>
@@ -52,10 +53,11 @@ struct DevModel {
     const uint32_t* cum_nb;  // [P]
     const double4_32a* edge;     // [E] neighbour position x, y, z and its index (bits of w)
     // FP32 copies for the trace's next-point filter: edge_hl[2i] = neighbour position
-    // times pos_scale as floats (hi) with its index in the bits of w, edge_hl[2i + 1] the
-    // rounding remainders (lo); pos_hl the same per point.  pos_scale is the power of
-    // two that brings every coordinate into [-1, 1].
-    const float4* edge_hl;       // [E][2]
+    // times pos_scale as floats (hi) with its index and boundary flag in the bits of w,
+    // edge_hl[2i + 1] the rounding remainders (lo) with the neighbour's own first record in
+    // the bits of w; pos_hl the positions per point.  pos_scale is the power of two that
+    // brings every coordinate into [-1, 1].
+    const float4* edge_hl;       // [E + 32][2], the last 32 unspecified
     const float4* pos_hl;        // [P][2]
     double pos_scale;
     const uint32_t* p2b;     // [P]

@@ -88,7 +88,9 @@ cudaError_t launch_edge_pack(MgrModel* model, const double4_32a* pos, const uint
 // next-point filter (DevModel::edge_hl, pos_hl), positions scaled by pos_scale.
 // ---------------------------------------------------------------------------------
 __global__ void hl_tables_kernel(const double4_32a* __restrict__ edge, uint64_t E, const double4_32a* __restrict__ pos,
-                                 uint32_t P, double scale, float4* __restrict__ edge_hl, float4* __restrict__ pos_hl) {
+                                 uint32_t P, double scale, const uint32_t* __restrict__ p2b,
+                                 const uint32_t* __restrict__ cum_nb, float4* __restrict__ edge_hl,
+                                 float4* __restrict__ pos_hl) {
     const uint64_t n = E + P;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const bool is_edge = i < E;
@@ -97,8 +99,12 @@ __global__ void hl_tables_kernel(const double4_32a* __restrict__ edge, uint64_t 
         split_hl(dmul_rn(q.x, scale), hi.x, lo.x);
         split_hl(dmul_rn(q.y, scale), hi.y, lo.y);
         split_hl(dmul_rn(q.z, scale), hi.z, lo.z);
-        hi.w = is_edge ? bits_f32((uint32_t)__double_as_longlong(q.w)) : 0.0f;
-        lo.w = 0.0f;
+        hi.w = lo.w = 0.0f;
+        if (is_edge) {
+            const uint32_t nb = (uint32_t)__double_as_longlong(q.w);
+            hi.w = bits_f32(nb | (p2b[nb] != P ? kEdgeBoundary : 0u));
+            lo.w = bits_f32(cum_nb[nb]);
+        }
         if (is_edge && !edge_hl) continue;
         float4* out = is_edge ? edge_hl + 2 * i : pos_hl + 2 * (i - E);
         out[0] = hi;
@@ -112,7 +118,7 @@ cudaError_t launch_hl_tables(MgrModel* model) {
     if (blocks > (uint64_t)model->sm_count * 16) blocks = (uint64_t)model->sm_count * 16;
     count_launch();
     hl_tables_kernel<<<(unsigned)(blocks ? blocks : 1), 256, 0, model->stream>>>(
-        model->dm.edge, model->n_edges, model->dm.pos, model->dm.P, model->dm.pos_scale,
+        model->dm.edge, model->n_edges, model->dm.pos, model->dm.P, model->dm.pos_scale, model->dm.p2b, model->dm.cum_nb,
         const_cast<float4*>(model->dm.edge_hl), const_cast<float4*>(model->dm.pos_hl));
     return cudaGetLastError();
 }
@@ -274,7 +280,7 @@ __global__ void __launch_bounds__(256, MINB)
 // per K consecutive (origin, ray pair) items, results as fo2_kernel's.
 // ---------------------------------------------------------------------------------
 template <int MODE, int GEO>
-__global__ void __launch_bounds__(256) trace_rays_kernel(const __grid_constant__ DevModel m, uint32_t cap,
+__global__ void __launch_bounds__(256, 4) trace_rays_kernel(const __grid_constant__ DevModel m, uint32_t cap,
                                                          uint32_t o_begin, uint32_t rr0, uint32_t nR, uint64_t n_halves,
                                                          unsigned char* __restrict__ rays, int* status) {
     const int lane = threadIdx.x & 31;
@@ -721,7 +727,9 @@ size_t fo2_work_bytes(const MgrModel* model, uint32_t n_origins, bool stage_u, b
 }
 
 // Whether the staged solve serves this model: its tiles hold one line's data, so the
-// frequencies come line by line and pairs that reach several lines are rare.
+// frequencies come line by line and pairs that reach several lines are rare (each of those is
+// solved twice).  33^3 sphere, 4 lines x 31, split: 17.9 ms staged, 42.1 ms by the general kernel;
+// 10^3 cube, 1 line x 11, FP64: 0.22 and 1.34 ms.
 bool staged_ok(const MgrModel* model) {
     const DevModel& m = model->dm;
     if (!model->line_blocks) return false;

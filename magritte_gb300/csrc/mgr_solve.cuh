@@ -260,37 +260,63 @@ MGR_HD int filt_ahead(const FiltCand& c, const TraceF32& t) {
     return diff > tol ? 1 : (diff < -tol ? -1 : 0);
 }
 
-// The filter's step, warp-cooperative (lane i holds neighbour i).  Returns 1 with the
-// next point, its neighbour-record index and its Zf / EZ when the filter decides; 0
-// when no neighbour can lie further along the ray; -1 when the exact argmin must decide.
-__device__ __forceinline__ int warp_next_point_f32(const DevModel& m, const TraceF32& t, uint32_t crt, int lane,
-                                                   uint32_t& nxt, uint32_t& eid, float& Zw, float& EZw) {
+// Index and boundary flag in a neighbour record's edge_hl[2i].w (points number below 2^31: each
+// has a neighbour record, and the records' numbers are 32-bit).
+constexpr uint32_t kEdgeBoundary = 0x80000000u, kEdgeIndex = 0x7fffffffu;
+
+// The filter's step, warp-cooperative (lane i holds neighbour i; cum: crt's first neighbour
+// record).  Returns 1 with the next point, its neighbour-record index, its first record, whether
+// it is a boundary point, and its Zf / EZ when the filter decides; 0 when no neighbour can lie
+// further along the ray; -1 when the exact argmin must decide.  A walk is a chain of such steps,
+// each waiting for the last one's loads: the records carry what the next step's addresses need,
+// the count is loaded beside them (lanes beyond it read on, into the table's padding), and the
+// minimum is one instruction (the bounds are not negative, so they order as integers).
+__device__ __forceinline__ int warp_next_point_f32(const DevModel& m, const TraceF32& t, uint32_t crt, uint32_t cum,
+                                                   int lane, uint32_t& nxt, uint32_t& eid, uint32_t& cum_nxt,
+                                                   bool& bdy, float& Zw, float& EZw) {
+    const float4 a = m.edge_hl[2 * (size_t)(cum + lane)];
+    const float4 b = m.edge_hl[2 * (size_t)(cum + lane) + 1];
     const uint32_t nnb = m.n_nb[crt];
     if (nnb > 32) return -1;
-    const uint32_t cum = m.cum_nb[crt];
-    int ah = -1;
-    FiltCand c{0.0f, 0.0f, 0.0f, 0.0f};
-    uint32_t idx = 0;
-    if ((uint32_t)lane < nnb) {
-        const float4 a = m.edge_hl[2 * (size_t)(cum + lane)];
-        const float4 b = m.edge_hl[2 * (size_t)(cum + lane) + 1];
-        c = filt_cand(a, b, t);
-        ah = filt_ahead(c, t);
-        idx = f32_bits(a.w);
-    }
-    float best = ah > 0 ? c.hi : INFINITY;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) best = fminf(best, __shfl_xor_sync(FULL_MASK, best, off));
+    const FiltCand c = filt_cand(a, b, t);
+    const int ah = (uint32_t)lane < nnb ? filt_ahead(c, t) : -1;
+    const float best = __uint_as_float(__reduce_min_sync(FULL_MASK, __float_as_uint(ah > 0 ? c.hi : INFINITY)));
     const unsigned cont = __ballot_sync(FULL_MASK, ah >= 0 && c.lo <= best);
     if (cont == 0) return 0;
     if (__popc(cont) != 1) return -1;
     const int w = __ffs(cont) - 1;
     if (__shfl_sync(FULL_MASK, ah, w) != 1) return -1;
-    nxt = __shfl_sync(FULL_MASK, idx, w);
+    const uint32_t id = __shfl_sync(FULL_MASK, f32_bits(a.w), w);
+    nxt = id & kEdgeIndex;
+    bdy = (id & kEdgeBoundary) != 0;
+    cum_nxt = __shfl_sync(FULL_MASK, f32_bits(b.w), w);
     eid = cum + (uint32_t)w;
     Zw = __shfl_sync(FULL_MASK, c.Zf, w);
     EZw = __shfl_sync(FULL_MASK, c.EZ, w);
     return 1;
+}
+
+// A step's distance Zn - Z for each of np steps (lane j: the j-th's Zn), chained through
+// Z += Zn - Z.  Z after a step is the step's Zn unless Z + fl(Zn - Z) rounds away from it: the
+// lanes take every step's distance from the previous Zn side by side, and the serial chain
+// runs only when one of the sums does not come back to its Zn (two FP64 warp instructions for
+// up to 32 steps instead of two per step).
+__device__ __forceinline__ double chain_z(double Zn, int np, double& Z, int lane) {
+    const double Zb = __shfl_up_sync(FULL_MASK, Zn, 1);
+    const double Zprev = lane == 0 ? Z : Zb;
+    double dz_lane = dsub_rn(Zn, Zprev);
+    const bool back = __double_as_longlong(dadd_rn(Zprev, dz_lane)) == __double_as_longlong(Zn);
+    if (__all_sync(FULL_MASK, back || lane >= np)) {
+        Z = __shfl_sync(FULL_MASK, Zn, np - 1);
+    } else {
+#pragma unroll 1
+        for (int j = 0; j < np; j++) {
+            const double dZl = dsub_rn(__shfl_sync(FULL_MASK, Zn, j), Z);
+            Z = dadd_rn(Z, dZl);
+            if (lane == j) dz_lane = dZl;
+        }
+    }
+    return dz_lane;
 }
 
 // The walk of trace_half in 1D spherical symmetry (Geometry::get_next_spherical_symmetry,
@@ -416,13 +442,12 @@ __device__ int trace_half(const DevModel& m, uint32_t o, uint32_t r, uint32_t ca
     // The last np steps are pending: lane j holds the point and edge of the j-th of them.
     uint32_t pend = 0, pend_eid = 0;
     int np = 0;
+    const bool filter = FILTER && m.edge_hl;
     uint32_t crt = o;
+    uint32_t cum = filter ? m.cum_nb[o] : 0u;
     int count = 0;
     // Stores the pending steps, one step per lane: exact Zn, dZ, Doppler shift and the FP32
-    // copies.  Z after a step is the step's Zn unless Z + fl(Zn - Z) rounds away from it: the
-    // lanes take every step's distance from the previous Zn side by side, and the serial
-    // chain Z += Zn - Z runs only when one of the sums does not come back to its Zn (two
-    // FP64 warp instructions for up to 32 steps instead of two per step).
+    // copies.
     auto flush = [&]() {
         if (np == 0) return;
         double Zn = 0.0;
@@ -430,20 +455,7 @@ __device__ int trace_half(const DevModel& m, uint32_t o, uint32_t r, uint32_t ca
             const double4_32a q = m.pos[pend];
             Zn = dot3_rn(dsub_rn(q.x, po.x), dsub_rn(q.y, po.y), dsub_rn(q.z, po.z), dx, dy, dz);
         }
-        const double Zb = __shfl_up_sync(FULL_MASK, Zn, 1);
-        const double Zprev = lane == 0 ? Z : Zb;
-        double dz_lane = dsub_rn(Zn, Zprev);
-        const bool back = __double_as_longlong(dadd_rn(Zprev, dz_lane)) == __double_as_longlong(Zn);
-        if (__all_sync(FULL_MASK, back || lane >= np)) {
-            Z = __shfl_sync(FULL_MASK, Zn, np - 1);
-        } else {
-#pragma unroll 1
-            for (int j = 0; j < np; j++) {
-                const double dZl = dsub_rn(__shfl_sync(FULL_MASK, Zn, j), Z);
-                Z = dadd_rn(Z, dZl);
-                if (lane == j) dz_lane = dZl;
-            }
-        }
+        const double dz_lane = chain_z(Zn, np, Z, lane);
         if (STORE && lane < np) {
             const int k = count - np + lane;
             h.ids[k] = pend;
@@ -456,9 +468,10 @@ __device__ int trace_half(const DevModel& m, uint32_t o, uint32_t r, uint32_t ca
     };
 #pragma unroll 1
     while (true) {
-        uint32_t nxt = 0, eid = 0;
+        uint32_t nxt = 0, eid = 0, cum_nxt = 0;
+        bool bdy = false;
         float Zw = 0.0f, EZw = 0.0f;
-        int found = (FILTER && m.edge_hl) ? warp_next_point_f32(m, t, crt, lane, nxt, eid, Zw, EZw) : -1;
+        int found = filter ? warp_next_point_f32(m, t, crt, cum, lane, nxt, eid, cum_nxt, bdy, Zw, EZw) : -1;
         if (found < 0) {
             flush();
             double bestZ;
@@ -466,6 +479,10 @@ __device__ int trace_half(const DevModel& m, uint32_t o, uint32_t r, uint32_t ca
             if (FILTER && found) {
                 Zw = (float)dmul_rn(bestZ, m.pos_scale);
                 EZw = fmaf(2.0f * kU32, fabsf(Zw), 32.0f * kU32Sq);
+            }
+            if (found) {
+                bdy = m.p2b[nxt] != m.P;
+                if (filter) cum_nxt = m.cum_nb[nxt];
             }
         }
         if (!found) {
@@ -492,8 +509,9 @@ __device__ int trace_half(const DevModel& m, uint32_t o, uint32_t r, uint32_t ca
             t.eZc = EZw;
         }
         if (np == 32) flush();
-        if (m.p2b[nxt] != m.P) break;
+        if (bdy) break;
         crt = nxt;
+        cum = cum_nxt;
     }
     if (STORE && count > 0) flush();
     __syncwarp();
