@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(256) image_new_kernel(DevModel m, ImagePlane i
 // memory, image_staged_kernel eliminates; pixels it gives up go to image_new_kernel.
 // ---------------------------------------------------------------------------------
 template <int MODE>
-__global__ void __launch_bounds__(256) image_trace_kernel(const __grid_constant__ DevModel m, ImagePlane ip,
+__global__ void __launch_bounds__(256, 4) image_trace_kernel(const __grid_constant__ DevModel m, ImagePlane ip,
                                                           uint32_t cap, uint32_t px0, uint32_t px1,
                                                           unsigned char* __restrict__ rays,
                                                           uint32_t* __restrict__ d_max, int* status) {
@@ -118,9 +118,10 @@ __global__ void __launch_bounds__(256) image_trace_kernel(const __grid_constant_
     pixel_origin(ip, ip.ImX[px], ip.ImY[px], org);
     double Z;
     const uint32_t start = pixel_start(m, org, ip, lane, Z);
-    const int n = trace_image<true, LAY, true>(m, org, ip, start, Z, cap, h, lane, status);
+    int walked = 0;
+    const int n = trace_image<true, LAY, true>(m, org, ip, start, Z, cap, h, lane, status, &walked);
     if (lane == 0) {
-        if (n > 0) atomicMax(d_max, (uint32_t)n);
+        if (walked > 0) atomicMax(d_max, (uint32_t)walked);
         HalfHead<MODE>* hd = reinterpret_cast<HalfHead<MODE>*>(base);
         const double sh0 = image_shift(m, org, ip, start, Z);
         if constexpr (MODE == MODE_SPLIT) {
@@ -236,10 +237,9 @@ cudaError_t image_size(MgrModel* model, const ImagePlane& ip, uint32_t* d_max, u
 template <int MODE, int AP, bool TAU>
 static cudaError_t launch_image_new_t(MgrModel* model, const ImagePlane& ip, uint32_t* d_max, double* I) {
     // Intensities of models whose lines are apart: the staged solve where its rays fit the work
-    // area (an image of 151 x 97 pixels x 41 frequencies, FP64, 20k points: see the kernel)
-    // Room for half rays a quarter longer than the formal solve's longest: nearly every pixel's
-    // fits without a walk to size it first (0.63 ms; 3.20 -> 2.57 ms without it), the others are
-    // listed.
+    // area (151 x 97 pixels x 41 frequencies, FP64, 20k points: 14.4 ms by the general kernel,
+    // 2.5 ms staged).  Room for half rays a quarter longer than the formal solve's longest: nearly
+    // every pixel's fits without a walk to size it first (0.63 ms), the others are listed.
     uint32_t cap = model->half_cap + model->half_cap / 4 + 8;
     const uint32_t npix = ip.nx * ip.ny;
     const size_t hb = staged_half_bytes(MODE, cap), list_bytes = (size_t)(npix + 1) * sizeof(uint32_t);

@@ -97,10 +97,11 @@ static __host__ __device__ __forceinline__ double image_shift(const DevModel& m,
 // shifts 1 + v . d of a motionless observer.  Returns the steps stored, 0 if the ray
 // met no interior point (the reference then keeps only the start point), -1 on
 // capacity overflow; with OVER the walk counts on instead, storing cap steps, and a result
-// above cap means that the ray isn't there.
+// above cap means that the ray isn't there.  walked: the steps, also of a ray without an
+// interior point, which the buffers have to hold as well.
 template <bool STORE, int LAY = LAY_FULL, bool OVER = false>
 static __device__ int trace_image(const DevModel& m, const double* org, const ImagePlane& ip, uint32_t start, double Z,
-                           uint32_t cap, HalfSmem h, int lane, int* status) {
+                                  uint32_t cap, HalfSmem h, int lane, int* status, int* walked = nullptr) {
     const double dx = ip.d[0], dy = ip.d[1], dz = ip.d[2];
     uint32_t crt = start;
     int count = 0;
@@ -137,58 +138,111 @@ static __device__ int trace_image(const DevModel& m, const double* org, const Im
             crt = nxt;
         }
         __syncwarp();
+        if (walked) *walked = count;
         return count;  // spherically symmetric models keep boundary-only rays (solver.tpp:891-896)
     }
+    // The next point by the FP32 filter of the formal solve's walk, whose bounds hold for unit
+    // directions and for coordinates (scaled, the origin's here up to 4) whose float remainders
+    // are below 4 u^2: image planes further out take the exact argmin at every step.  The exact
+    // argmin alone spent 15 FP64 and 25 shuffle instructions a step.
+    const double sx = dmul_rn(org[0], m.pos_scale), sy = dmul_rn(org[1], m.pos_scale), sz = dmul_rn(org[2], m.pos_scale);
+    const double n2 = dadd_rn(dadd_rn(dmul_rn(dx, dx), dmul_rn(dy, dy)), dmul_rn(dz, dz));
+    const bool filter = m.edge_hl && fabs(dsub_rn(n2, 1.0)) <= 2.0e-15 && fabs(sx) <= 4.0 && fabs(sy) <= 4.0 &&
+                        fabs(sz) <= 4.0;
+    TraceF32 t{};
+    if (filter) {
+        split_hl(sx, t.poh.x, t.pol.x);
+        split_hl(sy, t.poh.y, t.pol.y);
+        split_hl(sz, t.poh.z, t.pol.z);
+        t.dx = (float)dx;
+        t.dy = (float)dy;
+        t.dz = (float)dz;
+        t.Zc = (float)dmul_rn(Z, m.pos_scale);
+        t.eZc = fmaf(2.0f * kU32, fabsf(t.Zc), 32.0f * kU32Sq);
+    }
+    // The last np steps are pending (trace_half): lane j holds the point and edge of the j-th.
+    uint32_t pend = 0, pend_eid = 0;
+    int np = 0;
+    auto flush = [&]() {
+        if (np == 0) return;
+        double Zn = 0.0;
+        if (lane < np) {
+            const double4_32a q = m.pos[pend];
+            Zn = dot3_rn(dsub_rn(q.x, org[0]), dsub_rn(q.y, org[1]), dsub_rn(q.z, org[2]), dx, dy, dz);
+        }
+        const double dz_lane = chain_z(Zn, np, Z, lane);
+        const int k = count - np + lane;
+        if (STORE && lane < np && (!OVER || (uint32_t)k < cap)) {
+            h.ids[k] = pend;
+            h.eid[k] = pend_eid;
+            store_dz<LAY>(m, h, k, dz_lane);
+        }
+        np = 0;
+    };
+    uint32_t cum = m.cum_nb[crt];
     while (true) {
-        const uint32_t nnb = m.n_nb[crt];
-        const uint32_t cum = m.cum_nb[crt];
-        const unsigned long long zkey = dkey(Z);
-        unsigned long long best = ~0ull;
-        uint32_t besti = 0xffffffffu;
-        double bestZ = 0.0;
-        for (uint32_t i = lane; i < nnb; i += 32) {
-            const double4_32a e = m.edge[cum + i];
-            const double Rx = dsub_rn(e.x, org[0]);
-            const double Ry = dsub_rn(e.y, org[1]);
-            const double Rz = dsub_rn(e.z, org[2]);
-            const double Zn = dot3_rn(Rx, Ry, Rz, dx, dy, dz);
-            if (dkey(Zn) > zkey) {
-                const unsigned long long k = dkey(dsub_rn(dot3_rn(Rx, Ry, Rz, Rx, Ry, Rz), dmul_rn(Zn, Zn)));
-                if (k < best) {
-                    best = k;
-                    besti = i;
-                    bestZ = Zn;
+        uint32_t nxt = 0, eid = 0, cum_nxt = 0;
+        bool bdy = false;
+        float Zw = 0.0f, EZw = 0.0f;
+        int found = filter ? warp_next_point_f32(m, t, crt, cum, lane, nxt, eid, cum_nxt, bdy, Zw, EZw) : -1;
+        if (found < 0) {
+            flush();
+            const uint32_t nnb = m.n_nb[crt];
+            const unsigned long long zkey = dkey(Z);
+            unsigned long long best = ~0ull;
+            uint32_t besti = 0xffffffffu;
+            double bestZ = 0.0;
+            for (uint32_t i = lane; i < nnb; i += 32) {
+                const double4_32a e = m.edge[cum + i];
+                const double Rx = dsub_rn(e.x, org[0]);
+                const double Ry = dsub_rn(e.y, org[1]);
+                const double Rz = dsub_rn(e.z, org[2]);
+                const double Zn = dot3_rn(Rx, Ry, Rz, dx, dy, dz);
+                if (dkey(Zn) > zkey) {
+                    const unsigned long long k = dkey(dsub_rn(dot3_rn(Rx, Ry, Rz, Rx, Ry, Rz), dmul_rn(Zn, Zn)));
+                    if (k < best) {
+                        best = k;
+                        besti = i;
+                        bestZ = Zn;
+                    }
                 }
             }
-        }
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const unsigned long long ob = __shfl_xor_sync(FULL_MASK, best, off);
-            const uint32_t oi = __shfl_xor_sync(FULL_MASK, besti, off);
-            const double oz = __shfl_xor_sync(FULL_MASK, bestZ, off);
-            if (ob < best || (ob == best && oi < besti)) {
-                best = ob;
-                besti = oi;
-                bestZ = oz;
+            for (int off = 16; off > 0; off >>= 1) {
+                const unsigned long long ob = __shfl_xor_sync(FULL_MASK, best, off);
+                const uint32_t oi = __shfl_xor_sync(FULL_MASK, besti, off);
+                const double oz = __shfl_xor_sync(FULL_MASK, bestZ, off);
+                if (ob < best || (ob == best && oi < besti)) {
+                    best = ob;
+                    besti = oi;
+                    bestZ = oz;
+                }
+            }
+            found = besti != 0xffffffffu;
+            if (found) {
+                eid = cum + besti;
+                nxt = (uint32_t)__double_as_longlong(m.edge[eid].w);
+                cum_nxt = m.cum_nb[nxt];
+                bdy = m.p2b[nxt] != m.P;
+                Zw = (float)dmul_rn(bestZ, m.pos_scale);
+                EZw = fmaf(2.0f * kU32, fabsf(Zw), 32.0f * kU32Sq);
             }
         }
-        if (besti == 0xffffffffu) break;  // no next point: the walk ends here
+        if (!found) break;  // no next point: the walk ends here
         if (STORE && !OVER && (uint32_t)count >= cap) {
             if (lane == 0) atomicOr(status, ST_CAPACITY);
-            count = -1;
-            break;
+            return -1;
         }
-        const uint32_t nxt = (uint32_t)__double_as_longlong(m.edge[cum + besti].w);
-        const double dZl = dsub_rn(bestZ, Z);
-        Z = dadd_rn(Z, dZl);
-        if (STORE && lane == 0 && (!OVER || (uint32_t)count < cap)) {
-            h.ids[count] = nxt;
-            h.eid[count] = cum + besti;
-            store_dz<LAY>(m, h, count, dZl);
+        if (lane == np) {
+            pend = nxt;
+            pend_eid = eid;
         }
+        np++;
         count++;
-        const bool interior = m.p2b[nxt] == m.P;
-        if (!interior) {
+        t.Zc = Zw;
+        t.eZc = EZw;
+        if (np == 32) flush();
+        if (bdy) {
             const double4_32a pn = m.pos[nxt];
             const double side = dot3_rn(dsub_rn(pn.x, ip.center[0]), dsub_rn(pn.y, ip.center[1]),
                                         dsub_rn(pn.z, ip.center[2]), dx, dy, dz);
@@ -197,8 +251,11 @@ static __device__ int trace_image(const DevModel& m, const double* org, const Im
             accessed = true;
         }
         crt = nxt;
+        cum = cum_nxt;
     }
+    if (STORE) flush();
     __syncwarp();
+    if (walked) *walked = count;
     if (count > 0 && !accessed) count = 0;
     if (STORE && count > 0 && (!OVER || (uint32_t)count <= cap)) {
         for (int s = lane; s < count; s += 32) {
@@ -242,7 +299,8 @@ static __global__ void image_size_kernel(DevModel m, ImagePlane ip, uint32_t* d_
         pixel_origin(ip, ip.ImX[px], ip.ImY[px], org);
         double Z;
         const uint32_t start = pixel_start(m, org, ip, lane, Z);
-        const int n = trace_image<false>(m, org, ip, start, Z, 0xffffffffu, h, lane, status);
+        int n = 0;
+        trace_image<false>(m, org, ip, start, Z, 0xffffffffu, h, lane, status, &n);
         if (lane == 0 && n > 0) atomicMax(d_max, (uint32_t)n);
     }
 }
