@@ -24,9 +24,10 @@
 namespace mgr {
 
 // ---- smooth FP64 counterparts of the reference's profile, interpolation, Planck ----
+// The Gaussian profile divided by the inverse width.
 MGR_HD double gauss_s(double iw, double diff) {
     const double x = iw * diff;
-    return iw * INVERSE_SQRT_PI * exp(-x * x);
+    return INVERSE_SQRT_PI * exp(-x * x);
 }
 
 // a^(1-f) b^f as a (b / a)^f (interpolate_log).  The power, and the erf difference below, are
@@ -145,6 +146,40 @@ struct AdjAcc {
     }
 };
 
+// Line centres are positive, so they order against any number but NaN as integers, off the FP64
+// pipe (half of a bracket's instructions there).
+MGR_HD int64_t line_key(double v) {
+#ifdef __CUDA_ARCH__
+    return __double_as_longlong(v);
+#else
+    int64_t b;
+    std::memcpy(&b, &v, 8);
+    return b;
+#endif
+}
+// lower_bound of left and upper_bound of right among the line centres.
+MGR_HD void lines_between(const double* sl, uint32_t L, double left, double right, uint32_t& a, uint32_t& b) {
+    const int64_t inf = 0x7ff0000000000000ll, mask = 0x7fffffffffffffffll;
+    const int64_t kl = line_key(left), kr = line_key(right);
+    if ((kl & mask) > inf || (kr & mask) > inf) {
+        a = lower_bound(sl, L, left);
+        b = upper_bound(sl, L, right);
+        return;
+    }
+    uint32_t lo = 0, hi = L;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (line_key(sl[mid]) < kl) lo = mid + 1; else hi = mid;
+    }
+    a = lo;
+    hi = L;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (line_key(sl[mid]) <= kr) lo = mid + 1; else hi = mid;
+    }
+    b = lo;
+}
+
 // Lines that contribute at frequency `freq` of an element (eta_chi_fp64's range).
 template <int AP>
 MGR_HD void elem_bracket(const DevModel& m, const double* sl, double freq, uint32_t nr, uint32_t& lo, uint32_t& hi) {
@@ -152,8 +187,7 @@ MGR_HD void elem_bracket(const DevModel& m, const double* sl, double freq, uint3
     hi = m.L;
     if (AP == APPROX_CLOSELINES) {
         const double ub = dmul_rn(m.max_dist, dmul_rn(freq, m.ub[nr]));
-        lo = lower_bound(sl, m.L, dsub_rn(freq, ub));
-        hi = upper_bound(sl, m.L, dadd_rn(freq, ub));
+        lines_between(sl, m.L, dsub_rn(freq, ub), dadd_rn(freq, ub), lo, hi);
     }
 }
 
@@ -162,33 +196,36 @@ MGR_HD uint32_t line_of(const DevModel& m, uint32_t s) {
     return (AP == APPROX_CLOSELINES) ? m.sorted_map[s] : s;
 }
 
-// A sweep's element, once evaluated: emissivity, opacity and source, the lines that contribute,
-// and the profile of the last of them.
+// A sweep's element, once evaluated: opacity, its inverse and the source, the lines that
+// contribute, and the profile over the inverse width of the last of them.
 struct ElemVal {
-    double eta, chi, S, prof;
+    double chi, rchi, S, prof;
     uint32_t lo, hi;
     bool ok;
 };
 
-// Element emissivity and opacity (eta_chi_fp64, smooth).
-template <int AP>
+// Element emissivity and opacity (eta_chi_fp64, smooth), at the rounded product nu shift or the
+// exact one.
+template <int AP, bool EXACT = false>
 MGR_HD void elem_s(const DevModel& m, const double* sl, double nu, const Elem& e, ElemVal& v) {
     const double freq = dmul_rn(nu, e.shift);
     elem_bracket<AP>(m, sl, freq, e.nr, v.lo, v.hi);
     const size_t b1 = (size_t)e.nr * m.L, b2 = (size_t)e.ni * m.L;
-    v.eta = 0.0;
+    double eta = 0.0;
     v.chi = m.min_opacity;
     v.prof = 0.0;
 #pragma unroll 1
     for (uint32_t s = v.lo; s < v.hi; s++) {
         const uint32_t l = line_of<AP>(m, s);
-        const double diff = freq - m.line[l];
+        const double diff = EXACT ? fma(nu, e.shift, -m.line[l]) : freq - m.line[l];
         const double iw = interpolate_linear(m.iw[b1 + l], m.iw[b2 + l], e.fac);
         v.prof = gauss_s(iw, diff);
-        v.eta += v.prof * ilog_s(m.em[b1 + l], m.em[b2 + l], e.fac);
-        v.chi += v.prof * ilog_s(m.op[b1 + l], m.op[b2 + l], e.fac);
+        const double prof = iw * v.prof;
+        eta += prof * ilog_s(m.em[b1 + l], m.em[b2 + l], e.fac);
+        v.chi += prof * ilog_s(m.op[b1 + l], m.op[b2 + l], e.fac);
     }
-    v.S = v.eta / v.chi;
+    v.rchi = 1.0 / v.chi;
+    v.S = eta * v.rchi;
     v.ok = true;
 }
 
@@ -211,13 +248,13 @@ MGR_HD void elem_s_adj(const DevModel& m, double nu, const Elem& e, const ElemVa
         if (s >= lo && s < hi) {
             const double diff = freq - m.line[l];
             const double iw = interpolate_linear(m.iw[b1 + l], m.iw[b2 + l], f);
-            const double prof = (hi == lo + 1) ? v.prof : gauss_s(iw, diff);
+            const double prof_iw = (hi == lo + 1) ? v.prof : gauss_s(iw, diff), prof = iw * prof_iw;
             const double x = iw * diff;
             const double emE = ilog_s(m.em[b1 + l], m.em[b2 + l], f);
             const double opE = ilog_s(m.op[b1 + l], m.op[b2 + l], f);
             const double gprof = g_eta * emE + g_chi * opE;
             const double g_emE = g_eta * prof, g_opE = g_chi * prof;
-            const double g_iwE = gprof * prof * (1.0 / iw - 2.0 * x * diff);
+            const double g_iwE = gprof * (prof_iw - 2.0 * x * diff * prof);
             g_shift += gprof * prof * (-2.0 * x * iw) * nu;
             gem_nr = g_emE;
             gop_nr = g_opE;
@@ -251,8 +288,7 @@ MGR_HD void pair_bracket(const DevModel& m, const double* sl, double cf, double 
         const double cb = dmul_rn(m.max_dist, dmul_rn(right, m.ub[lo_nr]));
         const double nb = dmul_rn(m.max_dist, dmul_rn(right, m.ub[hi_nr]));
         const double ubw = cb > nb ? cb : nb;
-        a = lower_bound(sl, m.L, dsub_rn(left, ubw));
-        b = upper_bound(sl, m.L, dadd_rn(right, ubw));
+        lines_between(sl, m.L, dsub_rn(left, ubw), dadd_rn(right, ubw), a, b);
     }
 }
 
@@ -268,7 +304,7 @@ MGR_HD double ld_s(const DevModel& m, const Elem& lo, const Elem& hi, uint32_t l
     const double avg_iw = (iwc + iwn) / 2.0;
     const double cop = ilog_s(m.op[c1 + l], m.op[c2 + l], lo.fac);
     const double nop = ilog_s(m.op[n1 + l], m.op[n2 + l], hi.fac);
-    if (cf == nf) return dz * (gauss_s(avg_iw, cf - linefreq) * ((cop + nop) / 2.0) + m.min_opacity);
+    if (cf == nf) return dz * (avg_iw * gauss_s(avg_iw, cf - linefreq) * ((cop + nop) / 2.0) + m.min_opacity);
     const double next_pos = (linefreq - nf) * avg_iw;
     const double curr_pos = (linefreq - cf) * avg_iw;
     const double diff_pos = next_pos - curr_pos;
@@ -295,7 +331,7 @@ MGR_HD LdAdj ld_s_adj(const DevModel& m, const Elem& lo, const Elem& hi, uint32_
     LdAdj r{0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     if (cf == nf) {
         const double diff = cf - linefreq;
-        const double prof = gauss_s(avg, diff);
+        const double prof = avg * gauss_s(avg, diff);
         const double x = avg * diff;
         const double gprof = gld * dz * ((cop + nop) / 2.0);
         r.g_cop = r.g_nop = gld * dz * prof / 2.0;
@@ -331,10 +367,12 @@ MGR_HD LdAdj ld_s_adj(const DevModel& m, const Elem& lo, const Elem& hi, uint32_
 struct PairS {
     bool large;
     double dtau, Slo, Shi;
-    double chi_o, chi_i;  // trapezoid branch
-    double sum_dtau;      // large branch, before the clamp
-    double E;             // large branch with one line in reach: its erf difference
-    uint32_t a, b;        // large branch: the lines in reach
+    double rchi_o, rchi_i;  // trapezoid branch
+    double sum_dtau;        // large branch, before the clamp
+    double E;               // large branch with one line in reach: its erf difference
+    uint32_t a, b;          // large branch: the lines in reach
+    bool unit;              // ld1 is set
+    LdAdj ld1;              // derivatives of the one line's optical depth
 };
 
 template <int AP>
@@ -346,29 +384,31 @@ MGR_HD bool pair_large(const DevModel& m, const Elem& outer, const Elem& inner) 
 
 // oc / ic: the outer / inner element's values if already known (evaluated and stored
 // otherwise, trapezoid branch).  E, dt: in the reverse sweep, the pair's erf difference (of one
-// line in reach) and its optical depth as the forward pass left them.
-template <int AP>
+// line in reach) and its optical depth as the forward pass left them.  EXACT (the imager's reverse
+// sweep, whose rows and elements take the exact products nu shift where its forward sweep rounds
+// them): elements at the exact products, a stored depth moved there to first order.
+template <int AP, bool EXACT = false>
 MGR_HD PairS pair_s(const DevModel& m, const double* sl, double nu, const Elem& outer, const Elem& inner, double dz,
                     ElemVal& oc, ElemVal& ic, const double* E = nullptr, const double* dt = nullptr) {
     PairS r{};
     r.large = pair_large<AP>(m, outer, inner);
     if (!r.large) {
-        for (int k = 0; k < 2; k++) {  // one site of elem_s
-            ElemVal& v = k ? ic : oc;
-            if (v.ok) continue;
-            elem_s<AP>(m, sl, nu, k ? inner : outer, v);
+#pragma unroll 1
+        for (int k = 0; k < 2; k++) {  // one site of elem_s; copies, as references would be to memory
+            ElemVal v = k ? ic : oc;
+            if (!v.ok) elem_s<AP, EXACT>(m, sl, nu, k ? inner : outer, v);
+            if (k) ic = v;
+            else oc = v;
         }
-        r.chi_o = oc.chi;
-        r.chi_i = ic.chi;
+        r.rchi_o = oc.rchi;
+        r.rchi_i = ic.rchi;
         r.Slo = oc.S;
         r.Shi = ic.S;
-        r.dtau = 0.5 * (r.chi_o + r.chi_i) * dz;
+        r.dtau = 0.5 * (oc.chi + ic.chi) * dz;
         return r;
     }
-    // Rounded products, here and in elem_s: fused into (nu shift - line) in the forward pass or in
-    // the adjoint alone, a position moves by 1e-10 of a width, and an adjoint whose state and
-    // recomputed pairs differ by that is off by 2e-10 to 6e-10 in every gradient (it was, against
-    // the restatement on the CPU; 1e-14 now).
+    // Rounded products: fused into (line - nu shift) at one site and not at another, a position
+    // would move by 1e-10 of a width against the stored erf difference.
     const double cf = dmul_rn(nu, outer.shift), nf = dmul_rn(nu, inner.shift);
     uint32_t a, b;
     pair_bracket<AP>(m, sl, cf, nf, outer.nr, inner.nr, a, b);
@@ -383,7 +423,13 @@ MGR_HD PairS pair_s(const DevModel& m, const double* sl, double nu, const Elem& 
     // nothing): the depth is the line's own, the sources are its own
     if (dt && one && (AP == APPROX_NONE || *dt != bound_min_dtau || *E == 0.0)) {
         const uint32_t l = line_of<AP>(m, a);
-        r.dtau = r.sum_dtau = *dt;
+        r.dtau = *dt;
+        if (EXACT) {
+            r.ld1 = ld_s_adj(m, outer, inner, l, cf, nf, dz, 1.0, *E);
+            r.unit = true;
+            r.dtau += r.ld1.g_cf * fma(nu, outer.shift, -cf) + r.ld1.g_nf * fma(nu, inner.shift, -nf);
+        }
+        r.sum_dtau = r.dtau;
         r.Slo = ilog_s(m.Sp[c1 + l], m.Sp[c2 + l], outer.fac);
         r.Shi = ilog_s(m.Sp[n1 + l], m.Sp[n2 + l], inner.fac);
         return r;
@@ -451,7 +497,15 @@ MGR_HD void pair_large_adj(const DevModel& m, double nu, const Elem& outer, cons
                 glsc = gsc * ld;
                 glsn = gsn * ld;
             }
-            const LdAdj r = ld_s_adj(m, outer, inner, l, cf, nf, dz, gld, E);
+            LdAdj r = f.ld1;
+            if (f.unit) {
+                r.g_iwc = r.g_iwn = gld * r.g_iwc;
+                r.g_cop = r.g_nop = gld * r.g_cop;
+                r.g_cf *= gld;
+                r.g_nf *= gld;
+            } else {
+                r = ld_s_adj(m, outer, inner, l, cf, nf, dz, gld, E);
+            }
             g_sh_o += r.g_cf * nu;
             g_sh_i += r.g_nf * nu;
             gop[0] = r.g_cop;
@@ -480,7 +534,7 @@ MGR_HD void pair_large_adj(const DevModel& m, double nu, const Elem& outer, cons
             }
         }
         // the elements' first points, then the second points of subdivided steps
-#pragma unroll 1
+#pragma unroll
         for (int j = 0; j < 2; j++) {
             if (j == 1 && fo == 0.0 && fi == 0.0) continue;
             const bool to_o = j == 0 || fo != 0.0, to_i = j == 0 || fi != 0.0;
@@ -498,6 +552,17 @@ MGR_HD void pair_large_adj(const DevModel& m, double nu, const Elem& outer, cons
 MGR_HD void elem_shift_adj(const Elem& e, double g_shift, const AdjAcc& acc) {
     acc.add_shift(e.nr, g_shift * (1.0 - e.fac));
     if (e.fac != 0.0) acc.add_shift(e.ni, g_shift * e.fac);
+}
+
+// 1 / a and 1 / dt (a pair's optical depth, possibly 0) by one division.
+MGR_HD void reciprocals(double a, double dt, double& ra, double& rdt) {
+    const double r = 1.0 / (a * dt);
+    ra = dt * r;
+    rdt = a * r;
+    if ((uint64_t)line_key(dt) << 1 == 0) {  // +-0, off the FP64 pipe
+        ra = 1.0 / a;
+        rdt = 1.0 / dt;
+    }
 }
 
 // Scratch of one lane: elimination state after pair k, (F, Su, dtau, erf difference) at
@@ -526,7 +591,7 @@ MGR_HD double image_lane_s(const DevModel& m, const double* sl, uint32_t o, doub
     iter_begin<MODE_FP64>(m, bk, o, kAllLines, nb, it);
     iter_next<MODE_FP64>(m, bk, o, kAllLines, it, prev);
     const double Ib = bdy_s(m, prev.nr, nu * prev.shift, dummy);
-    double F = 0.0, FI = 0.0, Su = 0.0, dt_prev = 0.0, S_last = 0.0;  // FI = 1 / (1 + F)
+    double F = 0.0, FI = 0.0, Su = 0.0, dt_prev = 0.0, rdt = 0.0, S_last = 0.0;  // FI = 1 / (1 + F), rdt = 1 / dt_prev
     ElemVal v_prev{};
     uint32_t k = 0;
     bool done = false;
@@ -545,14 +610,14 @@ MGR_HD double image_lane_s(const DevModel& m, const double* sl, uint32_t o, doub
             // multiplied through by dt^2/2 (no 1/dt: well conditioned for thin pairs)
             const double h = dt * (0.5 * dt + 1.0);
             F = h;
-            FI = 1.0 / (1.0 + F);
+            reciprocals(1.0 + F, dt, FI, rdt);
             Su = (ps.Slo * (0.5 * dt * dt) + Ib * dt) * FI;
         } else {
             // elimination row with q = A iC = dt / dt_prev
-            const double q = dt / dt_prev;
+            const double q = dt * rdt;
             const double iC = 0.5 * (dt_prev + dt) * dt;
             F = q * (F * FI) + iC;
-            FI = 1.0 / (1.0 + F);
+            reciprocals(1.0 + F, dt, FI, rdt);
             Su = (q * Su + ps.Slo * iC) * FI;
         }
         if (scr) {
@@ -620,8 +685,9 @@ MGR_HD bool image_lane_adj(const DevModel& m, const double* sl, uint32_t o, doub
         const double dz = outer.dzin;
         const double E = scr.at(kk, 3);
         ElemVal v_outer{};
-        const double dt = scr.at(kk, 2);
-        const PairS ps = pair_s<AP>(m, sl, nu, outer, inner, dz, v_outer, v_inner, &E, &dt);
+        const double dts = scr.at(kk, 2);
+        const PairS ps = pair_s<AP, true>(m, sl, nu, outer, inner, dz, v_outer, v_inner, &E, &dts);
+        const double dt = ps.dtau;
         double gSlo = 0.0, gShi = 0.0;
         if (kk == M - 1) {
             const double N = Su_last + ps.Shi * (0.5 * dtl * dtl) + Ibl * dtl;
@@ -641,9 +707,10 @@ MGR_HD bool image_lane_adj(const DevModel& m, const double* sl, uint32_t o, doub
             // pair kk: F_k = q G' + iC, Su_k = Z / (1 + F_k), G' = F'/(1 + F'),
             // Z = q Su' + S iC, q = dt / dto, iC = (dto + dt) dt / 2
             const double Fp = scr.at(kk - 1, 0), Sup = scr.at(kk - 1, 1), dto = scr.at(kk - 1, 2);
-                        const double q = dt / dto;
+            double FIp, rdto;  // FIp: the next pair's FIk
+            reciprocals(1.0 + Fp, dto, FIp, rdto);
+            const double q = dt * rdto;
             const double iC = 0.5 * (dto + dt) * dt;
-            const double FIp = 1.0 / (1.0 + Fp);  // the next pair's FIk
             const double G = Fp * FIp;
             const double Z = q * Sup + ps.Slo * iC;
             const double gZ = gSu * FIk;
@@ -651,7 +718,7 @@ MGR_HD bool image_lane_adj(const DevModel& m, const double* sl, uint32_t o, doub
             const double gq = gFt * G + gZ * Sup;
             const double giC = gFt + gZ * ps.Slo;
             gSlo = gZ * iC;
-            const double gqd = gq / dto;
+            const double gqd = gq * rdto;
             g_dt_k = gdt + gqd + giC * (0.5 * dto + dt);
             // hand the state adjoint to pair kk - 1
             gF = gFt * q * FIp * FIp;
@@ -679,7 +746,7 @@ MGR_HD bool image_lane_adj(const DevModel& m, const double* sl, uint32_t o, doub
             carry_eta = carry_chi = 0.0;
             have_carry = false;
         } else {
-            const double ti = gShi / ps.chi_i, to = gSlo / ps.chi_o, half = 0.5 * dz * g_dt_k;
+            const double ti = gShi * ps.rchi_i, to = gSlo * ps.rchi_o, half = 0.5 * dz * g_dt_k;
             elem_s_adj<AP>(m, nu, inner, v_inner, carry_eta + ti, carry_chi + half - ti * ps.Shi, acc, g_sh_i);
             carry_eta = to;
             carry_chi = half - to * ps.Slo;

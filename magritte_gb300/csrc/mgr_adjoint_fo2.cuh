@@ -62,7 +62,7 @@ MGR_HD HalfS half_s(const DevModel& m, const double* sl, uint32_t o, double nu, 
     iter_next<MODE_FP64>(m, h, o, l, it, prev);
     double dummy;
     const double Ib = bdy_s(m, prev.nr, nu * prev.shift, dummy);
-    double F = 0.0, FI = 0.0, Su = 0.0, dt_prev = 0.0, S_carry = 0.0;  // FI = 1 / (1 + F)
+    double F = 0.0, FI = 0.0, Su = 0.0, dt_prev = 0.0, rdt = 0.0, S_carry = 0.0;  // FI = 1 / (1 + F), rdt = 1 / dt_prev
     ElemVal v_prev{};
     uint32_t k = 0;
     bool done = false;
@@ -80,13 +80,13 @@ MGR_HD HalfS half_s(const DevModel& m, const double* sl, uint32_t o, double nu, 
         if (k == 0) {
             const double h0 = dt * (0.5 * dt + 1.0);
             F = h0;
-            FI = 1.0 / (1.0 + F);
+            reciprocals(1.0 + F, dt, FI, rdt);
             Su = (S_row * (0.5 * dt * dt) + Ib * dt) * FI;
         } else {
-            const double q = dt / dt_prev;
+            const double q = dt * rdt;
             const double iC = 0.5 * (dt_prev + dt) * dt;
             F = q * (F * FI) + iC;
-            FI = 1.0 / (1.0 + F);
+            reciprocals(1.0 + F, dt, FI, rdt);
             Su = (q * Su + S_row * iC) * FI;
         }
         if (scr) {
@@ -215,9 +215,10 @@ MGR_HD void half_s_adj(const DevModel& m, const double* sl, uint32_t o, double n
         double g_dt_k, gSrow, g_sh_o = 0.0;
         if (kk > 0) {
             const double Fp = scr.at(k0 + kk - 1, 0), Sup = scr.at(k0 + kk - 1, 1), dto = scr.at(k0 + kk - 1, 2);
-            const double q = dt / dto;
+            double FIp, rdto;  // FIp: the next pair's FIk
+            reciprocals(1.0 + Fp, dto, FIp, rdto);
+            const double q = dt * rdto;
             const double iC = 0.5 * (dto + dt) * dt;
-            const double FIp = 1.0 / (1.0 + Fp);  // the next pair's FIk
             const double G = Fp * FIp;
             const double Z = q * Sup + S_row * iC;
             const double gZ = gSu * FIk;
@@ -225,7 +226,7 @@ MGR_HD void half_s_adj(const DevModel& m, const double* sl, uint32_t o, double n
             const double gq = gFt * G + gZ * Sup;
             const double giC = gFt + gZ * S_row;
             gSrow = gZ * iC;
-            const double gqd = gq / dto;
+            const double gqd = gq * rdto;
             g_dt_k = gdt + gqd + giC * (0.5 * dto + dt);
             gF = gFt * q * FIp * FIp;
             gSu = gZ * q;
@@ -252,7 +253,7 @@ MGR_HD void half_s_adj(const DevModel& m, const double* sl, uint32_t o, double n
             carry_eta = carry_chi = 0.0;
             have_carry = false;
         } else {
-            const double ti = gShi / ps.chi_i, to = gSlo / ps.chi_o, half = 0.5 * dz * g_dt_k;
+            const double ti = gShi * ps.rchi_i, to = gSlo * ps.rchi_o, half = 0.5 * dz * g_dt_k;
             elem_s_adj<AP>(m, nu, inner, v_inner, carry_eta + ti, carry_chi + half - ti * ps.Shi, acc, g_sh_i);
             carry_eta = to;
             carry_chi = half - to * ps.Slo;
