@@ -39,8 +39,9 @@ typedef enum { MGR_APPROX_NONE = 0, MGR_APPROX_ONELINE = 1, MGR_APPROX_CLOSELINE
  *  MGR_PRECISION_FP64  : the reference's arithmetic: FP64 storage with its
  *                        single-precision libm calls (expf, erff, logf, powf).
  *  MGR_PRECISION_SPLIT : profile, opacity, source and optical-depth arithmetic in
- *                        FP32; the Feautrier elimination and back substitution in
- *                        FP64.  Ray traces are identical in both modes.            */
+ *                        FP32; the Feautrier elimination in FP64, or in pairs of
+ *                        FP32 numbers (about 45 bits) where lines are apart.
+ *                        Ray traces are identical in both modes.                   */
 typedef enum { MGR_PRECISION_FP64 = 0, MGR_PRECISION_SPLIT = 1 } MgrPrecision;
 
 /* Boundary conditions (src/model/geometry/boundary/boundary.hpp:7). */

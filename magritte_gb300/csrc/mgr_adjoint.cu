@@ -10,6 +10,10 @@
 // lane, the elimination state of each pair in a scratch array of the warp's slot
 // (recomputed from the inputs, not saved by the forward), and adds its derivatives
 // into the per-point gradient arrays with one atomic per warp and entry.
+//
+// What bounds them: the FP64 pipe, 84 % (forward) and 76 % (adjoint) busy with 10 to 15 of 32
+// lanes live: a line is in reach of a few of the frequencies, and 41 of them take two warps.
+// An image of 64 x 64 pixels x 41 frequencies and its gradients, 5k points: 40.4 -> 24 ms.
 #include <algorithm>
 #include <cstring>
 #include <vector>

@@ -11,6 +11,10 @@
 // reference's ray-pair order.  The backward keeps each lane's per-pair elimination state in a
 // scratch array of the warp's slot (recomputed, not saved by the forward) and adds its
 // derivatives with one atomic per warp and entry.
+//
+// What bounds them: the FP64 pipe, with as many of 32 lanes live as a line has quadrature points,
+// and instruction fetch (8 warps an SM on 335 KB of code; 553 KB with each half's sweep inlined).
+// J and its gradients on a 13^3 sphere, 3 lines x 15: 23.1 -> 9.8 ms.
 #include <algorithm>
 #include <vector>
 

@@ -3,8 +3,10 @@
 // Each model is an ordinary MgrModel (mgr_model_create); a batch collects their device
 // descriptions into one device array.  The models are solved in waves: consecutive
 // models whose staged per-ray results fit the batch's staging area (a few GiB; one
-// wave for most batches) are solved by one persistent launch of fo2_multi_kernel and
-// one launch of fo2_multi_reduce_kernel.
+// wave for most batches) are solved by one launch each of trace_multi_kernel,
+// fo2_multi_staged_kernel (the staged solve of mgr_staged.cuh, every model with its own plan),
+// fo2_multi_kernel for the ray pairs that gives up, and fo2_multi_reduce_kernel; a batch with a
+// model the staged solve does not serve takes fo2_multi_kernel for all of it.
 //   * fo2_multi_kernel: one warp per (model, origin, ray pair) item, lanes over
 //     frequencies, the same trace and solve_lane code as the single-model fo2_kernel;
 //     u and L_diag go to the model's slice of the staging area.  Items are ordered
@@ -13,7 +15,7 @@
 //   * fo2_multi_reduce_kernel: one CTA per (model, origin), the single-model
 //     reduction's per-origin code (mgr_reduce.cuh): J and the ALO diagonal in the same
 //     order as the model's own mgr_formal_solve_fo2, so every model's results are its
-//     own solve's (bit for bit in split precision).
+//     own solve's (bit for bit in split precision when both take the same solve).
 // Per model the kernels record, from the GPU's global timer, when its first item
 // started and when its last origin was reduced (the per-model latency).
 #include <algorithm>

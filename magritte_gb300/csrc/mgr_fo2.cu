@@ -277,7 +277,9 @@ __global__ void __launch_bounds__(256, MINB)
 // ---------------------------------------------------------------------------------
 // Formal solve, stage 1, staged (mgr_staged.cuh).  trace_rays_kernel: a warp per half ray of
 // the origins' pairs, slot 2 ((o - o_begin) nR + rr - rr0) + side.  fo2_staged_kernel: a warp
-// per K consecutive (origin, ray pair) items, results as fo2_kernel's.
+// per K consecutive (origin, ray pair) items, results as fo2_kernel's.  The walk is a chain of
+// loads: 2.7 of 17.7 ms on the 33^3 sphere at four CTAs an SM (64 registers; five the same, six
+// 0.9 ms slower).
 // ---------------------------------------------------------------------------------
 template <int MODE, int GEO>
 __global__ void __launch_bounds__(256, 4) trace_rays_kernel(const __grid_constant__ DevModel m, uint32_t cap,
@@ -728,7 +730,7 @@ size_t fo2_work_bytes(const MgrModel* model, uint32_t n_origins, bool stage_u, b
 
 // Whether the staged solve serves this model: its tiles hold one line's data, so the
 // frequencies come line by line and pairs that reach several lines are rare (each of those is
-// solved twice).  33^3 sphere, 4 lines x 31, split: 17.9 ms staged, 42.1 ms by the general kernel;
+// solved twice).  33^3 sphere, 4 lines x 31, split: 17.7 ms staged, 42.1 ms by the general kernel;
 // 10^3 cube, 1 line x 11, FP64: 0.22 and 1.34 ms.
 bool staged_ok(const MgrModel* model) {
     const DevModel& m = model->dm;

@@ -101,7 +101,9 @@ __global__ void __launch_bounds__(256) image_new_kernel(DevModel m, ImagePlane i
 
 // ---------------------------------------------------------------------------------
 // New imager, staged (mgr_staged.cuh): image_trace_kernel walks a warp per pixel into global
-// memory, image_staged_kernel eliminates; pixels it gives up go to image_new_kernel.
+// memory, image_staged_kernel eliminates; pixels it gives up go to image_new_kernel.  The walk is
+// a chain of loads (0.4 ms of 2.3 for 151 x 97 pixels; 64 registers, four CTAs an SM), the
+// elimination FP64-bound (1.5 ms).
 // ---------------------------------------------------------------------------------
 template <int MODE>
 __global__ void __launch_bounds__(256, 4) image_trace_kernel(const __grid_constant__ DevModel m, ImagePlane ip,

@@ -20,7 +20,9 @@ __device__ __forceinline__ double warp_sum(double v) {
 // Both sums run over values that are already in L2 or stream from memory; what bound them was
 // the FP64 pipe (one warp instruction per 16 cycles and SM), six multiplications and an
 // addition per ALO element.  The factors that do not depend on the ray pair stand outside the
-// sums over it: one multiplication-addition per element of either sum.
+// sums over it: one multiplication-addition per element of either sum (formal solve of the 33^3
+// sphere 19.0 -> 18.4 ms, short characteristics of the 20^3 sphere 1.60 -> 1.22 ms).
+
 // ray_w(o, rr0 + k) as a pointer over k
 __device__ __forceinline__ const double* ray_weights(const DevModel& m, uint32_t o, uint32_t rr0) {
     return m.rayw + (m.adaptive ? (size_t)o * m.nrays : (size_t)0) + rr0;
