@@ -35,9 +35,9 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "point.ray.freq solves/s"
-# DRAM bytes per solve of the split formal-solve kernel, ncu on the 32^3 sphere cutout:
-# (1004.8 MB read + 1575.3 MB written) / 45.9 M solves
-TRAFFIC_BYTES_PER_SOLVE = (1004.780e6 + 1575.276e6) / 45_854_208.0
+# DRAM bytes per solve of the split staged solve kernel, ncu on the 33^3 sphere cutout:
+# 4715.4 MB read + written / 50.8 M solves
+TRAFFIC_BYTES_PER_SOLVE = 4715.425e6 / 50_821_152.0
 UNIT = "solves/s"
 
 
@@ -933,10 +933,11 @@ def run_ours(args, rank, ws):
                    "ray_pairs_rank0": [rr0, rr1]},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": TRAFFIC_BYTES_PER_SOLVE * solves * (rr1 - rr0) / R,
-                     "traffic_note": "DRAM read + write bytes per launch from an ncu capture of the 32^3 case "
-                                     "(1004.8 MB read + 1575.3 MB written for 45.9 M solves; ncu flushes the caches "
-                                     "between its passes), scaled by the solves of this launch; the writes are the "
-                                     "u / L_diag staging, proportional to solves",
+                     "traffic_note": "DRAM read + write bytes per launch from an ncu capture of the staged solve kernel "
+                                     "on the 33^3 case (4715.4 MB for 50.8 M solves; ncu flushes the caches between "
+                                     "its passes; the kernel that walks the half rays is not in it), scaled by the "
+                                     "solves of this launch: the half rays read and the u / L_diag staging written "
+                                     "are proportional to solves",
                      "peak_source": peak_src,
                      "algorithmic_bytes_per_launch": alg_bytes,
                      "note": "algorithmic bytes = 28 per trace step and per neighbour record + 52 per ray-pair "

@@ -158,7 +158,7 @@ cudaError_t launch_size_rays(MgrModel* model, uint32_t* d_max_steps);
 // origins, u [hnrays][P][F] (may be NULL).  Per-ray results are staged in `work`
 // (sized by fo2_work_bytes for the same u / lam choice) behind the chunk's traced half rays, in
 // chunks of origins that fit.  6.5 GiB: the 64^3 benchmark model (6.2 GB of u and L_diag, 17 GB
-// of half rays) in four chunks.
+// of half rays) in three chunks.
 constexpr size_t kFo2WorkBudget = size_t(13) << 29;
 size_t fo2_work_bytes(const MgrModel* model, uint32_t n_origins, bool stage_u, bool stage_ld);
 // Ray pairs [rr_begin, rr_end) only (partial J / ALO sums, u must then be NULL).
