@@ -4,6 +4,8 @@ its frequencies in reverse order takes the general kernel.
 Bar: 1e-9 of each element of u.  The two take the same single-precision physics, and their rows
 differ by their roundings, 2^-45 and 2^-46 a row over some hundred rows, with room for rows that
 amplify a hundredfold; one single-precision rounding that differs is 6e-8."""
+from dataclasses import replace
+
 import numpy as np
 import pytest
 
@@ -39,3 +41,13 @@ def test_edge_of_a_lines_reach(gpu_lib, reach, seed):
     edge of its reach shows in u, and with 1e8 pairs some ten lie at the edge's rounding."""
     raw = S.batch_model(npoints=4000, nside=2, nlev=5, nquads=31, seed=seed)
     assert_same_u(H.setup(raw, max_distance_opacity_contribution=reach))
+
+
+def test_boundary_intensities_fp64(gpu_lib):
+    """A transparent model at rest: u is the mean of the boundary intensities the two halves start
+    from.  At most three rows a half, each with four roundings of 2^-53 in either kernel, and the
+    combination's: below 6e-15.  Intensities formed in double-float are off by up to 3e-14 (mean
+    3e-15), and by 6e-8 where their exponent rounds to another float."""
+    raw = S.batch_model(npoints=65, nside=2, nlev=5, nquads=31)
+    raw = replace(raw, abundance=raw.abundance * np.array([1.0e-20, 1.0]), velocity=np.zeros_like(raw.velocity))
+    assert_same_u(H.setup(raw), 6e-15, ("fp64",))
