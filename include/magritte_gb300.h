@@ -441,6 +441,12 @@ void* mgr_batch_stream(MgrBatch* batch);
  * (the n_tot of solver.tpp:492-496 per line).  Used for algorithmic-byte counts. */
 int mgr_ray_statistics(MgrModel* model, uint64_t* steps, uint64_t* neighbor_reads, uint64_t* elements);
 
+/* Ray pairs and image pixels that the staged solve took in this model's solves, images and
+ * batches since the last call of this function, and how many of them it left to the
+ * general kernel (which then solves them again).  0 taken: the general kernel solved all.
+ * Blocks until the model's stream is done. */
+int mgr_staged_statistics(MgrModel* model, uint64_t* taken, uint64_t* given_up);
+
 /* Self-check of the ray trace (no reference counterpart; the reference's trace is
  * Geometry::get_next_general_geometry, src/model/geometry/geometry.tpp:13-44).  The
  * kernels pick each next point with an FP32 filter whose error bounds decide the

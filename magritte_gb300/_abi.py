@@ -116,6 +116,7 @@ SIGNATURES = {
                                       _f64p, _f64p, C.c_uint32]),
     "mgr_set_column": (C.c_int, [C.c_void_p, _f64p, _f64p]),
     "mgr_formal_solve_fo2_device_noalloc": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]),
+    "mgr_staged_statistics": (C.c_int, [C.c_void_p, C.POINTER(C.c_uint64), C.POINTER(C.c_uint64)]),
     "mgr_ray_statistics": (C.c_int, [C.c_void_p, C.POINTER(C.c_uint64), C.POINTER(C.c_uint64),
                                      C.POINTER(C.c_uint64)]),
     "mgr_trace_self_check": (C.c_int, [C.c_void_p, C.POINTER(C.c_uint64), C.POINTER(C.c_uint64),
@@ -399,6 +400,12 @@ class DeviceModel:
         a, b, c = C.c_uint64(), C.c_uint64(), C.c_uint64()
         _check(load().mgr_ray_statistics(self.h, C.byref(a), C.byref(b), C.byref(c)))
         return dict(steps=a.value, neighbor_reads=b.value, elements=c.value)
+
+    def staged_statistics(self):
+        """(ray pairs and pixels the staged solve took, those it left to the general kernel) since the last call."""
+        a, b = C.c_uint64(), C.c_uint64()
+        _check(load().mgr_staged_statistics(self.h, C.byref(a), C.byref(b)))
+        return a.value, b.value
 
     def sync(self):
         _check(load().mgr_sync(self.h))

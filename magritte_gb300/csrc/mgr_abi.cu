@@ -488,6 +488,8 @@ int mgr_model_create(const MgrModelDesc* d, MgrModel** out) {
         if ((e = upload(m, &dm.quad_w, d->quad_weights, (size_t)d->nlspecs * d->nquads)) != cudaSuccess) break;
         if ((e = dalloc(m, &m->status, 1)) != cudaSuccess) break;
         if ((e = cudaMemsetAsync(m->status, 0, sizeof(int), m->stream)) != cudaSuccess) break;
+        if ((e = dalloc(m, &dm.staged_counts, 2)) != cudaSuccess) break;
+        if ((e = cudaMemsetAsync(dm.staged_counts, 0, 2 * sizeof(unsigned long long), m->stream)) != cudaSuccess) break;
     } while (false);
     if (e != cudaSuccess) {
         int rc = cuda_fail(e, "model upload");
@@ -991,6 +993,22 @@ int mgr_ray_statistics(MgrModel* model, uint64_t* steps, uint64_t* neighbor_read
     *steps = h[0];
     *neighbor_reads = h[1];
     *elements = h[2];
+    return MGR_OK;
+}
+
+int mgr_staged_statistics(MgrModel* model, uint64_t* taken, uint64_t* given_up) {
+    MGR_MODEL_DEVICE(model);
+    if (!model || !taken || !given_up) {
+        set_error("mgr_staged_statistics: null argument");
+        return MGR_ERR_ARGUMENT;
+    }
+    unsigned long long h[2] = {0, 0};
+    cudaError_t e = cudaMemcpyAsync(h, model->dm.staged_counts, sizeof(h), cudaMemcpyDeviceToHost, model->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(model->dm.staged_counts, 0, sizeof(h), model->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(model->stream);
+    if (e != cudaSuccess) return cuda_fail(e, "staged solve statistics");
+    *taken = h[0];
+    *given_up = h[1];
     return MGR_OK;
 }
 

@@ -143,11 +143,17 @@ __global__ void __launch_bounds__(256, MINB)
     // list: only the items listed (list[0] of them, from list[1] on, counted from i0)
     const uint64_t n = list ? (uint64_t)list[0] : item_off[m1] - i0;
     const uint64_t s0 = stage_off[m0];
+    if (list && blockIdx.x == 0)
+        for (uint32_t i = m0 + threadIdx.x; i < m1; i += blockDim.x)
+            atomicAdd(models[i].staged_counts, (unsigned long long)(item_off[i + 1] - item_off[i]));
     const uint64_t stride = (uint64_t)gridDim.x * nw;
     uint32_t mi = m0, desc_mi = 0xffffffffu;
     for (uint64_t q = (uint64_t)blockIdx.x * nw + w; q < n; q += stride) {
         const uint64_t item = i0 + (list ? (uint64_t)list[1 + q] : q);
-        if (list) mi = model_of(item_off, m0, m1, item);
+        if (list) {
+            mi = model_of(item_off, m0, m1, item);
+            if (lane == 0) atomicAdd(models[mi].staged_counts + 1, 1ull);
+        }
         // the item's model: items only grow within a warp
         while (item_off[mi + 1] <= item) mi++;
         if (mi != desc_mi) {

@@ -117,6 +117,9 @@ struct DevModel {
     // erf about the nodes x0 = i / 2048 up to 3.92 (kErfNodes, one table per device): erf(x0)
     // and erf'(x0), each as two floats
     const float4* erf_node;
+    // ray pairs and pixels that the staged solve took, and those of them that it left to the
+    // general kernel (mgr_staged_statistics)
+    unsigned long long* staged_counts;  // [2]
     const float2* line_nb;       // [L] offsets of the neighbouring lines (sorted by frequency), -+inf at the ends
     const float* dls;            // [L][L] (float)(sorted_line[s] - line[l0]) at l0*L + s
     const float* dll;            // [L][L] (float)(line[l] - line[l0]) at l0*L + l

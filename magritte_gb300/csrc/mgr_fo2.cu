@@ -248,6 +248,10 @@ __global__ void __launch_bounds__(256, MINB)
 
     // list: only the items listed (list[0] of them, from list[1] on)
     const uint64_t n_items = list ? (uint64_t)list[0] : (uint64_t)(o_end - o_begin) * nR;
+    if (list && blockIdx.x == 0 && threadIdx.x == 0) {
+        atomicAdd(m.staged_counts, (unsigned long long)(o_end - o_begin) * nR);
+        atomicAdd(m.staged_counts + 1, (unsigned long long)n_items);
+    }
     const uint64_t stride = (uint64_t)gridDim.x * nw;
     for (uint64_t k = (uint64_t)blockIdx.x * nw + w; k < n_items; k += stride) {
         const uint64_t item = list ? (uint64_t)list[1 + k] : k;

@@ -74,6 +74,10 @@ __global__ void __launch_bounds__(256) image_new_kernel(DevModel m, ImagePlane i
     __syncthreads();
     // list: only the pixels listed (list[0] of them, from list[1] on)
     const uint32_t npix = list ? list[0] : ip.nx * ip.ny;
+    if (list && blockIdx.x == 0 && threadIdx.x == 0) {
+        atomicAdd(m.staged_counts, (unsigned long long)ip.nx * ip.ny);
+        atomicAdd(m.staged_counts + 1, (unsigned long long)npix);
+    }
     for (uint32_t k = blockIdx.x * nw + w; k < npix; k += gridDim.x * nw) {
         const uint32_t px = list ? list[1 + k] : k;
         double org[3];

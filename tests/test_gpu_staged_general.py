@@ -4,6 +4,7 @@ its frequencies in reverse order takes the general kernel.
 Bar: 1e-9 of each element of u.  The two take the same single-precision physics, and their rows
 differ by their roundings, 2^-45 and 2^-46 a row over some hundred rows, with room for rows that
 amplify a hundredfold; one single-precision rounding that differs is 6e-8."""
+import ctypes as C
 from dataclasses import replace
 
 import numpy as np
@@ -23,12 +24,41 @@ def in_reverse(a):
     return b
 
 
+def with_velocity(a, velocity):
+    """The model of arrays `a` given other velocities after its creation."""
+    torch = pytest.importorskip("torch")
+    dev = _abi.DeviceModel(a)
+    v = torch.tensor(np.ascontiguousarray(velocity), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    _abi._check(_abi.load().mgr_model_set_velocity_device(dev.h, C.c_void_p(v.data_ptr())))
+    dev.sync()
+    return dev
+
+
+def close_lines(nside=1, nquads=11, seed=0, npoints=1200):
+    """Arrays of a model whose two lines lie 30 km/s apart, at rest nearly (0.3 km/s) and with 50
+    times the velocities: at rest no pair reaches both lines, with the velocities many do, and a
+    model created with them is the general kernel's."""
+    raw = S.batch_model(npoints=npoints, nside=nside, nlev=3, nquads=nquads, seed=seed, sigma_v=0.3e3)
+    ld = raw.linedata[0]
+    f = np.array(ld.frequency, np.float64)
+    f[1] = f[0] * (1.0 + 1.0e-4)
+    raw = replace(raw, linedata=[replace(ld, frequency_given=f)])
+    return H.setup(raw), H.setup(replace(raw, velocity=50.0 * raw.velocity))
+
+
+def taken(dev):
+    return dev.staged_statistics()[0]
+
+
 def assert_same_u(a, bar=1e-9, precisions=("split",)):
     dev, general = _abi.DeviceModel(a), _abi.DeviceModel(in_reverse(a))
     try:
         for precision in precisions:
             u = dev.formal_solve_fo2(precision, want_u=True)["u"]
+            assert taken(dev) == dev.P * dev.R
             g = general.formal_solve_fo2(precision, want_u=True)["u"][:, :, ::-1]
+            assert taken(general) == 0
             assert H.max_rel(u, g) < bar, precision
     finally:
         dev.close()
@@ -51,3 +81,98 @@ def test_boundary_intensities_fp64(gpu_lib):
     raw = S.batch_model(npoints=65, nside=2, nlev=5, nquads=31)
     raw = replace(raw, abundance=raw.abundance * np.array([1.0e-20, 1.0]), velocity=np.zeros_like(raw.velocity))
     assert_same_u(H.setup(raw), 6e-15, ("fp64",))
+
+
+@pytest.mark.parametrize("nquads,approx", [(1, "None"), (5, "None"), (16, "OneLine"), (31, "CloseLines"),
+                                           (32, "CloseLines"), (33, "CloseLines"), (50, "OneLine")])
+def test_one_line(gpu_lib, nquads, approx):
+    """The reverse order of one line's frequencies is its own, so the general kernel here is the
+    (u, v) solve's, which is never staged.  Its origin row takes FP64 quotients where the other's
+    has single-precision coefficients (three roundings of 2^-24 and one of 2^-22): 1e-6 in split
+    precision.  FP64: the two positions' errors of 2^-53 line / width = 2e-10 on differences of
+    0.35 and more, 1e-9 a pair, ten pairs alike: 1e-8."""
+    raw = S.batch_model(npoints=1000, nside=1, nlev=2, nquads=nquads)
+    dev = _abi.DeviceModel(H.setup(raw, approx=approx))
+    try:
+        for precision, bar in (("split", 1e-6), ("fp64", 1e-8)):
+            u = dev.formal_solve_fo2(precision, want_u=True)["u"]
+            assert taken(dev) == dev.P * dev.R
+            v = dev.formal_solve_fo2_uv(precision)["u"]
+            assert taken(dev) == 0
+            assert H.max_rel(u, v) < bar, precision
+    finally:
+        dev.close()
+
+
+@pytest.mark.parametrize("nside,nquads", [(1, 11), (1, 31), (2, 7)])
+def test_pairs_left_to_the_general_kernel(gpu_lib, nside, nquads):
+    """Ray pairs that reach both lines are listed, the others are not, and both are right: single,
+    batched and as pixels."""
+    at_rest, moving = close_lines(nside, nquads)
+    dev, general = with_velocity(at_rest, moving["velocity"]), _abi.DeviceModel(moving)
+    batch = _abi.Batch([dev])
+    try:
+        for precision, bar in (("split", 1e-9), ("fp64", 1e-8)):
+            ref = general.formal_solve_fo2(precision, want_u=True)
+            assert taken(general) == 0
+            out = dev.formal_solve_fo2(precision, want_u=True)
+            n, listed = dev.staged_statistics()
+            assert n == dev.P * dev.R and 0 < listed < n, (n, listed)
+            assert H.max_rel(out["u"], ref["u"]) < bar, precision
+            assert H.max_rel(batch.formal_solve_fo2(precision)[0]["J"], ref["J"]) < bar, precision
+            n, in_batch = dev.staged_statistics()
+            assert n == dev.P * dev.R and in_batch == listed
+    finally:
+        batch.close()
+        dev.close()
+        general.close()
+
+
+def test_pixels_left_to_the_general_kernel(gpu_lib):
+    raw = S.grid_sphere(n=11, nside=1, nquads=5, nlev=3)
+    ld = raw.linedata[0]
+    f = np.array(ld.frequency, np.float64)
+    f[1] = f[0] * (1.0 + 1.0e-4)
+    slow = replace(raw, linedata=[replace(ld, frequency_given=f)], velocity=0.02 * raw.velocity)
+    fast = replace(slow, velocity=raw.velocity)
+    nu = (f[0] * (1.0 - 5.0e-5), f[0] * (1.0 + 1.5e-4), 41)
+    d = np.array((0.48, 0.36, 0.8))
+    fast = H.setup(fast, image_freqs=nu)
+    dev, general = with_velocity(H.setup(slow, image_freqs=nu), fast["velocity"]), _abi.DeviceModel(fast)
+    try:
+        for precision, bar in (("split", 1e-9), ("fp64", 1e-8)):
+            ref = general.image_new(d, 19, 14, precision)["I"]
+            assert taken(general) == 0
+            I = dev.image_new(d, 19, 14, precision)["I"]
+            n, listed = dev.staged_statistics()
+            assert n == 19 * 14 and 0 < listed, (n, listed)
+            assert H.max_rel(I, ref, floor=1e-6 * ref.max()) < bar, precision
+    finally:
+        dev.close()
+        general.close()
+
+
+@pytest.mark.parametrize("npoints,nside,nquads,nlev,staged", [(9000, 2, 31, 3, True), (600, 2, 60, 42, False)])
+def test_fixed_area(gpu_lib, npoints, nside, nquads, nlev, staged):
+    """The 64 MiB of mgr_formal_solve_fo2_device_noalloc: several passes, each with its list, or
+    the general kernel where the area's rays would not fill the GPU."""
+    torch = pytest.importorskip("torch")
+    if staged:
+        at_rest, moving = close_lines(nside, nquads, npoints=npoints)
+        dev, general = with_velocity(at_rest, moving["velocity"]), _abi.DeviceModel(moving)
+    else:
+        moving = H.setup(S.batch_model(npoints=npoints, nside=nside, nlev=nlev, nquads=nquads))
+        dev, general = _abi.DeviceModel(moving), _abi.DeviceModel(in_reverse(moving))
+    try:
+        J = torch.empty((dev.P, dev.F), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        _abi._check(_abi.load().mgr_formal_solve_fo2_device_noalloc(dev.h, _abi.PRECISION["split"],
+                                                                    C.c_void_p(J.data_ptr()), None, None))
+        dev.sync()
+        n, listed = dev.staged_statistics()
+        assert n == (dev.P * dev.R if staged else 0) and (listed > 0) == staged
+        ref = general.formal_solve_fo2("split")["J"]
+        assert H.max_rel(J.cpu().numpy(), ref if staged else ref[:, ::-1]) < 1e-9
+    finally:
+        dev.close()
+        general.close()
