@@ -176,3 +176,46 @@ def test_fixed_area(gpu_lib, npoints, nside, nquads, nlev, staged):
     finally:
         dev.close()
         general.close()
+
+
+def hardly_any_listed(raw, share, bar=1e-9):
+    """The staged solve takes all but `share` of the model's ray pairs by itself, and its u is the
+    general kernel's."""
+    a = H.setup(raw)
+    dev, general = _abi.DeviceModel(a), _abi.DeviceModel(in_reverse(a))
+    try:
+        u = dev.formal_solve_fo2("split", want_u=True)["u"]
+        n, listed = dev.staged_statistics()
+        assert n == dev.P * dev.R and listed <= share * n, (n, listed)
+        g = general.formal_solve_fo2("split", want_u=True)["u"][:, :, ::-1]
+        assert H.max_rel(u, g) < bar
+    finally:
+        dev.close()
+        general.close()
+
+
+@pytest.mark.parametrize("step,boundary,share", [(1.0e12, S.BC_CMB, 0.0), (1.0e12, S.BC_ZERO, 0.01),
+                                                 (1.0e7, S.BC_CMB, 0.0), (1.0e7, S.BC_ZERO, 0.01)])
+def test_faint_rays(gpu_lib, step, boundary, share):
+    """Pairs out of their line's reach have the minimum opacity's depth, 1e-26 per metre: 1e-14 with
+    a step of 1e12 m, where a dark boundary leaves the sweep's source below 1e-28, and 1e-19 with
+    one of 1e7 m; between points of a grid that lie at the same distance along the ray but for
+    roundings it is 1e-30 and below.  The density keeps the depth of a pair in reach the same."""
+    raw = S.batch_model(npoints=1500, nside=1, nlev=4, nquads=21, box=14 * step, n_h2=1.0e24 / step, sigma_v=2.0e3)
+    hardly_any_listed(replace(raw, boundary_condition=np.full(len(raw.boundary2point), boundary, np.int32)), share)
+
+
+def test_many_levels(gpu_lib):
+    """30 levels at 10 to 100 K: sources over thirty powers of ten.  The general kernel takes its
+    sources in true units and as zero below 1.2e-38; u is a mean of sources and boundary
+    intensities, so that is off by 1.2e-38 at most."""
+    a = H.setup(S.nlte_sphere(npoints=2000, nside=1, nlev=30, nquads=11))
+    dev, general = _abi.DeviceModel(a), _abi.DeviceModel(in_reverse(a))
+    try:
+        u = dev.formal_solve_fo2("split", want_u=True)["u"]
+        assert dev.staged_statistics() == (dev.P * dev.R, 0)
+        g = general.formal_solve_fo2("split", want_u=True)["u"][:, :, ::-1]
+        assert np.all(np.abs(u - g) < 1e-9 * np.abs(g) + 1.2e-38)
+    finally:
+        dev.close()
+        general.close()
