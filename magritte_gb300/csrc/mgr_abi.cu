@@ -666,10 +666,10 @@ int mgr_formal_solve_fo2_device(MgrModel* model, int precision, double* J_dev, d
                   "(nfreqs = nlines*nquads with every frequency mapped to its line)");
         return MGR_ERR_UNSUPPORTED;
     }
-    const size_t wb = fo2_work_bytes(model, model->dm.P, u_dev == nullptr, lambda_diag_dev != nullptr);
-    int rc = ensure_scratch(model, &model->work, &model->work_bytes, wb);
-    if (rc != MGR_OK) return rc;
-    cudaError_t e = launch_fo2_range(model, precision, 0, model->dm.P, J_dev, u_dev, lambda_diag_dev, model->work,
+    cudaError_t e = ensure_fo2_work(
+        model, fo2_work_bytes(model, model->dm.P, u_dev == nullptr, lambda_diag_dev != nullptr, precision));
+    if (e != cudaSuccess) return cuda_fail(e, "scratch allocation");
+    e = launch_fo2_range(model, precision, 0, model->dm.P, J_dev, u_dev, lambda_diag_dev, model->work,
                                      model->work_bytes);
     if (e != cudaSuccess) return cuda_fail(e, "formal solve launch");
     model->last_J = J_dev;
@@ -710,10 +710,11 @@ int mgr_formal_solve_fo2_alo_device(MgrModel* model, double* J_dev, double* u_de
         set_error("mgr_formal_solve_fo2_alo_device: the formal solve needs a line spectral discretisation");
         return MGR_ERR_UNSUPPORTED;
     }
-    const size_t wb = fo2_work_bytes(model, model->dm.P, true, true);
-    int rc = ensure_scratch(model, &model->work, &model->work_bytes, wb);
-    if (rc != MGR_OK) return rc;
-    cudaError_t e = launch_fo2_range(model, MGR_PRECISION_FP64, 0, model->dm.P, J_dev, u_dev, lambda_diag_dev,
+    // the banded kernel traces into shared memory
+    cudaError_t e =
+        ensure_fo2_work(model, fo2_work_bytes(model, model->dm.P, true, true, MGR_PRECISION_FP64, /*staged=*/false));
+    if (e != cudaSuccess) return cuda_fail(e, "scratch allocation");
+    e = launch_fo2_range(model, MGR_PRECISION_FP64, 0, model->dm.P, J_dev, u_dev, lambda_diag_dev,
                                      model->work, model->work_bytes, 0, 0xffffffffu, nullptr, nullptr, nullptr,
                                      alo_off_dev, alo_nr_dev);
     if (e != cudaSuccess) return cuda_fail(e, "banded formal solve launch");
@@ -777,10 +778,10 @@ int mgr_formal_solve_fo2_rays_device(MgrModel* model, int precision, uint32_t rr
         set_error("mgr_formal_solve_fo2_rays_device: the formal solve needs a line spectral discretisation");
         return MGR_ERR_UNSUPPORTED;
     }
-    const size_t wb = fo2_work_bytes(model, model->dm.P, true, lambda_diag_dev != nullptr);
-    int rc = ensure_scratch(model, &model->work, &model->work_bytes, wb);
-    if (rc != MGR_OK) return rc;
-    cudaError_t e = launch_fo2_range(model, precision, 0, model->dm.P, J_dev, nullptr, lambda_diag_dev, model->work,
+    cudaError_t e =
+        ensure_fo2_work(model, fo2_work_bytes(model, model->dm.P, true, lambda_diag_dev != nullptr, precision));
+    if (e != cudaSuccess) return cuda_fail(e, "scratch allocation");
+    e = launch_fo2_range(model, precision, 0, model->dm.P, J_dev, nullptr, lambda_diag_dev, model->work,
                                      model->work_bytes, rr_begin, rr_end);
     if (e != cudaSuccess) return cuda_fail(e, "partial formal solve launch");
     return MGR_OK;
@@ -850,10 +851,10 @@ int mgr_formal_solve_fo2_sparse_device(MgrModel* model, int precision, double* J
         set_error("mgr_formal_solve_fo2_sparse_device: the formal solve needs a line spectral discretisation");
         return MGR_ERR_UNSUPPORTED;
     }
-    const size_t wb = fo2_work_bytes(model, model->dm.P, true, lambda_diag_dev != nullptr);
-    int rc = ensure_scratch(model, &model->work, &model->work_bytes, wb);
-    if (rc != MGR_OK) return rc;
-    cudaError_t e = launch_fo2_range(model, precision, 0, model->dm.P, nullptr, nullptr, lambda_diag_dev, model->work,
+    cudaError_t e =
+        ensure_fo2_work(model, fo2_work_bytes(model, model->dm.P, true, lambda_diag_dev != nullptr, precision));
+    if (e != cudaSuccess) return cuda_fail(e, "scratch allocation");
+    e = launch_fo2_range(model, precision, 0, model->dm.P, nullptr, nullptr, lambda_diag_dev, model->work,
                                      model->work_bytes, 0, model->dm.hnrays, Jlin_dev);
     if (e != cudaSuccess) return cuda_fail(e, "memory-lean formal solve launch");
     model->last_J = nullptr;
@@ -903,11 +904,12 @@ int mgr_formal_solve_fo2_anis(MgrModel* model, int precision, double* J, double*
     }
     const DevModel& dm = model->dm;
     const size_t PL = (size_t)dm.P * dm.L;
-    int rc = ensure_scratch(model, &model->work, &model->work_bytes, fo2_work_bytes(model, dm.P, true, false));
-    if (rc != MGR_OK) return rc;
+    cudaError_t e = ensure_fo2_work(model, fo2_work_bytes(model, dm.P, true, false, precision));
+    if (e != cudaSuccess) return cuda_fail(e, "scratch allocation");
     // the six [P][L] results live in the u scratch
-    if ((rc = ensure_scratch(model, &model->u_scratch, &model->u_scratch_bytes, 6 * PL * 8)) != MGR_OK) return rc;
-    cudaError_t e = launch_fo2_range(model, precision, 0, dm.P, nullptr, nullptr, nullptr, model->work,
+    int rc = ensure_scratch(model, &model->u_scratch, &model->u_scratch_bytes, 6 * PL * 8);
+    if (rc != MGR_OK) return rc;
+    e = launch_fo2_range(model, precision, 0, dm.P, nullptr, nullptr, nullptr, model->work,
                                      model->work_bytes, 0, dm.hnrays, nullptr, model->u_scratch);
     double* outs[6] = {J, J2_0, J2_1_Re, J2_1_Im, J2_2_Re, J2_2_Im};
     for (int k = 0; k < 6 && e == cudaSuccess; k++)
@@ -1069,8 +1071,8 @@ int mgr_autotune_fo2(MgrModel* model, int precision, uint32_t sample_points, int
     const uint32_t o0 = (dm.P - n) / 2, o1 = o0 + n;
     int rc = ensure_scratch(model, &model->J_scratch, &model->J_scratch_bytes, (size_t)dm.P * dm.F * 8);
     if (rc != MGR_OK) return rc;
-    rc = ensure_scratch(model, &model->work, &model->work_bytes, fo2_work_bytes(model, n, true, false));
-    if (rc != MGR_OK) return rc;
+    cudaError_t e = ensure_fo2_work(model, fo2_work_bytes(model, n, true, false, precision));
+    if (e != cudaSuccess) return cuda_fail(e, "scratch allocation");
     int& minb = precision == MGR_PRECISION_SPLIT ? model->fo2_minb_split : model->fo2_minb_fp64;
     int& nwarps = precision == MGR_PRECISION_SPLIT ? model->fo2_warps_split : model->fo2_warps_fp64;
     const int keep_minb = minb, keep_warps = nwarps;
@@ -1081,7 +1083,6 @@ int mgr_autotune_fo2(MgrModel* model, int precision, uint32_t sample_points, int
     int bm = keep_minb, bw = keep_warps;
     const int minbs[3] = {2, 3, 4};
     const int warps[2] = {4, 8};
-    cudaError_t e = cudaSuccess;
     for (int mi = 0; mi < 3 && e == cudaSuccess; mi++) {
         for (int wi = 0; wi < 2 && e == cudaSuccess; wi++) {
             minb = minbs[mi];

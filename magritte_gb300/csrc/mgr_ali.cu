@@ -1743,7 +1743,8 @@ int mgr_compute_level_populations(MgrModel* model, int precision, int use_ng, lo
     if ((rc = scratch(&model->J_scratch, &model->J_scratch_bytes, PF * 8)) != MGR_OK) return rc;
     if ((rc = scratch(&model->lam_scratch, &model->lam_scratch_bytes, PL * 8)) != MGR_OK) return rc;
     if (st.sparse && (rc = scratch(&st.Jlin_buf, &st.Jlin_bytes, PL * 8)) != MGR_OK) return rc;
-    if ((rc = scratch(&model->work, &model->work_bytes, fo2_work_bytes(model, dm.P, true, true))) != MGR_OK) return rc;
+    cudaError_t ew = ensure_fo2_work(model, fo2_work_bytes(model, dm.P, true, true, precision, /*staged=*/!bands));
+    if (ew != cudaSuccess) return cuda_fail(ew, "scratch allocation");
     if (bands) {
         cudaError_t eg = ensure_global(model);
         if (eg != cudaSuccess) return cuda_fail(eg, "global rate system allocation");

@@ -1,4 +1,7 @@
 // Kernels of the formal-solve path and their launchers.
+#include <algorithm>
+
+#include "mgr_ali.h"
 #include "mgr_internal.h"
 #include "mgr_reduce.cuh"
 #include "mgr_solve.cuh"
@@ -719,17 +722,57 @@ static size_t fo2_bytes_per_origin(const MgrModel* model) {
     return (size_t)model->dm.hnrays * model->dm.F * sizeof(double);
 }
 
-static size_t fo2_ray_bytes(const MgrModel* model, uint32_t nR);
+static size_t fo2_ray_bytes(const MgrModel* model, int precision, uint32_t nR);
 
-size_t fo2_work_bytes(const MgrModel* model, uint32_t n_origins, bool stage_u, bool stage_ld) {
+Fo2Work fo2_work_bytes(const MgrModel* model, uint32_t n_origins, bool stage_u, bool stage_ld, int precision,
+                       bool staged) {
     const int k = (stage_u ? 1 : 0) + (stage_ld ? 1 : 0);
-    const size_t rays = staged_ok(model) ? fo2_ray_bytes(model, model->dm.hnrays) : 0;
-    if ((k == 0 && rays == 0) || n_origins == 0) return 0;
-    const size_t per = fo2_bytes_per_origin(model) * k + rays;
-    size_t chunk = kFo2WorkBudget / per;
-    if (chunk < 1) chunk = 1;
-    if (chunk > n_origins) chunk = n_origins;
-    return chunk * per + 32;
+    auto area = [&](size_t per) -> size_t {
+        if (per == 0 || n_origins == 0) return 0;
+        const size_t chunk = std::min<size_t>(std::max<size_t>(kFo2WorkBudget / per, 1), n_origins);
+        return chunk * per;
+    };
+    const size_t per = fo2_bytes_per_origin(model) * k;
+    Fo2Work w;
+    w.least = w.most = area(per);
+    if (staged && staged_ok(model) && n_origins)
+        w.most = std::max(w.least, area(per + fo2_ray_bytes(model, precision, model->dm.hnrays)) + 32);
+    return w;
+}
+
+cudaError_t ensure_fo2_work(MgrModel* model, const Fo2Work& w) {
+    if (model->work_bytes >= w.most) return cudaSuccess;
+    const bool enough = model->work_bytes >= w.least;
+    if (enough) {
+        // an area the general kernel can do with: not worth an allocation inside a stream capture
+        // (which would end it), nor a second one where the device had no room before
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        cudaError_t e = cudaStreamIsCapturing(model->stream, &st);
+        if (e != cudaSuccess) return e;
+        if (st != cudaStreamCaptureStatusNone || w.most >= model->work_refused) return cudaSuccess;
+    }
+    void* q = nullptr;
+    size_t bytes = w.most;
+    cudaError_t e = cudaMalloc(&q, bytes);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        model->work_refused = std::min(model->work_refused, bytes);
+        if (enough) return cudaSuccess;
+    }
+    if (model->work) cudaFree(model->work);  // waits for the work that uses it
+    ali_shard_changed(model);                // a captured ALI iteration holds the old address
+    model->work = nullptr;
+    model->work_bytes = 0;
+    // where there is no room: less and less of the rays, down to none
+    while (e != cudaSuccess) {
+        if ((e = cudaMalloc(&q, bytes)) == cudaSuccess) break;
+        if (bytes == w.least) return e;
+        cudaGetLastError();
+        bytes = std::max(bytes / 2, w.least);
+    }
+    model->work = static_cast<double*>(q);
+    model->work_bytes = bytes;
+    return cudaSuccess;
 }
 
 // Whether the staged solve serves this model: its tiles hold one line's data, so the
@@ -774,10 +817,11 @@ StagedPlan staged_plan(const DevModel& m) {
     return best;
 }
 
-// Memory of one origin for the staged solve: its half rays in either precision's layout and
+// Memory of one origin for the staged solve: its half rays in the precision's layout and
 // its share of the list of ray pairs given up.
-static size_t fo2_ray_bytes(const MgrModel* model, uint32_t nR) {
-    return staged_origin_bytes(MODE_FP64, model->half_cap, nR) + (size_t)nR * sizeof(uint32_t);
+static size_t fo2_ray_bytes(const MgrModel* model, int precision, uint32_t nR) {
+    return staged_origin_bytes(precision == MGR_PRECISION_SPLIT ? MODE_SPLIT : MODE_FP64, model->half_cap, nR) +
+           (size_t)nR * sizeof(uint32_t);
 }
 
 template <int MODE, int AP, int MINB>
@@ -1011,7 +1055,7 @@ cudaError_t launch_fo2_range(MgrModel* model, int precision, uint32_t o_begin, u
     // GPU (or of all of them); the general kernel traces into shared memory
     bool staged = work && !v && !alo_off && staged_ok(model) && (uint64_t)chunk * nR < 0xffffffffu;
     if (staged) {
-        const size_t fit = work_bytes > 32 ? (work_bytes - 32) / (per * k + fo2_ray_bytes(model, m.hnrays)) : 0;
+        const size_t fit = work_bytes > 32 ? (work_bytes - 32) / (per * k + fo2_ray_bytes(model, precision, m.hnrays)) : 0;
         if (fit >= chunk) {
         } else if (fit * nR >= (uint64_t)model->sm_count * 32) {
             chunk = (uint32_t)fit;

@@ -78,6 +78,7 @@ struct MgrModel {
     // staging of u(rr, o, f) / L_diag(rr, o, f) between the two formal-solve stages
     double* work = nullptr;
     size_t work_bytes = 0;
+    size_t work_refused = SIZE_MAX;  // smallest size there was no room for
     // J [P][F] and ALO diagonal [P][L] of the last formal solve (device), for Jeff
     const double* last_J = nullptr;
     const double* last_lam = nullptr;
@@ -156,11 +157,19 @@ void count_launch();
 cudaError_t launch_size_rays(MgrModel* model, uint32_t* d_max_steps);
 // Formal solve of origins [o_begin, o_end): J [P][F] and lam [P][L] rows of those
 // origins, u [hnrays][P][F] (may be NULL).  Per-ray results are staged in `work`
-// (sized by fo2_work_bytes for the same u / lam choice) behind the chunk's traced half rays, in
-// chunks of origins that fit.  6.5 GiB: the 64^3 benchmark model (6.2 GB of u and L_diag, 17 GB
-// of half rays) in three chunks.
+// (ensure_fo2_work for the same u / lam choice) behind the chunk's traced half rays, in
+// chunks of origins that fit.  6.5 GiB: the 64^3 benchmark model in split precision (6.2 GB of u
+// and L_diag, 8.1 GB of half rays: 130,536 points, 24 ray pairs, 62 steps) in three chunks.
 constexpr size_t kFo2WorkBudget = size_t(13) << 29;
-size_t fo2_work_bytes(const MgrModel* model, uint32_t n_origins, bool stage_u, bool stage_ld);
+// The area of a formal solve: `least` what the general kernel stages, `most` with the half rays of
+// the staged solve (the same where that does not serve the model, or `staged` is false).
+struct Fo2Work {
+    size_t least, most;
+};
+Fo2Work fo2_work_bytes(const MgrModel* model, uint32_t n_origins, bool stage_u, bool stage_ld, int precision,
+                       bool staged = true);
+// The model's work area grown to w.most, or to as much above w.least as there is room for.
+cudaError_t ensure_fo2_work(MgrModel* model, const Fo2Work& w);
 // Ray pairs [rr_begin, rr_end) only (partial J / ALO sums, u must then be NULL).
 // J may be NULL; Jlin [P][L] (may be NULL) receives the line-integrated J in the order
 // of the memory-lean solve; anis [6][P][L] (may be NULL) the line-integrated J and
