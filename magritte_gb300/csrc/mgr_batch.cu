@@ -566,8 +566,6 @@ int mgr_batch_create(MgrModel* const* models, uint32_t n_models, MgrBatch** out)
     if (e == cudaSuccess) e = cudaMalloc(&b->d_ray_off, (n_models + 1) * sizeof(uint64_t));
     if (e == cudaSuccess)
         e = cudaMemcpy(b->d_ray_off, b->ray_off.data(), (n_models + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && b->ray_bytes) e = cudaMalloc(&b->rays, b->ray_bytes);
-    if (e == cudaSuccess && b->staged) e = cudaMalloc(&b->list, (item_off[n_models] + 1) * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMalloc(&b->stage_u, b->stage_entries * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&b->stage_ld, b->stage_entries * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_J, n_models * sizeof(double*));
@@ -586,6 +584,23 @@ int mgr_batch_create(MgrModel* const* models, uint32_t n_models, MgrBatch** out)
     if (e != cudaSuccess) {
         batch_release(b);
         return cuda_fail(e, "batch set-up");
+    }
+    // where there is no room for the rays of a wave: shorter waves, and the general kernel, which
+    // needs neither rays nor list, where there is none for the largest model's
+    if (b->staged) {
+        bool room = cudaMalloc(&b->list, (item_off[n_models] + 1) * sizeof(uint32_t)) == cudaSuccess;
+        while (room && cudaMalloc(&b->rays, b->ray_bytes) != cudaSuccess) {
+            room = b->ray_bytes > largest_rays;
+            b->ray_bytes = std::max(b->ray_bytes / 2, largest_rays);
+        }
+        if (!room) {
+            cudaFree(b->list);
+            b->list = nullptr;
+            b->rays = nullptr;
+            b->ray_bytes = 0;
+            b->staged = false;
+        }
+        cudaGetLastError();
     }
     const size_t per_warp = batch_need_bytes(b);
     int max_smem = 0;

@@ -91,3 +91,29 @@ def test_capture_of_a_first_solve(gpu_lib, long_rays):
     finally:
         dev.close()
         warm.close()
+
+
+@pytest.mark.parametrize("share,staged", [(1.2, True), (0.75, True), (0.3, False)])
+def test_batch_with_little_memory(gpu_lib, long_rays, share, staged):
+    """A share of the memory that a batch of two models takes, nearly all of it their half rays:
+    both in a wave, one, or the general kernel."""
+    devs = [_abi.DeviceModel(long_rays) for _ in range(2)]
+    try:
+        ref = devs[0].formal_solve_fo2("split")
+        devs[0].staged_statistics()
+        before = free_bytes()
+        batch = _abi.Batch(devs)
+        taken = before - free_bytes()
+        batch.close()
+        with Little(int(share * taken)):
+            batch = _abi.Batch(devs)
+        try:
+            for out in batch.formal_solve_fo2("split"):
+                assert H.max_rel(out["J"], ref["J"]) < 1e-9
+        finally:
+            batch.close()
+        for d in devs:
+            assert d.staged_statistics()[0] == (d.P * d.R if staged else 0)
+    finally:
+        for d in devs:
+            d.close()
