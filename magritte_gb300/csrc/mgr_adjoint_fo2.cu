@@ -224,13 +224,13 @@ int mgr_formal_solve_fo2_smooth_device(MgrModel* model, const uint32_t* origins_
     int nw;
     size_t smem;
     unsigned grid;
-    // u staged in the work area, for as many origins at a time as a pass of kSmoothStageBytes
-    // (or the area there is) holds
+    // u staged, for as many origins at a time as a pass of kSmoothStageBytes (or the room there
+    // is) holds
     const size_t per = (size_t)model->dm.hnrays * model->dm.F * sizeof(double);
     const size_t want = std::min<size_t>(n_o, std::max<size_t>(1, kSmoothStageBytes / per)) * per;
-    if (!grow_work(model, want) && model->work_bytes < per)
+    if (!grow_pass(model, want, per))
         return cuda_fail(cudaErrorMemoryAllocation, "mgr_formal_solve_fo2_smooth_device: staging");
-    const uint32_t pass = (uint32_t)std::min<size_t>(n_o, model->work_bytes / per);
+    const uint32_t pass = (uint32_t)std::min<size_t>(n_o, model->pass_bytes / per);
     auto run = [&](auto kern) -> cudaError_t {
         for (uint32_t i0 = 0; i0 < n_o; i0 += pass) {
             const uint32_t i1 = n_o - i0 > pass ? i0 + pass : n_o;
@@ -238,12 +238,12 @@ int mgr_formal_solve_fo2_smooth_device(MgrModel* model, const uint32_t* origins_
                                                 &grid);
             if (r != cudaSuccess) return r;
             count_launch();
-            kern<<<grid, nw * 32, smem, model->stream>>>(model->dm, cap, origins_dev, i0, i1, model->work, model->status);
+            kern<<<grid, nw * 32, smem, model->stream>>>(model->dm, cap, origins_dev, i0, i1, model->pass, model->status);
             if ((r = cudaGetLastError()) != cudaSuccess) return r;
             const uint64_t threads = (uint64_t)(i1 - i0) * model->dm.F;
             const uint64_t blocks = std::min<uint64_t>((threads + 255) / 256, (uint64_t)model->sm_count * 16);
             count_launch();
-            fo2_s_sum_kernel<<<(unsigned)blocks, 256, 0, model->stream>>>(model->dm, origins_dev, i0, i1, model->work,
+            fo2_s_sum_kernel<<<(unsigned)blocks, 256, 0, model->stream>>>(model->dm, origins_dev, i0, i1, model->pass,
                                                                           J_dev, model->status);
             if ((r = cudaGetLastError()) != cudaSuccess) return r;
         }

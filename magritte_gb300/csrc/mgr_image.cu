@@ -13,7 +13,6 @@
 #include <algorithm>
 #include <vector>
 
-#include "mgr_ali.h"
 #include "mgr_image.cuh"
 #include "mgr_staged.cuh"
 
@@ -208,17 +207,21 @@ static cudaError_t launch_image_t(MgrModel* model, uint32_t rr, double* I) {
 // Half rays of a pass of the staged imager at most.
 constexpr size_t kImageRayBytes = size_t(1) << 30;
 
-bool grow_work(MgrModel* model, size_t bytes) {
-    if (model->work_bytes >= bytes) return true;
+bool grow_pass(MgrModel* model, size_t bytes, size_t least) {
+    if (model->pass_bytes >= bytes || (model->pass_bytes >= least && bytes >= model->pass_refused)) return true;
+    if (least >= model->pass_refused) return false;
+    if (model->pass) cudaFree(model->pass);  // waits for the work that uses it
+    model->pass = nullptr;
+    model->pass_bytes = 0;
     void* q = nullptr;
-    if (cudaMalloc(&q, bytes) != cudaSuccess) {
+    while (cudaMalloc(&q, bytes) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        model->pass_refused = std::min(model->pass_refused, bytes);
+        if (bytes <= least) return false;
+        bytes = std::max(bytes / 2, least);
     }
-    if (model->work) cudaFree(model->work);  // waits for the work that uses it
-    ali_shard_changed(model);                // a captured ALI iteration holds the old address
-    model->work = static_cast<double*>(q);
-    model->work_bytes = bytes;
+    model->pass = static_cast<double*>(q);
+    model->pass_bytes = bytes;
     return true;
 }
 
@@ -242,8 +245,8 @@ cudaError_t image_size(MgrModel* model, const ImagePlane& ip, uint32_t* d_max, u
 
 template <int MODE, int AP, bool TAU>
 static cudaError_t launch_image_new_t(MgrModel* model, const ImagePlane& ip, uint32_t* d_max, double* I) {
-    // Intensities of models whose lines are apart: the staged solve where its rays fit the work
-    // area (151 x 97 pixels x 41 frequencies, FP64, 20k points: 14.4 ms by the general kernel,
+    // Intensities of models whose lines are apart: the staged solve where there is room for its
+    // rays (151 x 97 pixels x 41 frequencies, FP64, 20k points: 14.4 ms by the general kernel,
     // 2.5 ms staged).  Room for half rays a quarter longer than the formal solve's longest: nearly
     // every pixel's fits without a walk to size it first (0.63 ms), the others are listed.
     uint32_t cap = model->half_cap + model->half_cap / 4 + 8;
@@ -252,10 +255,10 @@ static cudaError_t launch_image_new_t(MgrModel* model, const ImagePlane& ip, uin
     const size_t pass = std::max<size_t>(1, std::min<size_t>(npix, kImageRayBytes / hb));
     const size_t list_at = (pass * hb + 15) & ~size_t(15);
     const bool staged = !TAU && (model->dm.L == 1 || (AP == APPROX_CLOSELINES && model->lines_apart)) &&
-                        grow_work(model, list_at + list_bytes);
+                        grow_pass(model, list_at + list_bytes, list_at + list_bytes);
     uint32_t* list = nullptr;
     if (staged) {
-        unsigned char* rays = reinterpret_cast<unsigned char*>(model->work);
+        unsigned char* rays = reinterpret_cast<unsigned char*>(model->pass);
         list = reinterpret_cast<uint32_t*>(rays + list_at);
         cudaError_t e = cudaMemsetAsync(list, 0, sizeof(uint32_t), model->stream);
         auto kern = image_staged_kernel<MODE, AP, MODE == MODE_SPLIT ? 4 : 2>;

@@ -97,6 +97,12 @@ struct MgrModel {
     // per-lane elimination scratch of the image adjoint (mgr_adjoint.cu), kept between calls
     double* adj_scratch = nullptr;
     size_t adj_scratch_bytes = 0;
+    // what a pass of the imager or of the smooth formal solves keeps (half rays, u, frequency
+    // derivatives): an area of its own, as a caller's stream capture of a formal solve holds the
+    // address of `work`
+    double* pass = nullptr;
+    size_t pass_bytes = 0;
+    size_t pass_refused = SIZE_MAX;  // smallest size there was no room for
     // host copies for the image-plane set-up (mgr_image.cu)
     std::vector<double> host_pos;     // [P][3]
     std::vector<uint32_t> host_p2b;   // [P]
@@ -179,8 +185,9 @@ cudaError_t launch_fo2_range(MgrModel* model, int precision, uint32_t o_begin, u
                              double* lam, double* work, size_t work_bytes, uint32_t rr_begin = 0,
                              uint32_t rr_end = 0xffffffffu, double* Jlin = nullptr, double* anis = nullptr,
                              double* v = nullptr, double* alo_off = nullptr, uint32_t* alo_nr = nullptr);
-// The model's work area grown to `bytes`; false (and the area as it was) when it cannot be.
-bool grow_work(MgrModel* model, size_t bytes);
+// The model's pass area grown to `bytes`, or to as much above `least` as there is room for; false
+// when there is no room for that.
+bool grow_pass(MgrModel* model, size_t bytes, size_t least);
 cudaError_t launch_trace_export(MgrModel* model, uint32_t o, uint32_t rr, uint32_t l, uint32_t capacity,
                                 uint32_t* d_meta, uint32_t* d_nr, uint32_t* d_ni, double* d_fac, double* d_shift,
                                 double* d_dZ);

@@ -1,6 +1,8 @@
 """The memory a formal solve takes beside its results: half rays only where the solve walks them into
 memory, less where the device has no room, and no allocation that a solve can do without inside a
 stream capture."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -117,3 +119,45 @@ def test_batch_with_little_memory(gpu_lib, long_rays, share, staged):
     finally:
         for d in devs:
             d.close()
+
+
+def smooth(dev, J):
+    _abi._check(_abi.load().mgr_formal_solve_fo2_smooth_device(dev.h, None, 0, C.c_void_p(J.data_ptr())))
+    return J.cpu().numpy()
+
+
+def test_captured_solve_outlives_images_and_smooth_solves(gpu_lib):
+    """A caller's graph of a formal solve holds the address of the work area: images and smooth
+    solves, however large, leave that where it is."""
+    a = H.setup(S.batch_model(npoints=1000, nside=1, nlev=3, nquads=11))
+    dev = _abi.DeviceModel(a)
+    try:
+        ref = dev.formal_solve_fo2("split", want_lambda=False)["J"]
+        J = torch.zeros((dev.P, dev.F), dtype=torch.float64, device="cuda")
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=torch.cuda.ExternalStream(dev.stream())):
+            dev.formal_solve_fo2_device("split", J.data_ptr())
+        dev.image_new(np.array((0.48, 0.36, 0.8)), 301, 299, "split")
+        smooth(dev, torch.zeros_like(J))
+        keep = [torch.full((1 << 24,), float("nan"), dtype=torch.float64, device="cuda") for _ in range(8)]
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(J.cpu().numpy(), ref)
+        del keep
+    finally:
+        dev.close()
+
+
+def test_smooth_solve_with_little_memory(gpu_lib):
+    """48 MB of u for every origin at once; with 20 MiB left, several passes and the same J."""
+    a = H.setup(S.batch_model(npoints=2000, nside=2, nlev=5, nquads=31))
+    dev, ref = _abi.DeviceModel(a), _abi.DeviceModel(a)
+    try:
+        J = torch.zeros((dev.P, dev.F), dtype=torch.float64, device="cuda")
+        want = smooth(ref, J).copy()
+        with Little(20 * MiB):
+            got = smooth(dev, J.zero_())
+        assert np.array_equal(got, want)
+    finally:
+        dev.close()
+        ref.close()
