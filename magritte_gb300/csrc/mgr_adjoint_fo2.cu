@@ -10,7 +10,8 @@
 // adjoint's warp sums need).  The forward stages u and a second kernel sums J(o, f) in the
 // reference's ray-pair order.  The backward keeps each lane's per-pair elimination state in a
 // scratch array of the warp's slot (recomputed, not saved by the forward) and adds its
-// derivatives with one atomic per warp and entry.
+// derivatives with one atomic per warp and entry; the frequencies' are staged per ray pair and
+// summed in order, as u is.
 //
 // What bounds them: the FP64 pipe, with as many of 32 lanes live as a line has quadrature points,
 // and instruction fetch (8 warps an SM on 335 KB of code; 553 KB with each half's sweep inlined).
@@ -72,10 +73,28 @@ __global__ void __launch_bounds__(256) fo2_s_sum_kernel(DevModel m, const uint32
     }
 }
 
+// The frequency derivatives of the origins, summed over the ray pairs in order (as the solve's
+// results are, and the same from run to run; one thread a sum, atomic for origins listed twice).
+__global__ void __launch_bounds__(256) fo2_nu_sum_kernel(DevModel m, const uint32_t* __restrict__ olist, uint32_t i0,
+                                                         uint32_t i1, const double* __restrict__ gJ,
+                                                         const double* __restrict__ GN, double* __restrict__ g_nu) {
+    const uint64_t n = (uint64_t)(i1 - i0) * m.F;
+    for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t i = i0 + (uint32_t)(k / m.F), f = (uint32_t)(k % m.F);
+        const uint32_t o = olist ? olist[i] : i;
+        if (gJ[(size_t)o * m.F + f] == 0.0) continue;
+        double v = 0.0;
+        for (uint32_t rr = 0; rr < m.hnrays; rr++) v += GN[((size_t)(i - i0) * m.hnrays + rr) * m.F + f];
+        atomicAdd(g_nu + (size_t)o * m.F + f, v);
+    }
+}
+
+// The adjoint of the listed origins i0 .. i1 - 1; frequency derivatives per ray pair in
+// GN[((i - i0) * hnrays + rr) * F + f], for the frequencies with a derivative of the loss.
 template <int AP>
 __global__ void __launch_bounds__(256) fo2_adj_kernel(DevModel m, uint32_t cap, const uint32_t* __restrict__ olist,
-                                                      uint32_t n_o, const double* __restrict__ gJ, AdjGrads g,
-                                                      double* __restrict__ g_nu, double* __restrict__ scratch,
+                                                      uint32_t i0, uint32_t i1, const double* __restrict__ gJ,
+                                                      AdjGrads g, double* __restrict__ GN, double* __restrict__ scratch,
                                                       uint32_t scratch_pairs, int* status) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int nw = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -87,9 +106,9 @@ __global__ void __launch_bounds__(256) fo2_adj_kernel(DevModel m, uint32_t cap, 
     __syncthreads();
     const size_t slot = (size_t)blockIdx.x * nw + w;
     const Fo2Scratch scr{scratch + slot * (size_t)scratch_pairs * 5 * 32 + lane, 32, scratch_pairs};
-    const uint64_t n = (uint64_t)n_o * m.hnrays;
+    const uint64_t n = (uint64_t)(i1 - i0) * m.hnrays;
     for (uint64_t item = (uint64_t)blockIdx.x * nw + w; item < n; item += (uint64_t)gridDim.x * nw) {
-        const uint32_t i = (uint32_t)(item / m.hnrays), rr = (uint32_t)(item % m.hnrays);
+        const uint32_t i = i0 + (uint32_t)(item / m.hnrays), rr = (uint32_t)(item % m.hnrays);
         const uint32_t o = olist ? olist[i] : i;
         // origins without a derivative of the loss contribute nothing
         bool any = false;
@@ -114,15 +133,16 @@ __global__ void __launch_bounds__(256) fo2_adj_kernel(DevModel m, uint32_t cap, 
                 const uint32_t q = q0 + lane;
                 const uint32_t f = m.lq2f[(size_t)l * m.Q + (q < m.Q ? q : m.Q - 1)];
                 const double gu = q < m.Q ? gJ[(size_t)o * m.F + f] * wt : 0.0;
-                if (!__any_sync(FULL_MASK, gu != 0.0)) continue;
                 double gvb = 0.0, gvf = 0.0, gn = 0.0;
-                if (!solve_lane_s_adj<AP>(m, sl, o, m.nu[(size_t)o * m.F + f], l, bk, nb, fw, nf, gu, scr, acc_b, acc_f,
-                                          gvb, gvf, gn)) {
-                    if (lane == 0) atomicOr(status, ST_CAPACITY);
-                    continue;
+                if (__any_sync(FULL_MASK, gu != 0.0)) {
+                    if (!solve_lane_s_adj<AP>(m, sl, o, m.nu[(size_t)o * m.F + f], l, bk, nb, fw, nf, gu, scr, acc_b,
+                                              acc_f, gvb, gvf, gn)) {
+                        if (lane == 0) atomicOr(status, ST_CAPACITY);
+                        continue;
+                    }
+                    for (int k = 0; k < 3; k++) vo[k] += gvb * db[k] + gvf * df[k];
                 }
-                for (int k = 0; k < 3; k++) vo[k] += gvb * db[k] + gvf * df[k];
-                if (q < m.Q && gn != 0.0) atomicAdd(g_nu + (size_t)o * m.F + f, gn);
+                if (q < m.Q) GN[(size_t)item * m.F + f] = gn;
                 __syncwarp();
             }
         for (int k = 0; k < 3; k++) {
@@ -283,8 +303,14 @@ int mgr_formal_solve_fo2_adjoint_device(MgrModel* model, const uint32_t* origins
     int nw;
     size_t smem;
     unsigned grid;
+    // the frequency derivatives per ray pair, in passes as the forward's u
+    const size_t per = (size_t)model->dm.hnrays * model->dm.F * sizeof(double);
+    const size_t want = std::min<size_t>(n_o, std::max<size_t>(1, kSmoothStageBytes / per)) * per;
+    if (!grow_pass(model, want, per))
+        return cuda_fail(cudaErrorMemoryAllocation, "mgr_formal_solve_fo2_adjoint_device: staging");
+    const uint32_t pass = (uint32_t)std::min<size_t>(n_o, model->pass_bytes / per);
     auto run = [&](auto kern) -> cudaError_t {
-        cudaError_t r = origin_launch_shape(model, kern, cap, (uint64_t)n_o * model->dm.hnrays, &nw, &smem, &grid);
+        cudaError_t r = origin_launch_shape(model, kern, cap, (uint64_t)pass * model->dm.hnrays, &nw, &smem, &grid);
         if (r != cudaSuccess) return r;
         const size_t need = (size_t)grid * nw * pairs * 5 * 32 * sizeof(double);
         if (model->adj_scratch_bytes < need) {  // grown on demand, kept for the next call
@@ -295,10 +321,20 @@ int mgr_formal_solve_fo2_adjoint_device(MgrModel* model, const uint32_t* origins
             if (r != cudaSuccess) return r;
             model->adj_scratch_bytes = need;
         }
-        count_launch();
-        kern<<<grid, nw * 32, smem, model->stream>>>(model->dm, cap, origins_dev, n_o, gJ_dev, g, g_nu_dev,
-                                                     model->adj_scratch, pairs, model->status);
-        return cudaGetLastError();
+        for (uint32_t i0 = 0; i0 < n_o; i0 += pass) {
+            const uint32_t i1 = n_o - i0 > pass ? i0 + pass : n_o;
+            count_launch();
+            kern<<<grid, nw * 32, smem, model->stream>>>(model->dm, cap, origins_dev, i0, i1, gJ_dev, g, model->pass,
+                                                         model->adj_scratch, pairs, model->status);
+            if ((r = cudaGetLastError()) != cudaSuccess) return r;
+            const uint64_t threads = (uint64_t)(i1 - i0) * model->dm.F;
+            const uint64_t blocks = std::min<uint64_t>((threads + 255) / 256, (uint64_t)model->sm_count * 16);
+            count_launch();
+            fo2_nu_sum_kernel<<<(unsigned)blocks, 256, 0, model->stream>>>(model->dm, origins_dev, i0, i1, gJ_dev,
+                                                                           model->pass, g_nu_dev);
+            if ((r = cudaGetLastError()) != cudaSuccess) return r;
+        }
+        return cudaSuccess;
     };
     e = (model->dm.approx == APPROX_CLOSELINES) ? run(fo2_adj_kernel<APPROX_CLOSELINES>)
                                                 : run(fo2_adj_kernel<APPROX_NONE>);
