@@ -194,6 +194,27 @@ static int adj_plane(MgrModel* model, const char* who, const double* raydir, uin
     return MGR_OK;
 }
 
+cudaError_t grow_adj_scratch(MgrModel* model, size_t per_block, unsigned* grid) {
+    if (model->adj_scratch_bytes >= *grid * per_block) return cudaSuccess;
+    if (model->adj_scratch_bytes >= per_block && *grid * per_block >= model->adj_refused) {
+        *grid = (unsigned)(model->adj_scratch_bytes / per_block);
+        return cudaSuccess;
+    }
+    cudaFree(model->adj_scratch);  // waits for the work that uses it
+    model->adj_scratch = nullptr;
+    model->adj_scratch_bytes = 0;
+    cudaError_t e;
+    while ((e = cudaMalloc(&model->adj_scratch, *grid * per_block)) != cudaSuccess) {
+        model->adj_refused = std::min(model->adj_refused, *grid * per_block);
+        model->adj_scratch = nullptr;
+        if (*grid <= 1) return e;
+        cudaGetLastError();
+        *grid /= 2;
+    }
+    model->adj_scratch_bytes = *grid * per_block;
+    return cudaSuccess;
+}
+
 static int finish(MgrModel* model, cudaError_t e, const char* who) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(model->stream);
     if (e != cudaSuccess) return cuda_fail(e, who);
@@ -352,15 +373,8 @@ int mgr_image_new_adjoint_device(MgrModel* model, const double* raydir, uint32_t
     auto run = [&](auto kern) -> cudaError_t {
         cudaError_t r = pixel_launch_shape(model, kern, cap, npix, &nw, &smem, &grid);
         if (r != cudaSuccess) return r;
-        const size_t need = (size_t)grid * nw * pairs * 4 * 32 * sizeof(double);
-        if (model->adj_scratch_bytes < need) {  // grown on demand, kept for the next call
-            cudaFree(model->adj_scratch);
-            model->adj_scratch = nullptr;
-            model->adj_scratch_bytes = 0;
-            r = cudaMalloc(&model->adj_scratch, need);
-            if (r != cudaSuccess) return r;
-            model->adj_scratch_bytes = need;
-        }
+        r = grow_adj_scratch(model, (size_t)nw * pairs * 4 * 32 * sizeof(double), &grid);
+        if (r != cudaSuccess) return r;
         count_launch();
         kern<<<grid, nw * 32, smem, model->stream>>>(model->dm, ip, cap, gI_dev, g, model->adj_scratch, pairs,
                                                      model->status);

@@ -312,15 +312,8 @@ int mgr_formal_solve_fo2_adjoint_device(MgrModel* model, const uint32_t* origins
     auto run = [&](auto kern) -> cudaError_t {
         cudaError_t r = origin_launch_shape(model, kern, cap, (uint64_t)pass * model->dm.hnrays, &nw, &smem, &grid);
         if (r != cudaSuccess) return r;
-        const size_t need = (size_t)grid * nw * pairs * 5 * 32 * sizeof(double);
-        if (model->adj_scratch_bytes < need) {  // grown on demand, kept for the next call
-            cudaFree(model->adj_scratch);
-            model->adj_scratch = nullptr;
-            model->adj_scratch_bytes = 0;
-            r = cudaMalloc(&model->adj_scratch, need);
-            if (r != cudaSuccess) return r;
-            model->adj_scratch_bytes = need;
-        }
+        r = grow_adj_scratch(model, (size_t)nw * pairs * 5 * 32 * sizeof(double), &grid);
+        if (r != cudaSuccess) return r;
         for (uint32_t i0 = 0; i0 < n_o; i0 += pass) {
             const uint32_t i1 = n_o - i0 > pass ? i0 + pass : n_o;
             count_launch();

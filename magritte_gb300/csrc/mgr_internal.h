@@ -97,6 +97,7 @@ struct MgrModel {
     // per-lane elimination scratch of the image adjoint (mgr_adjoint.cu), kept between calls
     double* adj_scratch = nullptr;
     size_t adj_scratch_bytes = 0;
+    size_t adj_refused = SIZE_MAX;  // smallest size there was no room for
     // what a pass of the imager or of the smooth formal solves keeps (half rays, u, frequency
     // derivatives): an area of its own, as a caller's stream capture of a formal solve holds the
     // address of `work`
@@ -188,6 +189,9 @@ cudaError_t launch_fo2_range(MgrModel* model, int precision, uint32_t o_begin, u
 // The model's pass area grown to `bytes`, or to as much above `least` as there is room for; false
 // when there is no room for that.
 bool grow_pass(MgrModel* model, size_t bytes, size_t least);
+// The adjoints' elimination scratch grown to *grid blocks of per_block bytes; a smaller *grid where
+// there is no room for that many.
+cudaError_t grow_adj_scratch(MgrModel* model, size_t per_block, unsigned* grid);
 cudaError_t launch_trace_export(MgrModel* model, uint32_t o, uint32_t rr, uint32_t l, uint32_t capacity,
                                 uint32_t* d_meta, uint32_t* d_nr, uint32_t* d_ni, double* d_fac, double* d_shift,
                                 double* d_dZ);

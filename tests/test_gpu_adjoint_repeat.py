@@ -50,3 +50,26 @@ def test_frequency_gradient_is_the_same_on_every_call(gpu_lib):
     finally:
         dev.close()
 
+
+def test_adjoint_with_little_memory(gpu_lib):
+    """42 MB of frequency derivatives and some hundred MB of elimination scratch; with 90 MiB left,
+    several passes of fewer warps and the same sums."""
+    a = H.setup(S.batch_model(npoints=2000, nside=2, nlev=5, nquads=31))
+    dev, ref = _abi.DeviceModel(a), _abi.DeviceModel(a)
+    try:
+        gJ = torch.ones((dev.P, dev.F), dtype=torch.float64, device="cuda")
+        before = torch.cuda.mem_get_info()[0]
+        want = gradients(ref, gJ)
+        torch.cuda.empty_cache()
+        took = before - torch.cuda.mem_get_info()[0]
+        assert took > 120 << 20
+        held = torch.empty(torch.cuda.mem_get_info()[0] - (90 << 20), dtype=torch.uint8, device="cuda")
+        got = gradients(dev, gJ)
+        del held
+        assert np.array_equal(got[5], want[5])
+        for a, b in zip(got[:5], want[:5]):
+            assert np.max(np.abs(a - b)) < 1e-11 * np.max(np.abs(b))
+    finally:
+        torch.cuda.empty_cache()
+        dev.close()
+        ref.close()
