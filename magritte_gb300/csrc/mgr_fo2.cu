@@ -781,7 +781,9 @@ cudaError_t ensure_fo2_work(MgrModel* model, const Fo2Work& w) {
 // 10^3 cube, 1 line x 11, FP64: 0.22 and 1.34 ms.
 bool staged_ok(const MgrModel* model) {
     const DevModel& m = model->dm;
-    if (!model->line_blocks) return false;
+    // without a minimum opacity a pair out of reach has no depth, and the reference's quotients by
+    // it are not finite: the general kernel reports that, difference rows would not
+    if (!model->line_blocks || !(m.min_opacity > 0.0)) return false;
     return m.approx == APPROX_ONELINE || m.L == 1 || (m.approx == APPROX_CLOSELINES && model->lines_apart);
 }
 

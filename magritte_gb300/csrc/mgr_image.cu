@@ -254,7 +254,7 @@ static cudaError_t launch_image_new_t(MgrModel* model, const ImagePlane& ip, uin
     const size_t hb = staged_half_bytes(MODE, cap), list_bytes = (size_t)(npix + 1) * sizeof(uint32_t);
     const size_t pass = std::max<size_t>(1, std::min<size_t>(npix, kImageRayBytes / hb));
     const size_t list_at = (pass * hb + 15) & ~size_t(15);
-    const bool staged = !TAU && (model->dm.L == 1 || (AP == APPROX_CLOSELINES && model->lines_apart)) &&
+    const bool staged = !TAU && model->dm.min_opacity > 0.0 && (model->dm.L == 1 || (AP == APPROX_CLOSELINES && model->lines_apart)) &&
                         grow_pass(model, list_at + list_bytes, list_at + list_bytes);
     uint32_t* list = nullptr;
     if (staged) {

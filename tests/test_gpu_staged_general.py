@@ -219,3 +219,22 @@ def test_many_levels(gpu_lib):
     finally:
         dev.close()
         general.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "split"])
+def test_no_minimum_opacity(gpu_lib, precision):
+    """Without a minimum opacity a pair out of its line's reach has no depth: a non-finite intensity,
+    which every solve and the imager report."""
+    raw = S.batch_model(npoints=300, nside=1, nlev=3, nquads=11, sigma_v=5.0e3)
+    f0, dd = raw.linedata[0].frequency[0], 8.0e3 / S.CC
+    d = np.array((0.48, 0.36, 0.8))
+    dev, image = (_abi.DeviceModel(H.setup(raw, min_opacity=0.0, image_freqs=q))
+                  for q in (None, (f0 * (1 - dd), f0 * (1 + dd), 11)))
+    try:
+        for call in (lambda: dev.formal_solve_fo2_uv(precision), lambda: dev.formal_solve_fo2(precision),
+                     lambda: image.image_new(d, 9, 9, precision)):
+            with pytest.raises(_abi.MgrError, match="non-finite"):
+                call()
+    finally:
+        dev.close()
+        image.close()
