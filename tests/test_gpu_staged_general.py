@@ -238,3 +238,14 @@ def test_no_minimum_opacity(gpu_lib, precision):
     finally:
         dev.close()
         image.close()
+
+
+def test_negative_opacities(gpu_lib):
+    """Every other point inverted, with an opacity of the minimum's size: the clamp at the minimum
+    decides the sources beside thick pairs.  (FP64: as in test_one_line.)"""
+    a = H.setup(S.batch_model(npoints=600, nside=1, nlev=3, nquads=11, sigma_v=2.0e3))
+    op = a["opacity"].copy()
+    op[::2] = -3.0e-22 * (1.0 + np.arange(len(op[::2]))[:, None] % 7)
+    a = dict(a, opacity=op, interp_criterion=np.ones_like(op))
+    assert_same_u(a, 1e-8, ("fp64",))
+    assert_same_u(a)
