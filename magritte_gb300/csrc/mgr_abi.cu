@@ -217,6 +217,7 @@ void mgr_model_free(MgrModel* model) {
     if (model->u_scratch) cudaFree(model->u_scratch);
     if (model->lam_scratch) cudaFree(model->lam_scratch);
     if (model->work) cudaFree(model->work);
+    for (void* p : model->work_before) cudaFree(p);
     if (model->pass) cudaFree(model->pass);
     if (model->adj_scratch) cudaFree(model->adj_scratch);
     if (model->v_scratch) cudaFree(model->v_scratch);

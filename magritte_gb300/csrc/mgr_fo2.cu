@@ -740,29 +740,40 @@ Fo2Work fo2_work_bytes(const MgrModel* model, uint32_t n_origins, bool stage_u, 
     return w;
 }
 
+cudaError_t note_work_capture(MgrModel* model, bool* capturing) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    const cudaError_t e = cudaStreamIsCapturing(model->stream, &st);
+    *capturing = e == cudaSuccess && st != cudaStreamCaptureStatusNone;
+    model->work_captured = model->work_captured || *capturing;
+    return e;
+}
+
+void drop_work(MgrModel* model) {
+    if (model->work && model->work_captured) model->work_before.push_back(model->work);
+    else if (model->work) cudaFree(model->work);  // waits for the work that uses it
+    ali_shard_changed(model);                     // a captured ALI iteration holds the old address
+    model->work = nullptr;
+    model->work_bytes = 0;
+    model->work_captured = false;
+}
+
 cudaError_t ensure_fo2_work(MgrModel* model, const Fo2Work& w) {
-    if (model->work_bytes >= w.most) return cudaSuccess;
+    bool capturing = false;
+    cudaError_t e = note_work_capture(model, &capturing);
+    if (e != cudaSuccess || model->work_bytes >= w.most) return e;
     const bool enough = model->work_bytes >= w.least;
-    if (enough) {
-        // an area the general kernel can do with: not worth an allocation inside a stream capture
-        // (which would end it), nor a second one where the device had no room before
-        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-        cudaError_t e = cudaStreamIsCapturing(model->stream, &st);
-        if (e != cudaSuccess) return e;
-        if (st != cudaStreamCaptureStatusNone || w.most >= model->work_refused) return cudaSuccess;
-    }
+    // an area the general kernel can do with: not worth an allocation inside a stream capture
+    // (which would end it), nor a second one where the device had no room before
+    if (enough && (capturing || w.most >= model->work_refused)) return cudaSuccess;
     void* q = nullptr;
     size_t bytes = w.most;
-    cudaError_t e = cudaMalloc(&q, bytes);
+    e = cudaMalloc(&q, bytes);
     if (e != cudaSuccess) {
         cudaGetLastError();
         model->work_refused = std::min(model->work_refused, bytes);
         if (enough) return cudaSuccess;
     }
-    if (model->work) cudaFree(model->work);  // waits for the work that uses it
-    ali_shard_changed(model);                // a captured ALI iteration holds the old address
-    model->work = nullptr;
-    model->work_bytes = 0;
+    drop_work(model);
     // where there is no room: less and less of the rays, down to none
     while (e != cudaSuccess) {
         if ((e = cudaMalloc(&q, bytes)) == cudaSuccess) break;

@@ -79,6 +79,8 @@ struct MgrModel {
     double* work = nullptr;
     size_t work_bytes = 0;
     size_t work_refused = SIZE_MAX;  // smallest size there was no room for
+    bool work_captured = false;      // a stream capture holds the address of `work`
+    std::vector<void*> work_before;  // earlier areas that one holds, kept as long as the model
     // J [P][F] and ALO diagonal [P][L] of the last formal solve (device), for Jeff
     const double* last_J = nullptr;
     const double* last_lam = nullptr;
@@ -177,6 +179,10 @@ Fo2Work fo2_work_bytes(const MgrModel* model, uint32_t n_origins, bool stage_u, 
                        bool staged = true);
 // The model's work area grown to w.most, or to as much above w.least as there is room for.
 cudaError_t ensure_fo2_work(MgrModel* model, const Fo2Work& w);
+// Notes a stream capture that will hold the area's address; *capturing: whether there is one.
+cudaError_t note_work_capture(MgrModel* model, bool* capturing);
+// Frees the area, or keeps it aside where a capture holds its address.
+void drop_work(MgrModel* model);
 // Ray pairs [rr_begin, rr_end) only (partial J / ALO sums, u must then be NULL).
 // J may be NULL; Jlin [P][L] (may be NULL) receives the line-integrated J in the order
 // of the memory-lean solve; anis [6][P][L] (may be NULL) the line-integrated J and

@@ -8,7 +8,6 @@
 // u, v and the per-direction ALO factors; stage 2 sums J and the ALO diagonal per
 // origin in the reference's order (ray pair outer, quadrature point inner, forward
 // then backward direction).
-#include "mgr_ali.h"
 #include "mgr_internal.h"
 #include "mgr_reduce.cuh"
 #include "mgr_solve.cuh"
@@ -208,11 +207,11 @@ int mgr_formal_solve_sc0_device(MgrModel* model, int precision, double* J_dev, d
         return MGR_ERR_UNSUPPORTED;
     }
     const size_t wb = sc0_work_bytes(model, model->dm.P, u_dev == nullptr, lambda_diag_dev != nullptr);
+    bool capturing = false;
+    cudaError_t ec = note_work_capture(model, &capturing);
+    if (ec != cudaSuccess) return cuda_fail(ec, "capture status");
     if (model->work_bytes < wb) {
-        if (model->work) cudaFree(model->work);
-        ali_shard_changed(model);  // a captured ALI iteration holds the old address
-        model->work = nullptr;
-        model->work_bytes = 0;
+        drop_work(model);
         void* q = nullptr;
         cudaError_t e = cudaMalloc(&q, wb);
         if (e != cudaSuccess) return cuda_fail(e, "scratch allocation");

@@ -161,3 +161,24 @@ def test_smooth_solve_with_little_memory(gpu_lib):
     finally:
         dev.close()
         ref.close()
+
+
+def test_captured_solve_outlives_larger_areas(gpu_lib):
+    """Solves that need a larger area leave the one a caller's graph holds."""
+    a = H.setup(S.batch_model(npoints=1000, nside=1, nlev=3, nquads=11))
+    dev = _abi.DeviceModel(a)
+    try:
+        ref = dev.formal_solve_fo2("split", want_lambda=False)["J"]
+        J = torch.zeros((dev.P, dev.F), dtype=torch.float64, device="cuda")
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=torch.cuda.ExternalStream(dev.stream())):
+            dev.formal_solve_fo2_device("split", J.data_ptr())
+        dev.formal_solve_fo2("fp64")
+        dev.formal_solve_sc0("split")
+        keep = [torch.full((1 << 24,), float("nan"), dtype=torch.float64, device="cuda") for _ in range(8)]
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(J.cpu().numpy(), ref)
+        del keep
+    finally:
+        dev.close()
