@@ -36,8 +36,8 @@ sys.path.insert(0, ROOT)
 
 METRIC = "point.ray.freq solves/s"
 # DRAM bytes per solve of the split staged solve kernel, ncu on the 33^3 sphere cutout:
-# 4715.4 MB read + written / 50.8 M solves
-TRAFFIC_BYTES_PER_SOLVE = 4715.425e6 / 50_821_152.0
+# 4870.5 MB read + written / 50.8 M solves
+TRAFFIC_BYTES_PER_SOLVE = 4870.516e6 / 50_821_152.0
 UNIT = "solves/s"
 
 
@@ -934,7 +934,7 @@ def run_ours(args, rank, ws):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": TRAFFIC_BYTES_PER_SOLVE * solves * (rr1 - rr0) / R,
                      "traffic_note": "DRAM read + write bytes per launch from an ncu capture of the staged solve kernel "
-                                     "on the 33^3 case (4715.4 MB for 50.8 M solves; ncu flushes the caches between "
+                                     "on the 33^3 case (4870.5 MB for 50.8 M solves; ncu flushes the caches between "
                                      "its passes; the kernel that walks the half rays is not in it), scaled by the "
                                      "solves of this launch: the half rays read and the u / L_diag staging written "
                                      "are proportional to solves",

@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(256, MINB)
 // Formal solve, stage 1, staged (mgr_staged.cuh).  trace_rays_kernel: a warp per half ray of
 // the origins' pairs, slot 2 ((o - o_begin) nR + rr - rr0) + side.  fo2_staged_kernel: a warp
 // per K consecutive (origin, ray pair) items, results as fo2_kernel's.  The walk is a chain of
-// loads: 2.7 of 17.7 ms on the 33^3 sphere at four CTAs an SM (64 registers; five the same, six
+// loads: 2.7 of 18.4 ms on the 33^3 sphere at four CTAs an SM (64 registers; five the same, six
 // 0.9 ms slower).
 // ---------------------------------------------------------------------------------
 template <int MODE, int GEO>
@@ -788,7 +788,7 @@ cudaError_t ensure_fo2_work(MgrModel* model, const Fo2Work& w) {
 
 // Whether the staged solve serves this model: its tiles hold one line's data, so the
 // frequencies come line by line and pairs that reach several lines are rare (each of those is
-// solved twice).  33^3 sphere, 4 lines x 31, split: 17.7 ms staged, 42.1 ms by the general kernel;
+// solved twice).  33^3 sphere, 4 lines x 31, split: 18.4 ms staged, 42.1 ms by the general kernel;
 // 10^3 cube, 1 line x 11, FP64: 0.22 and 1.34 ms.
 bool staged_ok(const MgrModel* model) {
     const DevModel& m = model->dm;
@@ -800,8 +800,11 @@ bool staged_ok(const MgrModel* model) {
 
 // How a warp's lanes are dealt out: K ray pairs per warp and chunks of whole lines (S = the
 // largest multiple of Q up to 32) or of 32 frequencies, whichever leaves the fewest
-// warp passes per ray pair, weighted by what more streams and pairs of different lengths
-// per warp cost.
+// warp passes per ray pair, weighted by what more streams (0.08, 0.2, 0.45 for 2, 4, 8) and pairs of
+// different lengths per warp (0.12 each) cost.  The weights are rough: over eleven sizes (1 to 9
+// lines of 5 to 50 points, spheres of 16^3 to 24^3) and both precisions the plan chosen is at most
+// 5.4 % slower than the best of all plans, 1.2 % on average, where one ray pair in chunks of
+// 32 is up to 40 % slower (5 points: 141 against 185 us, FP64 183 against 257).
 StagedPlan staged_plan(const DevModel& m) {
     StagedPlan best{1, 32, 32};
     double best_cost = 1e30;
@@ -1065,7 +1068,10 @@ cudaError_t launch_fo2_range(MgrModel* model, int precision, uint32_t o_begin, u
     const size_t per = fo2_bytes_per_origin(model);
     uint32_t chunk = o_end - o_begin;
     // the staged solve where the work area takes the half rays of enough origins to fill the
-    // GPU (or of all of them); the general kernel traces into shared memory
+    // GPU (or of all of them); the general kernel traces into shared memory.  Passes of 32 ray
+    // pairs an SM beat the general kernel in one pass (33^3 sphere, 4 x 31, split: 23.4 against
+    // 45.8 ms; 24^3, 4 x 11: 5.4 and 6.8; 24^3, 1 x 11: 0.79 and 1.11; FP64 by 3.8 to 4.4 times),
+    // passes of 16 not all (34.2, 8.3 and 1.21 ms), of 8 none in split precision
     bool staged = work && !v && !alo_off && staged_ok(model) && (uint64_t)chunk * nR < 0xffffffffu;
     if (staged) {
         const size_t fit = work_bytes > 32 ? (work_bytes - 32) / (per * k + fo2_ray_bytes(model, precision, m.hnrays)) : 0;

@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(256) image_new_kernel(DevModel m, ImagePlane i
 // ---------------------------------------------------------------------------------
 // New imager, staged (mgr_staged.cuh): image_trace_kernel walks a warp per pixel into global
 // memory, image_staged_kernel eliminates; pixels it gives up go to image_new_kernel.  The walk is
-// a chain of loads (0.4 ms of 2.3 for 151 x 97 pixels; 64 registers, four CTAs an SM), the
+// a chain of loads (0.4 ms of 2.4 for 151 x 97 pixels; 64 registers, four CTAs an SM), the
 // elimination FP64-bound (1.5 ms).
 // ---------------------------------------------------------------------------------
 template <int MODE>
@@ -247,7 +247,7 @@ template <int MODE, int AP, bool TAU>
 static cudaError_t launch_image_new_t(MgrModel* model, const ImagePlane& ip, uint32_t* d_max, double* I) {
     // Intensities of models whose lines are apart: the staged solve where there is room for its
     // rays (151 x 97 pixels x 41 frequencies, FP64, 20k points: 14.4 ms by the general kernel,
-    // 2.5 ms staged).  Room for half rays a quarter longer than the formal solve's longest: nearly
+    // 2.4 ms staged).  Room for half rays a quarter longer than the formal solve's longest: nearly
     // every pixel's fits without a walk to size it first (0.63 ms), the others are listed.
     uint32_t cap = model->half_cap + model->half_cap / 4 + 8;
     const uint32_t npix = ip.nx * ip.ny;
