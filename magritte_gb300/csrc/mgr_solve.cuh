@@ -901,9 +901,10 @@ MGR_HD void eta_chi_f32(const DevModel& m, const LaneCtx& c, const Elem& e, floa
     uint32_t lo = 0, hi = m.L;
     if (AP == APPROX_CLOSELINES) {
         // lines inside freq -+ max_dist * freq * ub[p] (solver.tpp:1216-1227)
+        // the roundings spelt out: the staged solve has to decide a line at the edge alike
         const float off0 = fmaf(c.fq, e.dsh, c.a0);
-        const float ub = m.max_dist_f * ((c.fq + c.fq * e.dsh) * m.ub_f[e.nr]);
-        bracket_f32(m, c, off0 - ub, off0 + ub, lo, hi);
+        const float width = fmaf(c.fq, e.dsh, c.fq) * m.ub_f[e.nr];
+        bracket_f32(m, c, fmaf(-m.max_dist_f, width, off0), fmaf(m.max_dist_f, width, off0), lo, hi);
     }
     for (uint32_t s = lo; s < hi; s++) {
         const uint32_t l = (AP == APPROX_CLOSELINES) ? m.sorted_map[s] : s;

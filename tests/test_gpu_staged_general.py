@@ -83,6 +83,14 @@ def test_boundary_intensities_fp64(gpu_lib):
     assert_same_u(H.setup(raw), 6e-15, ("fp64",))
 
 
+@pytest.mark.parametrize("seed", range(4))
+def test_edge_of_an_elements_reach(gpu_lib, seed):
+    """The same for the pairs of the trapezoid rule, whose elements decide by themselves: two of
+    these four models have a line at the edge's rounding that shows."""
+    raw = S.batch_model(npoints=6000, nside=2, nlev=5, nquads=31, seed=seed)
+    assert_same_u(H.setup(raw, max_distance_opacity_contribution=1.5))
+
+
 @pytest.mark.parametrize("nquads,approx", [(1, "None"), (5, "None"), (16, "OneLine"), (31, "CloseLines"),
                                            (32, "CloseLines"), (33, "CloseLines"), (50, "OneLine")])
 def test_one_line(gpu_lib, nquads, approx):
